@@ -66,6 +66,7 @@ struct TwoD : SinglesTab {
     int es;                   // UVvis family: two-level doubles (no |aa>)
     float anh;                // Anharmonicity keyword (0: per-frame files)
     const void *Us;           // Sparse/Diagonal doubles: substep propagators U[t][n][n] (f/ts, truncated)
+    int trunc;                // the Threshold drops elements of Us
     long e0;                  // eigen data for frames [e0, e0 + ne)
     const double *eV, *ew;    // V [ne][n][n], w [ne][n]
     float f32_full;           // deltat*icm2ifs*2pi in float
@@ -988,78 +989,441 @@ __device__ void rk4_doubles_step(const TwoD &D, long t, typename Vec2<R>::T *F, 
     }
 }
 
-// propagate_double_sparce (propagate.c:1304-1394) through frame t: ts times
-// an anharmonic half phase on |aa>, the symmetrised U (x) U update over the
-// element pairs of the truncated substep propagator (time_evolution_mat,
-// propagate.c:1241-1299, called with its row and column lists exchanged,
-// propagate.c:1496), and the second half phase.  Elements are enumerated in
-// time_evolution_mat's order (row a outer, column b inner); zero (truncated)
-// elements are not in the list.  V is the temporary of the update.
+// ---------------------------------------------------------------- doubles, sparse U
+// propagate_double_sparce (propagate.c:1304-1394; two-level sites
+// :1400-1473) with the truncated sub-step propagator of time_evolution_mat
+// (propagate.c:1241-1299): per sub-step an anharmonic half phase on |aa>, the
+// symmetrised U (x) U update, the second half phase.  Two kernels share what
+// follows: FP32 keeps the reference's order of terms (k2d_doubles_sparse32:
+// the response's cancellation amplifies another order by 10^3), FP64 multiplies
+// matrices (k2d_doubles_sparse64).
+
+// Which vector of a start point: u < 9 -> fr for (p1,p2) = (u/3, u%3); else
+// ft1[t1] for (p0,p2).
+struct DblVec { int kind, pa, p2, t1; };
+__device__ __forceinline__ DblVec dbl_vec(int u, int T1) {
+    if (u < 9) return {0, u / 3, u % 3, 0};
+    const int w = u - 9, cmb = w / T1;
+    return {1, cmb / 3, cmb % 3, w % T1};
+}
+
+// dipole_double (NISE_subs.c:485-509) of vector u: element (i, j), i <= j.
 template <typename R>
-__device__ void sparse_doubles_step(const TwoD &D, long t, typename Vec2<R>::T *F, typename Vec2<R>::T *V) {
+__device__ __forceinline__ typename Vec2<R>::T dbl_init(const TwoD &D, int s, int u, int i, int j) {
     typedef typename Vec2<R>::T R2;
     typedef Ar<R> A;
-    const int n = D.n, N2 = n * (n + 1) / 2, nn = n * n;
-    const R2 *Us = (const R2 *)D.Us + (t - D.f0) * nn;
-    const R sq2 = (R)1.41421356237f;
-    // fm = f * 0.5 / m with f = deltat*icm2ifs*twoPi (float), the product in double
-    const R fm = sizeof(R) == 4 ? (R)(float)((double)D.f32_full * 0.5 / D.ts) : (R)(D.f64_full * 0.5 / D.ts);
-    for (int sub = 0; sub < D.ts; sub++) {
-        for (int half = 0; half < 2; half++) {
-            if (half == 1)
-                for (int e = 0; e < N2; e++) F[e] = V[e];
-            else
-                for (int e = 0; e < N2; e++) V[e] = F[e];
-            for (int a = 0; a < n; a++) {
-                if (D.es) {  // propagate.c:1422-1426, 1465-1469: plain copies
-                    int ia = sindex(a, a, n);
-                    F[ia] = V[ia];
-                    continue;
-                }
-                R an = D.anh != 0.0f ? (R)D.anh : (R)D.T.anh[t * (1L + n) + 1 + a];
-                R arg = A::mul(fm, an);
-                R co = (R)cos((double)arg), si = (R)sin((double)arg);
-                int ia = sindex(a, a, n);
-                R2 v = V[ia], o;
-                o.x = A::sub(A::mul(co, v.x), A::mul(si, v.y));
-                o.y = A::add(A::mul(co, v.y), A::mul(si, v.x));
-                F[ia] = o;
+    const DblVec w = dbl_vec(u, D.T1);
+    const long tk = tk_of(D, s);
+    const R2 *src = (const R2 *)D.SE + ((size_t)s * D.T3 * nvec_se(D) + (w.kind == 0 ? w.pa : 3 + w.pa * D.T1 + w.t1)) * D.n;
+    R2 f;
+    if (i == j) {
+        const R o = (R)over_mu(D, tk, w.p2, i);
+        f.x = A::mul(o, src[i].x);
+        f.y = A::mul(o, src[i].y);
+    } else {
+        const R mi = (R)traj_mu(D.T, tk, w.p2, i), mj = (R)traj_mu(D.T, tk, w.p2, j);
+        f.x = A::add(A::mul(mi, src[j].x), A::mul(mj, src[i].x));
+        f.y = A::add(A::mul(mi, src[j].y), A::mul(mj, src[i].y));
+    }
+    return f;
+}
+
+// EA projections and dot products of the CTA's vectors u0 .. u0 + nv - 1 at t3
+// (calc_2DIR.c:456-488): dipole_double_last into G[q][p3][n] (float sums in
+// site order), then a warp per dot product.  at(q, j, a) is element (j, a) of
+// vector q; mu and ov [3][n] hold the frame's dipoles.
+template <typename R, typename At>
+__device__ __forceinline__ void dbl_ea(const TwoD &D, int s, int t3, int u0, int nv, typename Vec2<R>::T *G,
+                                       const R *mu, const R *ov, At at) {
+    typedef typename Vec2<R>::T R2;
+    typedef Ar<R> A;
+    const int n = D.n, NV = nvec_se(D), lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int e = threadIdx.x; e < nv * 3 * n; e += blockDim.x) {
+        const int q = e / (3 * n), p3 = e / n % 3, a = e % n;
+        R gr = 0, gi = 0;
+        for (int j = 0; j < n; j++) {
+            const R m = j == a ? ov[p3 * n + a] : mu[p3 * n + j];
+            const R2 f = at(q, j, a);
+            gr = A::add(gr, A::mul(m, f.x));
+            gi = A::add(gi, A::mul(m, f.y));
+        }
+        G[e].x = gr;
+        G[e].y = gi;
+    }
+    __syncthreads();
+    for (int qm = 0, item = 0; qm < 21 * nv; qm++) {
+        const int q = qm / 21, m = qm % 21;
+        const DblVec w = dbl_vec(u0 + q, D.T1);
+        const int p0 = c_px[m][0], p1 = c_px[m][1], p3 = c_px[m][3];
+        if (c_px[m][2] != w.p2 || (w.kind == 0 ? p1 : p0) != w.pa) continue;
+        const int reps = w.kind == 0 ? D.T1 : 1;
+        // the products of all matching (q, m) are dealt to the warps in turn
+        for (int r = (warp - item % nw + nw) % nw; r < reps; r += nw) {
+            const R2 *rv = (const R2 *)D.SE + (((size_t)s * D.T3 + t3) * NV + (w.kind == 0 ? 3 + p0 * D.T1 + r : p1)) * n;
+            double a1 = 0, a2 = 0;
+            for (int a = lane; a < n; a += 32) {
+                const R2 gq = G[(q * 3 + p3) * n + a];
+                const R rr = rv[a].x, ri = -rv[a].y;
+                a1 += (double)A::add(A::mul(gq.y, rr), A::mul(gq.x, ri));
+                a2 += (double)A::sub(A::mul(gq.x, rr), A::mul(ri, gq.y));
             }
-            if (half == 1) break;
-            for (int e = 0; e < N2; e++) V[e].x = V[e].y = 0;
-            for (int ea = 0; ea < nn; ea++) {
-                R2 ua = Us[ea];
-                if (ua.x == (R)0 && ua.y == (R)0) continue;
-                const int sA = ea % n, tA = ea / n;  // R = column, C = row (exchanged lists)
-                for (int eb = 0; eb <= ea; eb++) {
-                    R2 ub = Us[eb];
-                    if (ub.x == (R)0 && ub.y == (R)0) continue;
-                    const int u = eb % n, v = eb / n;
-                    R g = 1;
-                    if (sA != u) g = sq2;
-                    if (v != tA) g = sq2;
-                    if (sA != u && v != tA) g = 1;
-                    // two-level sites: g = 0 when exactly one index differs
-                    // (propagate.c:1448-1450); those terms add only zeros
-                    if (D.es && g != (R)1) continue;
-                    const int iA = sindex(sA, u, n), iB = sindex(tA, v, n);
-                    R pr = A::sub(A::mul(ua.x, ub.x), A::mul(ua.y, ub.y));
-                    R pi = A::add(A::mul(ua.y, ub.x), A::mul(ua.x, ub.y));
-                    R2 fb = F[iB], acc = V[iA];
-                    acc.x = A::add(acc.x, A::mul(A::mul(pr, fb.x), g));
-                    acc.x = A::sub(acc.x, A::mul(A::mul(pi, fb.y), g));
-                    acc.y = A::add(acc.y, A::mul(A::mul(pr, fb.y), g));
-                    acc.y = A::add(acc.y, A::mul(A::mul(pi, fb.x), g));
-                    V[iA] = acc;
+            for (int o = 16; o > 0; o >>= 1) {
+                a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+                a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+            }
+            if (lane == 0) {
+                const size_t o = (((size_t)s * D.T3 + t3) * 21 + m) * D.T1 + (w.kind == 0 ? r : w.t1);
+                (w.kind == 0 ? D.eaI : D.eaII)[o] = make_double2(a1, a2);
+            }
+        }
+        item += reps;
+    }
+}
+
+// The frame's dipoles, overtone dipoles and anharmonic half phases exp(i fm
+// Delta_a), fm = f * 0.5 / m with f = deltat*icm2ifs*twoPi (float), the
+// product in double; the identity for two-level sites (plain copies,
+// propagate.c:1422-1426, 1465-1469).
+template <typename R>
+__device__ __forceinline__ void dbl_frame(const TwoD &D, long tl, R *mu, R *ov, typename Vec2<R>::T *ph) {
+    const int n = D.n;
+    const R fm = sizeof(R) == 4 ? (R)(float)((double)D.f32_full * 0.5 / D.ts) : (R)(D.f64_full * 0.5 / D.ts);
+    for (int i = threadIdx.x; i < 3 * n; i += blockDim.x) {
+        mu[i] = (R)traj_mu(D.T, tl, i / n, i % n);
+        ov[i] = (R)over_mu(D, tl, i / n, i % n);
+    }
+    for (int a = threadIdx.x; a < n; a += blockDim.x) {
+        ph[a] = make_vec2<R>(1, 0);
+        if (!D.es) {
+            const R an = D.anh != 0.0f ? (R)D.anh : (R)D.T.anh[tl * (1L + n) + 1 + a], arg = Ar<R>::mul(fm, an);
+            ph[a] = make_vec2<R>((R)cos((double)arg), (R)sin((double)arg));
+        }
+    }
+}
+
+template <typename R>
+__device__ __forceinline__ typename Vec2<R>::T dbl_half(typename Vec2<R>::T ph, R x, R y) {
+    typedef Ar<R> A;
+    return make_vec2<R>(A::sub(A::mul(ph.x, x), A::mul(ph.y, y)), A::add(A::mul(ph.x, y), A::mul(ph.y, x)));
+}
+
+// Two single-precision operations per instruction, each rounded by itself.
+// The assembler contracts a two-wide product and sum into a fused multiply-add
+// whatever their rounding modifiers say, so the sum is written as a * one + b
+// with a one that it cannot see (a kernel argument): the same value and one
+// rounding.  The lane rate is that of the scalar operations; the two-wide form
+// halves the issue slots and the coefficient registers.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b, f32x2 one) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(one), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 both(float a) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(a));
+    return d;
+}
+
+// FP32: every term of the reference's sum, in its order and roundings.
+// time_evolution_mat lists U's kept elements row by row and
+// propagate_double_sparce adds, for every pair ea >= eb of them, U_ea U_eb g
+// F{rows} to V{columns}: for V{p,q} that is, t ascending, column p of row t
+// with column q of the rows v < t, then column q of row t with column p of the
+// rows v <= t.  So a thread owns one V{p,q} and runs its n^2 terms, and the
+// outputs run in parallel.  The product U_ea U_eb is the same for every
+// vector: a thread carries 8 vectors of one start point, kept in pairs for the
+// two-wide instructions, and the lanes of a warp read the same F{t,v} (four
+// broadcast 16-byte loads per term).  g is sqrt2 for t = v where p != q (peeled
+// off the loop) and for t != v where p = q (those outputs come last, so that a
+// warp seldom holds both kinds).  Small N: NG groups of 8 vectors per CTA, so
+// that the outputs fill 8 warps.  TRUNC: the Threshold truncates, so zero
+// elements are skipped; else the list is full.
+constexpr int kSpVG = 8;
+
+template <bool G>
+__device__ __forceinline__ void sp32_term(f32x2 *ar, f32x2 *ai, float2 ua, float2 ub, const float *Fr, const float *Fi,
+                                          f32x2 one) {
+    typedef Ar<float> A;
+    const float pr = A::sub(A::mul(ua.x, ub.x), A::mul(ua.y, ub.y)), pi = A::add(A::mul(ua.y, ub.x), A::mul(ua.x, ub.y));
+    const f32x2 P = both(pr), Q = both(pi), M = both(-pi), g = both(1.41421356237f);
+#pragma unroll
+    for (int h = 0; h < kSpVG / 4; h++) {
+        const ulonglong2 fr = *(const ulonglong2 *)(Fr + 4 * h), fi = *(const ulonglong2 *)(Fi + 4 * h);
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const f32x2 x = k ? fr.y : fr.x, y = k ? fi.y : fi.x;
+            f32x2 a = mul2(P, x), b = mul2(M, y), c = mul2(P, y), d = mul2(Q, x);
+            if (G) { a = mul2(a, g); b = mul2(b, g); c = mul2(c, g); d = mul2(d, g); }
+            ar[2 * h + k] = add2(b, add2(a, ar[2 * h + k], one), one);
+            ai[2 * h + k] = add2(d, add2(c, ai[2 * h + k], one), one);
+        }
+    }
+}
+
+// The terms of row element ua with column c of the rows v < t.
+template <bool G, bool TRUNC>
+__device__ __forceinline__ void sp32_row(f32x2 *ar, f32x2 *ai, float2 ua, const float2 *Uc, int t, int n,
+                                         const float *Fr, const float *Fi, f32x2 one) {
+    if (TRUNC) {
+        if (ua.x == 0.0f && ua.y == 0.0f) return;
+        for (int v = 0; v < t; v++) {
+            const float2 ub = Uc[v * n];
+            if (ub.x == 0.0f && ub.y == 0.0f) continue;
+            sp32_term<G>(ar, ai, ua, ub, Fr + v * kSpVG, Fi + v * kSpVG, one);
+        }
+    } else {
+#pragma unroll 2
+        for (int v = 0; v < t; v++) sp32_term<G>(ar, ai, ua, Uc[v * n], Fr + v * kSpVG, Fi + v * kSpVG, one);
+    }
+}
+
+// F and V hold element {v,t}, v <= t, of a group's 8 vectors at
+// ([v + t(t+1)/2])[8], real and imaginary parts apart; with U in shared memory
+// (SM) where they fit, else F and V are in a workspace that stays in L2.
+template <bool SM, bool TRUNC>
+__global__ void __launch_bounds__(256, 3) k2d_doubles_sparse32(TwoD D, int vec_per_sample, int NG, float onef, float *ws) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int n = D.n, N2 = n * (n + 1) / 2, noff = n * (n - 1) / 2, tid = threadIdx.x, VC = NG * kSpVG;
+    const int blocks = (vec_per_sample + VC - 1) / VC, s = blockIdx.x / blocks, u0 = (blockIdx.x % blocks) * VC;
+    const int nv = min(VC, vec_per_sample - u0);
+    const size_t gp = (size_t)N2 * kSpVG, plane = gp * NG;
+    float *Fr = SM ? (float *)smem_raw : ws + blockIdx.x * 4 * plane, *Fi = Fr + plane, *Vr = Fi + plane, *Vi = Vr + plane;
+    float2 *Ush = SM ? (float2 *)(Vi + plane) : (float2 *)smem_raw;  // [n][n] (SM)
+    float2 *G = SM ? Ush + n * n : Ush;                              // [VC][3][n]
+    float2 *ph = G + 3 * VC * n;                                     // [n]
+    float *mu = (float *)(ph + n), *ov = mu + 3 * n;                 // [3][n] each
+    short2 *pq = (short2 *)(ov + 3 * n);                             // [N2] the outputs: p < q, then p = q
+    const f32x2 one = both(onef);
+    // element {j, a} of vector q
+    auto at = [&](int q, int j, int a) {
+        return (q / kSpVG) * gp + (size_t)(j < a ? j + a * (a + 1) / 2 : a + j * (j + 1) / 2) * kSpVG + q % kSpVG;
+    };
+    for (int q = tid; q < n; q += blockDim.x) {
+        for (int p = 0; p < q; p++) pq[q * (q - 1) / 2 + p] = make_short2((short)p, (short)q);
+        pq[noff + q] = make_short2((short)q, (short)q);
+    }
+    __syncthreads();
+    for (int e = tid; e < VC * N2; e += blockDim.x) {
+        const int q = e % VC;
+        const short2 ij = pq[e / VC];
+        const float2 f = q < nv ? dbl_init<float>(D, s, u0 + q, ij.x, ij.y) : make_float2(0, 0);
+        const size_t o = at(q, ij.x, ij.y);
+        Fr[o] = f.x;
+        Fi[o] = f.y;
+    }
+    for (int t3 = 0; t3 < D.T3; t3++) {
+        const long tl = tk_of(D, s) + t3;
+        const float2 *U = (const float2 *)D.Us + (size_t)(tl - D.f0) * n * n;
+        __syncthreads();
+        dbl_frame<float>(D, tl, mu, ov, ph);
+        if (SM && t3 < D.T3 - 1) {
+            for (int e = tid; e < n * n; e += blockDim.x) Ush[e] = U[e];
+            U = Ush;
+        }
+        __syncthreads();
+        if (D.ea) dbl_ea<float>(D, s, t3, u0, nv, G, mu, ov, [&](int q, int j, int a) {
+            const size_t o = at(q, j, a);
+            return make_float2(Fr[o], Fi[o]);
+        });
+        if (t3 == D.T3 - 1) break;
+        __syncthreads();
+        auto half = [&](int e) {
+            const int a = e / VC;
+            const size_t o = at(e % VC, a, a);
+            const float2 v = dbl_half<float>(ph[a], Fr[o], Fi[o]);
+            Fr[o] = v.x;
+            Fi[o] = v.y;
+        };
+        for (int sub = 0; sub < D.ts; sub++) {
+            for (int e = tid; e < VC * n; e += blockDim.x) half(e);
+            __syncthreads();
+            for (int e = tid; e < NG * N2; e += blockDim.x) {
+                const bool off = e < NG * noff;
+                const int eo = off ? e : e - NG * noff, per = off ? noff : n, grp = eo / per;
+                const short2 o2 = pq[(off ? 0 : noff) + eo % per];
+                const int p = o2.x, q = o2.y;
+                const float *fr = Fr + grp * gp, *fi = Fi + grp * gp;
+                f32x2 ar[kSpVG / 2], ai[kSpVG / 2];
+#pragma unroll
+                for (int k = 0; k < kSpVG / 2; k++) ar[k] = ai[k] = 0;
+                if (off) {
+                    for (int t = 0; t < n; t++) {
+                        const float2 up = U[t * n + p], uq = U[t * n + q];
+                        sp32_row<false, TRUNC>(ar, ai, up, U + q, t, n, fr, fi, one);
+                        sp32_row<false, TRUNC>(ar, ai, uq, U + p, t, n, fr, fi, one);
+                        // two-level sites: g = 0 when exactly one index differs (propagate.c:1448-1450)
+                        if (!D.es) sp32_term<true>(ar, ai, uq, up, fr + t * kSpVG, fi + t * kSpVG, one);
+                        fr += (t + 1) * kSpVG;
+                        fi += (t + 1) * kSpVG;
+                    }
+                } else {
+                    for (int t = 0; t < n; t++) {
+                        const float2 up = U[t * n + p];
+                        if (!D.es) sp32_row<true, TRUNC>(ar, ai, up, U + p, t, n, fr, fi, one);
+                        sp32_term<false>(ar, ai, up, up, fr + t * kSpVG, fi + t * kSpVG, one);
+                        fr += (t + 1) * kSpVG;
+                        fi += (t + 1) * kSpVG;
+                    }
                 }
+                const size_t o = at(grp * kSpVG, p, q);
+#pragma unroll
+                for (int k = 0; k < kSpVG / 2; k++) {
+                    *(f32x2 *)(Vr + o + 2 * k) = ar[k];
+                    *(f32x2 *)(Vi + o + 2 * k) = ai[k];
+                }
+            }
+            float *sw = Fr;
+            Fr = Vr;
+            Vr = sw;
+            sw = Fi;
+            Fi = Vi;
+            Vi = sw;
+            __syncthreads();
+            for (int e = tid; e < VC * n; e += blockDim.x) half(e);
+            // the next sub-step's first half phase is the same thread's
+        }
+    }
+}
+
+// FP64: on the symmetric matrix F_tv (its diagonal scaled by g = sqrt2) the
+// reference's N^4 / 2 terms are the product W = U F U^T:
+//   V_su = W_su (s != u),
+//   V_ss = g/2 W_ss + (1 - g^2/2) sum_t U_st^2 F_tt,
+// the second term because g is the reference's float constant, not exactly the
+// root of two.  Two-level sites keep a zero diagonal.  Both products have one
+// form, out[i][j] = sum_t A[t][i] B[t][j] (U is symmetric; the first product is
+// stored transposed), so lanes run over i and read A contiguously, the lanes of
+// a row block share the four columns of B, and 16 multiply-adds follow each set
+// of loads.  A CTA takes as many vectors of one start point as fill its 256
+// threads (they share U).
+//
+// acc[c] = sum_t A[t][i] B[t][j0 + c]; rows of la and lb elements, columns
+// past the last clamped (their results are not used).
+__device__ __forceinline__ void sp_tile(const double2 *A, int la, const double2 *B, int lb, int n, int i, int j0,
+                                        double2 *acc) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) acc[c] = make_double2(0, 0);
+#pragma unroll 2
+    for (int t = 0; t < n; t++) {
+        const double2 a = A[(size_t)t * la + i];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const double2 b = B[(size_t)t * lb + min(j0 + c, n - 1)];
+            acc[c].x += a.x * b.x - a.y * b.y;
+            acc[c].y += a.x * b.y + a.y * b.x;
+        }
+    }
+}
+
+// CTA per group of VC doubles vectors of one start point.  U, F and W are in
+// shared memory where they fit (SM); else F and W are in a workspace that
+// stays in L2.
+template <bool SM>
+__global__ void __launch_bounds__(256) k2d_doubles_sparse64(TwoD D, int vec_per_sample, int VC, double2 *ws) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int n = D.n, N2 = n * (n + 1) / 2, tid = threadIdx.x;
+    const size_t mat = (size_t)n * n;
+    const int groups = (vec_per_sample + VC - 1) / VC, s = blockIdx.x / groups, u0 = (blockIdx.x % groups) * VC;
+    const int nv = min(VC, vec_per_sample - u0);
+    double2 *sh = (double2 *)smem_raw;
+    double2 *Ush = sh;                                             // [n][n] (SM)
+    double2 *F = SM ? Ush + mat : ws + blockIdx.x * 2 * VC * mat;  // [VC][n][n], the diagonal scaled by g inside a step
+    double2 *W = F + VC * mat;                                     // [VC][n][n], first product, transposed
+    double2 *dF = SM ? W + VC * mat : sh;                          // [VC][n] the diagonal, unscaled
+    double2 *G = dF + VC * n;                                      // [VC][3][n]
+    double2 *ph = G + 3 * VC * n;                                  // [n]
+    double *mu = (double *)(ph + n), *ov = mu + 3 * n;             // [3][n] each
+    const double g = (double)1.41421356237f, corr = 1.0 - 0.5 * g * g;
+    for (int e = tid; e < nv * N2; e += blockDim.x) {
+        const int q = e / N2;
+        int i = 0, rem = e % N2;
+        while (rem >= n - i) { rem -= n - i; i++; }
+        const double2 f = dbl_init<double>(D, s, u0 + q, i, i + rem);
+        F[q * mat + (size_t)i * n + i + rem] = f;
+        F[q * mat + (size_t)(i + rem) * n + i] = f;
+    }
+    const int tiles = n * ((n + 3) / 4);
+    for (int t3 = 0; t3 < D.T3; t3++) {
+        const long tl = tk_of(D, s) + t3;
+        const double2 *U = (const double2 *)D.Us + (size_t)(tl - D.f0) * mat;
+        __syncthreads();
+        dbl_frame<double>(D, tl, mu, ov, ph);
+        if (SM && t3 < D.T3 - 1) {
+            for (int e = tid; e < n * n; e += blockDim.x) Ush[e] = U[e];
+            U = Ush;
+        }
+        __syncthreads();
+        if (D.ea) dbl_ea<double>(D, s, t3, u0, nv, G, mu, ov, [&](int q, int j, int a) { return F[q * mat + (size_t)j * n + a]; });
+        if (t3 == D.T3 - 1) break;
+        __syncthreads();
+        for (int e = tid; e < nv * n; e += blockDim.x) {
+            const int q = e / n, a = e % n;
+            double2 *d = F + q * mat + (size_t)a * n + a;
+            const double2 v = dbl_half<double>(ph[a], d->x, d->y);
+            dF[e] = v;
+            *d = make_double2(g * v.x, g * v.y);
+        }
+        for (int sub = 0; sub < D.ts; sub++) {
+            __syncthreads();
+            for (int e = tid; e < nv * tiles; e += blockDim.x) {
+                const int q = e / tiles, i = e % tiles % n, j0 = e % tiles / n * 4;
+                double2 acc[4];
+                sp_tile(U, n, F + q * mat, n, n, i, j0, acc);
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    if (j0 + c < n) W[q * mat + (size_t)(j0 + c) * n + i] = acc[c];
+            }
+            __syncthreads();
+            for (int e = tid; e < nv * tiles; e += blockDim.x) {
+                const int q = e / tiles, i = e % tiles % n, j0 = e % tiles / n * 4;
+                if (j0 + 3 < i) continue;  // the lower half is the mirror image
+                double2 acc[4];
+                sp_tile(W + q * mat, n, U, n, n, i, j0, acc);
+#pragma unroll
+                for (int c = 0; c < 4; c++) {
+                    const int j = j0 + c;
+                    if (j < i || j >= n) continue;
+                    double2 v = acc[c];
+                    if (j == i) {
+                        double2 dd = make_double2(0, 0);
+                        for (int t = 0; t < n; t++) {
+                            const double2 w = U[(size_t)t * n + i], f = dF[q * n + t];
+                            const double wr = w.x * w.x - w.y * w.y, wi = 2 * w.x * w.y;
+                            dd.x += wr * f.x - wi * f.y;
+                            dd.y += wr * f.y + wi * f.x;
+                        }
+                        v = D.es ? make_double2(0, 0)
+                                 : make_double2(0.5 * g * v.x + corr * dd.x, 0.5 * g * v.y + corr * dd.y);
+                    }
+                    F[q * mat + (size_t)i * n + j] = v;
+                    if (j != i) F[q * mat + (size_t)j * n + i] = v;
+                }
+            }
+            __syncthreads();
+            // the second half phase, and the next sub-step's first
+            for (int e = tid; e < nv * n; e += blockDim.x) {
+                const int q = e / n, a = e % n;
+                double2 *d = F + q * mat + (size_t)a * n + a;
+                double2 v = dbl_half<double>(ph[a], d->x, d->y);
+                if (sub + 1 < D.ts) {
+                    v = dbl_half<double>(ph[a], v.x, v.y);
+                    dF[e] = v;
+                    v = make_double2(g * v.x, g * v.y);
+                }
+                *d = v;
             }
         }
     }
 }
 
 // Thread per doubles vector: dipole_double at tk, then per t3 the EA
-// projections (dipole_double_last) and dot products, then one doubles step
-// (RK4, or the Sparse/Diagonal U (x) U step).
+// projections (dipole_double_last) and dot products, then one RK4 step.
 template <typename R>
 __global__ void k2d_doubles_seq(TwoD D, int vec_per_sample, void *Fbuf, void *Kbuf, void *hdbuf) {
     typedef typename Vec2<R>::T R2;
@@ -1125,8 +1489,7 @@ __global__ void k2d_doubles_seq(TwoD D, int vec_per_sample, void *Fbuf, void *Kb
                     }
                 }
         if (t3 == D.T3 - 1) break;
-        if (is_eigen_scheme(D.prop)) sparse_doubles_step<R>(D, tl, F, Kq);
-        else rk4_doubles_step<R>(D, tl, F, Kq, hd);
+        rk4_doubles_step<R>(D, tl, F, Kq, hd);
     }
 }
 
@@ -1210,10 +1573,6 @@ __global__ void k2d_reduce(const double *Rs, int S, size_t plane, double *R, int
     R[e] = a;
 }
 
-// Doubles RK4 (propagate_vec_RK4_doubles, propagate.c:376-590) and sparse
-// (time_evolution_mat + propagate_double_sparce) schemes are not provided by
-// this engine build; see nise_2dir's status message.
-
 template <typename R>
 __global__ void k2d_leftr(TwoD D) {
     typedef typename Vec2<R>::T R2;
@@ -1277,7 +1636,39 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf) {
         k2d_se<R><<<(nv + B - 1) / B, B, sm, st>>>(D);
         c->launches++;
     }
-    if (D.ea && (D.prop == NISE_PROP_RK4 || is_eigen_scheme(D.prop))) {
+    if (D.ea && is_eigen_scheme(D.prop)) {
+        const int vps = 9 + 9 * D.T1, n = D.n, N2 = n * (n + 1) / 2;
+        void *ws = nullptr;
+        if (sizeof(R) == 4) {
+            const int NG = std::max(1, std::min(128 / N2, (vps + kSpVG - 1) / kSpVG)), VC = NG * kSpVG;
+            const size_t small = sizeof(float2) * (3 * (size_t)VC + 1) * n + sizeof(float) * 6 * n + sizeof(short2) * N2;
+            const size_t all = sizeof(float) * 4 * VC * N2 + sizeof(float2) * n * n + small;
+            const int ctas = D.S * ((vps + VC - 1) / VC), threads = std::min(256, (NG * N2 + 31) / 32 * 32);
+            const bool sm = all <= 227 * 1024;  // up to 53 sites
+            auto kern = sm ? (D.trunc ? k2d_doubles_sparse32<true, true> : k2d_doubles_sparse32<true, false>)
+                           : (D.trunc ? k2d_doubles_sparse32<false, true> : k2d_doubles_sparse32<false, false>);
+            if ((e = smem_attr(kern, sm ? all : small))) return e;
+            if (!sm && (e = (int)cudaMallocAsync(&ws, sizeof(float) * 4 * VC * N2 * ctas, st))) return e;
+            kern<<<ctas, threads, sm ? all : small, st>>>(D, vps, NG, 1.0f, (float *)ws);
+        } else {
+            // vectors per CTA: enough 4-column tiles for 256 threads
+            const int tiles = n * ((n + 3) / 4), VC = std::min(vps, std::max(1, (256 + tiles - 1) / tiles));
+            const size_t mat = (size_t)n * n;
+            const size_t small = sizeof(double2) * (size_t)(4 * VC + 1) * n + sizeof(double) * 6 * n;
+            const size_t all = sizeof(double2) * mat * (1 + 2 * VC) + small;
+            const int ctas = D.S * ((vps + VC - 1) / VC);
+            if (all <= 227 * 1024) {  // up to 68 sites
+                if ((e = smem_attr(k2d_doubles_sparse64<true>, all))) return e;
+                k2d_doubles_sparse64<true><<<ctas, 256, all, st>>>(D, vps, VC, nullptr);
+            } else {
+                if ((e = smem_attr(k2d_doubles_sparse64<false>, small))) return e;
+                if ((e = (int)cudaMallocAsync(&ws, sizeof(double2) * mat * 2 * VC * ctas, st))) return e;
+                k2d_doubles_sparse64<false><<<ctas, 256, small, st>>>(D, vps, VC, (double2 *)ws);
+            }
+        }
+        if (ws) cudaFreeAsync(ws, st);
+        c->launches++;
+    } else if (D.ea && D.prop == NISE_PROP_RK4) {
         int vps = 9 + 9 * D.T1, tot = D.S * vps, N2 = D.n * (D.n + 1) / 2;
         void *Fb = nullptr, *Kb = nullptr, *Hb = nullptr;
         if ((e = (int)cudaMallocAsync(&Fb, sizeof(R2) * (size_t)tot * N2, st))) return e;
@@ -1426,6 +1817,7 @@ extern "C" int nise_2dir(nise_ctx *c, double *R, int *sample_count) {
     D.f32_dsub = nise_f32(p, 1, p.ts);
     D.f64_dsub = nise_f64(p, 1, p.ts);
     D.Us = SB.Us;
+    D.trunc = p.propagation == NISE_PROP_SPARSE && c->thres > 0;
     DevBuf<char> dcoef;
     D.rot_static = p.hamiltonian == NISE_HAM_COUPLING;
     if (ea) {  // doubles coupling coefficients: once (static couplings) or per frame
@@ -1461,8 +1853,10 @@ extern "C" int nise_2dir(nise_ctx *c, double *R, int *sample_count) {
     const int NV = 3 + 3 * T1;
     size_t per_sample = r2 * ((size_t)3 * T1 * N + 3 * N + (size_t)T3 * NV * N) + sizeof(double2) * (9 * (size_t)T1 + 9 * T3) +
                         2 * sizeof(double2) * (size_t)T3 * 21 * T1 + sizeof(double) * 12 * plane;
-    if (D.ea && (D.prop == NISE_PROP_RK4 || is_eigen_scheme(D.prop)))  // sequential doubles: state, 4 stages, diagonal
+    if (D.ea && D.prop == NISE_PROP_RK4)  // sequential doubles: state, 4 stages, diagonal
         per_sample += (9 + 9 * (size_t)T1) * (size_t)N * (N + 1) / 2 * (5 * r2 + r2 / 2);
+    if (D.ea && is_eigen_scheme(D.prop))  // two matrices per doubles vector where they exceed shared memory
+        per_sample += (40 + 9 * (size_t)T1) * 2 * r2 * (size_t)N * (N + 1);
     size_t budget = (size_t)1536 << 20;
     int chunk = (int)(budget / (per_sample > 0 ? per_sample : 1));
     if (chunk < 1) chunk = 1;
