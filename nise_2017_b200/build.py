@@ -37,6 +37,7 @@ CU_SOURCES = [
     "taylor_rv.cu",
     "eigen_large.cu",
     "dia_tc.cu",
+    "rk4.cu",
 ]
 CPP_SOURCES = [
     "api.cpp",

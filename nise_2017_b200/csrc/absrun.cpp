@@ -268,6 +268,8 @@ struct AbsRun {
     // RK4
     DevBuf<int2> dent;
     DevBuf<char> rkval;
+    DevBuf<uint32_t> rkrows;
+    DevBuf<int> rklen;
     Rk4Plan RP;
     // Taylor
     DevBuf<int> drp, dcol, dorder, dsptr, dcorder, drows, dsptr4, drows4;
@@ -438,6 +440,23 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
         if ((rc = dent.upload(c, ent)) || (rc = rkval.alloc(c, rsz * (size_t)nf * RP.k))) return rc;
         RP.entries = dent.p;
         RP.val = rkval.p;
+        if (N <= NISE_RK4_ROW_MAX_N) {
+            // every row's entries in ascending neighbour order: the entry list
+            // visits row i with its lower neighbours, itself, its upper ones
+            std::vector<std::vector<uint32_t>> row(N);
+            for (int k = 0; k < RP.k; k++) {
+                row[ent[k].x].push_back((uint32_t)ent[k].y | (uint32_t)k << 10);
+                if (ent[k].x != ent[k].y) row[ent[k].y].push_back((uint32_t)ent[k].x | (uint32_t)k << 10);
+            }
+            std::vector<int> len(N);
+            for (int i = 0; i < N; i++) RP.slots = std::max(RP.slots, len[i] = (int)row[i].size());
+            std::vector<uint32_t> rows((size_t)RP.slots * N, 0);
+            for (int i = 0; i < N; i++)
+                for (int q = 0; q < len[i]; q++) rows[(size_t)q * N + i] = row[i][q];
+            if ((rc = rkrows.upload(c, rows)) || (rc = rklen.upload(c, len))) return rc;
+            RP.rows = rkrows.p;
+            RP.len = rklen.p;
+        }
     } else {
         // Sparse / Diagonal: the exact propagator exp(-i H dt) (propagate_vec_DIA,
         // propagate.c:60-125).  Threshold > 0 keeps only large elements of U
@@ -834,7 +853,8 @@ int AbsRun::run_main(cudaStream_t s, int cfg, double2 *dst) {
             if (cfg > 0) return launch_abs_trotter_lv(pr, T, TP, Js, r, lvptr.p, nlev, cfg, s);
             return launch_abs_trotter(pr, T, TP, Js, r, s);
         case SCHEME_RK4:
-            return launch_abs_rk4(pr, T, RP, Js, r, s);
+            // a thread per site row up to the size that a CTA holds, a thread per vector above
+            return RP.rows ? launch_abs_rk4_row(pr, T, RP, Js, r, s) : launch_abs_rk4(pr, T, RP, Js, r, s);
         case SCHEME_TAYLOR: {
             TaylorPlan P = XP;
             P.only_v2 = cfg < 0;

@@ -32,7 +32,14 @@ struct Rk4Plan {
     long f0, nf;
     void *val;          // R [nf][k]
     int singleshift;
+    // rows for the row-owner kernel: row i's entries in ascending neighbour
+    // order at rows[slot * n + i] = neighbour | entry << 10, len[i] of them
+    const uint32_t *rows;
+    const int *len;
+    int slots;
 };
+// Sites the row-owner RK4 kernel takes: a CTA holds three vectors of them.
+#define NISE_RK4_ROW_MAX_N 320
 
 // Complex numbers per site row of the sliced-ELL Taylor kernel's state (the
 // 8 vectors of a CTA, unpadded): FP32 rows are 64 bytes, so even and odd rows
@@ -122,6 +129,9 @@ int launch_abs_trotter_wv2(int prec, const DevTraj &T, const TrotterPlan &P, con
                            const int *chk, int nchk, cudaStream_t s);
 int launch_prep_rk4(int prec, const DevTraj &T, const Rk4Plan &P, double fsub, float fsub32, cudaStream_t s);
 int launch_abs_rk4(int prec, const DevTraj &T, const Rk4Plan &P, const AbsJob &J, double2 *resp, cudaStream_t s);
+// The same with a thread per site row (rk4.cu; P.rows set, at most
+// NISE_RK4_ROW_MAX_N sites), bitwise identical in FP32.
+int launch_abs_rk4_row(int prec, const DevTraj &T, const Rk4Plan &P, const AbsJob &J, double2 *resp, cudaStream_t s);
 int launch_prep_taylor(int prec, const DevTraj &T, TaylorPlan &P, double rowabs_max, double f, int *order,
                        cudaStream_t s);
 // kernels (optional): the number of kernels launched (the sliced-ELL Taylor
