@@ -44,6 +44,7 @@ CPP_SOURCES = [
     "absrun.cpp",
     "input.cpp",
     "singles.cpp",
+    "rotsched.cpp",
     "translate.cpp",
 ]
 

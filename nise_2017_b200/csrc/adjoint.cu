@@ -23,10 +23,12 @@
 //   half phase  y_a = exp(-i h_a f/2) x_a:   dL/db_a += (f/2) Im(conj(l_a) y_a)
 //   rotation    y = R(theta) x, theta = s J f:  dL/ds += J f Re(l . dR/dtheta x)
 // and the response gradient G(t1) is injected as l_a += mu_a(t) G(t1).
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
 #include "engine.h"
+#include "rotsched.h"
 
 namespace {
 
@@ -185,6 +187,280 @@ __global__ void k_adj_bwd(DevTraj T, AdjPlan P, AbsJob J, const double2 *G, cons
     gscale[v] = gsc;
 }
 
+// ------------------------------------------------- a warp per vector
+// The same model with the rotations of a time step, or of a window of W time
+// steps, spread over a warp's lanes by nise_step_schedule: the lanes apply a
+// row of disjoint rotations, a __syncwarp separates the rows.  The half-step
+// phases ride on the first and the last rotation of each site.  A CTA takes
+// one start point; its three polarisations share the window's coefficients in
+// shared memory (read from global memory where they do not fit).  The states at
+// the steps inside a window are kept in `snap` by the lane that finishes a
+// site, for the responses; the backward sweep injects mu_a(t) G(t) when it
+// reaches a site's first rotation of step t.  W divides the checkpoint
+// interval.  Bound by the dependent issue of one or two warps per scheduler (a
+// row loads the state, runs four to six dependent double operations and stores
+// it), so what counts is the number of rows.
+// 256-site chain, 244 start points, RunTimes 128, with a thread per vector (23
+// warps in all, 1275 rotations in sequence per step): forward 32.4 ms, backward
+// 50.2 ms; now 3.6 and 5.6 ms (157 instructions per row, 4.3 cycles each).
+struct AdjCoef {
+    uint32_t e, p;
+    double2 cs, ua, ub;
+};
+
+__device__ __forceinline__ double2 cmul(double2 u, double2 z) {
+    return make_double2(z.x * u.x - z.y * u.y, z.y * u.x + z.x * u.y);
+}
+__device__ __forceinline__ double2 cmul_conj(double2 u, double2 z) {
+    return make_double2(z.x * u.x + z.y * u.y, z.y * u.x - z.x * u.y);
+}
+
+__device__ __forceinline__ AdjCoef adj_coef(const AdjPlan &P, uint32_t e, const uint32_t *parts, const double2 *rot,
+                                            const double2 *U) {
+    AdjCoef c;
+    c.e = e;
+    c.p = 0;
+    const uint32_t q = NISE_SCHED_Q(e), w = NISE_SCHED_W(e);
+    if (q != NISE_SCHED_NONE) {
+        c.p = parts[q];
+        c.cs = rot[(size_t)w * P.k + q];
+        c.ua = U[(size_t)w * P.n + NISE_SCHED_A(c.p)];
+        c.ub = U[(size_t)w * P.n + NISE_SCHED_B(c.p)];
+    }
+    return c;
+}
+
+// Copies the coefficients of `steps` frames from fi on into shared memory.
+__device__ __forceinline__ void adj_stage(const AdjPlan &P, long fi, int steps, double2 *rot, double2 *U, double *jf) {
+    for (int e = threadIdx.x; e < steps * P.k; e += blockDim.x) rot[e] = P.rot[fi * P.k + e];
+    for (int e = threadIdx.x; e < steps * P.n; e += blockDim.x) U[e] = P.U[fi * P.n + e];
+    if (jf)
+        for (int e = threadIdx.x; e < steps * P.k; e += blockDim.x) jf[e] = P.jf[fi * P.k + e];
+}
+
+template <bool SM>
+__global__ void __launch_bounds__(96) k_adj_fwd_warp(DevTraj T, AdjPlan P, AbsJob J, double2 *resp, double2 *ckpt) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int n = P.n, lane = threadIdx.x & 31, x = threadIdx.x >> 5, v = 3 * blockIdx.x + x;
+    double2 *X = (double2 *)smem_raw + (size_t)x * P.W * n, *snap = X + n;  // [3][X, W - 1 snapshots][n]
+    double2 *rsh = (double2 *)smem_raw + 3 * (size_t)P.W * n, *ush = rsh + (SM ? (size_t)P.W * P.k : 0);
+    uint32_t *psh = (uint32_t *)(ush + (SM ? (size_t)P.W * n : 0));
+    const uint32_t *parts = SM ? psh : P.parts;
+    if (SM)
+        for (int e = threadIdx.x; e < P.k; e += blockDim.x) psh[e] = P.parts[e];
+    const long ti = (long)(J.begin + blockIdx.x) * J.sample;
+    for (int a = lane; a < n; a += 32) X[a] = make_double2((double)traj_mu(T, ti, x, a), 0.0);
+    double2 *ck = ckpt + (size_t)v * P.nck * n;
+    auto respond = [&](int t1, const double2 *Z) {
+        double re = 0, im = 0;
+        for (int a = lane; a < n; a += 32) {
+            const double m = (double)traj_mu(T, ti + t1, x, a);
+            re += m * Z[a].x;
+            im += m * Z[a].y;
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            re += __shfl_xor_sync(0xffffffffu, re, o);
+            im += __shfl_xor_sync(0xffffffffu, im, o);
+        }
+        if (lane == 0) resp[(size_t)v * J.tmax + t1] = make_double2(re, im);
+    };
+    __syncwarp();
+    int t1 = 0;
+    while (true) {
+        respond(t1, X);
+        if (t1 % P.K == 0)
+            for (int a = lane; a < n; a += 32) ck[(size_t)(t1 / P.K) * n + a] = X[a];
+        if (t1 == J.tmax - 1) break;
+        const int steps = J.tmax - 1 - t1 >= P.W ? P.W : 1;
+        const uint32_t *rows = steps == P.W ? P.schedW : P.sched1;
+        const int nrow = steps == P.W ? P.nrowW : P.nrow1;
+        const long fi = ti + t1 - P.f0;
+        const double2 *rot = P.rot + fi * P.k, *U = P.U + fi * n;
+        if (SM) {
+            __syncthreads();
+            adj_stage(P, fi, steps, rsh, ush, nullptr);
+            __syncthreads();
+            rot = rsh;
+            U = ush;
+        }
+        AdjCoef c = adj_coef(P, nrow > 0 ? rows[lane] : NISE_SCHED_NONE, parts, rot, U);
+        uint32_t e1 = nrow > 1 ? rows[32 + lane] : NISE_SCHED_NONE;
+        for (int r = 0; r < nrow; r++) {
+            const AdjCoef nx = adj_coef(P, e1, parts, rot, U);
+            e1 = r + 2 < nrow ? rows[(size_t)(r + 2) * 32 + lane] : NISE_SCHED_NONE;
+            if (NISE_SCHED_Q(c.e) != NISE_SCHED_NONE) {
+                const int a = NISE_SCHED_A(c.p), b = NISE_SCHED_B(c.p);
+                double2 xa = X[a], xb = X[b];
+                if (NISE_SCHED_PRE_A(c.p)) xa = cmul(c.ua, xa);
+                if (NISE_SCHED_PRE_B(c.p)) xb = cmul(c.ub, xb);
+                // ya = co xa + i si xb, yb = co xb + i si xa
+                double2 ya = make_double2(c.cs.x * xa.x - c.cs.y * xb.y, c.cs.x * xa.y + c.cs.y * xb.x);
+                double2 yb = make_double2(c.cs.x * xb.x - c.cs.y * xa.y, c.cs.x * xb.y + c.cs.y * xa.x);
+                if (NISE_SCHED_POST_A(c.p)) ya = cmul(c.ua, ya);
+                if (NISE_SCHED_POST_B(c.p)) yb = cmul(c.ub, yb);
+                X[a] = ya;
+                X[b] = yb;
+                const int w = NISE_SCHED_W(c.e);
+                if (NISE_SCHED_LAST(c.e) && w < steps - 1) {
+                    if (NISE_SCHED_POST_A(c.p)) snap[(size_t)w * n + a] = ya;
+                    if (NISE_SCHED_POST_B(c.p)) snap[(size_t)w * n + b] = yb;
+                }
+            }
+            __syncwarp();
+            c = nx;
+        }
+        for (int i = lane; i < P.niso; i += 32) {
+            const int a = P.iso[i];
+            double2 z = X[a];
+            for (int w = 0; w < steps; w++) {
+                const double2 u = U[(size_t)w * n + a];
+                for (int s = 0; s < 2 * P.ts; s++) z = cmul(u, z);
+                if (w < steps - 1) snap[(size_t)w * n + a] = z;
+            }
+            X[a] = z;
+        }
+        __syncwarp();
+        for (int w = 0; w < steps - 1; w++) respond(t1 + w + 1, snap + (size_t)w * n);
+        __syncwarp();
+        t1 += steps;
+    }
+    for (int a = lane; a < n; a += 32) ck[(size_t)(P.nck - 1) * n + a] = X[a];
+}
+
+// Undo a half phase and carry the adjoint back, as adj_phase_back.
+__device__ __forceinline__ void adj_unphase(double2 u, double hf, double2 &y, double2 &l, double &g) {
+    g += hf * (l.x * y.y - l.y * y.x);
+    y = cmul_conj(u, y);
+    l = cmul_conj(u, l);
+}
+
+template <bool SM>
+__global__ void __launch_bounds__(96) k_adj_bwd_warp(DevTraj T, AdjPlan P, AbsJob J, const double2 *G,
+                                                     const double2 *ckpt, double *gshift, double *gscale) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int n = P.n, lane = threadIdx.x & 31, x = threadIdx.x >> 5, v = 3 * blockIdx.x + x;
+    double2 *X = (double2 *)smem_raw + 2 * (size_t)x * n, *L = X + n;
+    double *gs = (double *)((double2 *)smem_raw + 6 * (size_t)n) + (size_t)x * n;
+    double2 *rsh = (double2 *)((double *)((double2 *)smem_raw + 6 * (size_t)n) + 3 * (size_t)n + (n & 1));
+    double2 *ush = rsh + (SM ? (size_t)P.W * P.k : 0);
+    double *jsh = (double *)(ush + (SM ? (size_t)P.W * n : 0));
+    float *mu = (float *)(jsh + (SM ? (size_t)P.W * P.k : 0)) + (size_t)x * P.W * n;  // [3][W][n]
+    uint32_t *psh = (uint32_t *)((float *)(jsh + (SM ? (size_t)P.W * P.k : 0)) + 3 * (size_t)P.W * n);
+    const uint32_t *parts = SM ? psh : P.parts;
+    if (SM)
+        for (int e = threadIdx.x; e < P.k; e += blockDim.x) psh[e] = P.parts[e];
+    const long ti = (long)(J.begin + blockIdx.x) * J.sample;
+    const double2 *ck = ckpt + (size_t)v * P.nck * n;
+    const double hf = 0.5 * P.f;
+    double gsc = 0;
+    for (int a = lane; a < n; a += 32) {
+        const double m = (double)traj_mu(T, ti + J.tmax - 1, x, a);
+        X[a] = ck[(size_t)(P.nck - 1) * n + a];
+        L[a] = make_double2(m * G[J.tmax - 1].x, m * G[J.tmax - 1].y);
+        gs[a] = 0;
+    }
+    for (int t2 = J.tmax - 1; t2 > 0;) {  // the window [t1, t2), whole windows at multiples of W
+        const int steps = t2 % P.W == 0 ? P.W : 1, t1 = t2 - steps;
+        const uint32_t *rows = steps == P.W ? P.schedW : P.sched1;
+        const int nrow = steps == P.W ? P.nrowW : P.nrow1;
+        const long fi = ti + t1 - P.f0;
+        const double2 *rot = P.rot + fi * P.k, *U = P.U + fi * n;
+        const double *jf = P.jf + fi * P.k;
+        for (int e = lane; e < steps * n; e += 32) mu[e] = traj_mu(T, ti + t1 + e / n, x, e % n);
+        if (SM) {
+            __syncthreads();
+            adj_stage(P, fi, steps, rsh, ush, jsh);
+            rot = rsh;
+            U = ush;
+            jf = jsh;
+            __syncthreads();
+        }
+        __syncwarp();
+        AdjCoef c = adj_coef(P, nrow > 0 ? rows[(size_t)(nrow - 1) * 32 + lane] : NISE_SCHED_NONE, parts, rot, U);
+        uint32_t e1 = nrow > 1 ? rows[(size_t)(nrow - 2) * 32 + lane] : NISE_SCHED_NONE;
+        for (int r = nrow - 1; r >= 0; r--) {
+            const AdjCoef nx = adj_coef(P, e1, parts, rot, U);
+            e1 = r - 2 >= 0 ? rows[(size_t)(r - 2) * 32 + lane] : NISE_SCHED_NONE;
+            const uint32_t q = NISE_SCHED_Q(c.e);
+            if (q != NISE_SCHED_NONE) {
+                const int a = NISE_SCHED_A(c.p), b = NISE_SCHED_B(c.p), w = NISE_SCHED_W(c.e);
+                const double co = c.cs.x, si = c.cs.y, jq = jf[(size_t)w * P.k + q];
+                double2 ya = X[a], yb = X[b], la = L[a], lb = L[b];
+                double ga = 0, gb = 0;
+                if (NISE_SCHED_POST_A(c.p)) adj_unphase(c.ua, hf, ya, la, ga);
+                if (NISE_SCHED_POST_B(c.p)) adj_unphase(c.ub, hf, yb, lb, gb);
+                // inputs: xa = co ya - i si yb, xb = co yb - i si ya
+                double2 xa = make_double2(co * ya.x + si * yb.y, co * ya.y - si * yb.x);
+                double2 xb = make_double2(co * yb.x + si * ya.y, co * yb.y - si * ya.x);
+                // dy/dtheta with sin(theta) = -si, cos(theta) = co:
+                // dya = si xa - i co xb, dyb = si xb - i co xa
+                const double2 da = make_double2(si * xa.x + co * xb.y, si * xa.y - co * xb.x);
+                const double2 db = make_double2(si * xb.x + co * xa.y, si * xb.y - co * xa.x);
+                gsc += jq * (la.x * da.x + la.y * da.y + lb.x * db.x + lb.y * db.y);
+                double2 ka = make_double2(co * la.x + si * lb.y, co * la.y - si * lb.x);
+                double2 kb = make_double2(co * lb.x + si * la.y, co * lb.y - si * la.x);
+                if (NISE_SCHED_PRE_A(c.p)) adj_unphase(c.ua, hf, xa, ka, ga);
+                if (NISE_SCHED_PRE_B(c.p)) adj_unphase(c.ub, hf, xb, kb, gb);
+                if (NISE_SCHED_FIRST(c.e) && w > 0) {  // back at the start of step t1 + w
+                    const double2 g = G[t1 + w];
+                    if (NISE_SCHED_PRE_A(c.p)) {
+                        const double m = (double)mu[(size_t)w * n + a];
+                        ka = make_double2(ka.x + m * g.x, ka.y + m * g.y);
+                    }
+                    if (NISE_SCHED_PRE_B(c.p)) {
+                        const double m = (double)mu[(size_t)w * n + b];
+                        kb = make_double2(kb.x + m * g.x, kb.y + m * g.y);
+                    }
+                }
+                X[a] = xa;
+                X[b] = xb;
+                L[a] = ka;
+                L[b] = kb;
+                gs[a] += ga;
+                gs[b] += gb;
+            }
+            __syncwarp();
+            c = nx;
+        }
+        for (int i = lane; i < P.niso; i += 32) {
+            const int a = P.iso[i];
+            double2 z = X[a], l = L[a];
+            double ga = 0;
+            for (int w = steps - 1; w >= 0; w--) {
+                const double2 u = U[(size_t)w * n + a];
+                for (int s = 0; s < 2 * P.ts; s++) adj_unphase(u, hf, z, l, ga);
+                if (w > 0) {
+                    const double m = (double)mu[(size_t)w * n + a];
+                    l = make_double2(l.x + m * G[t1 + w].x, l.y + m * G[t1 + w].y);
+                }
+            }
+            X[a] = z;
+            L[a] = l;
+            gs[a] += ga;
+        }
+        __syncwarp();
+        for (int a = lane; a < n; a += 32) {
+            if (t1 % P.K == 0) X[a] = ck[(size_t)(t1 / P.K) * n + a];
+            const double m = (double)mu[a];
+            L[a] = make_double2(L[a].x + m * G[t1].x, L[a].y + m * G[t1].y);
+        }
+        __syncwarp();
+        t2 = t1;
+    }
+    for (int a = lane; a < n; a += 32) gshift[(size_t)v * n + a] = gs[a];
+    for (int o = 16; o > 0; o >>= 1) gsc += __shfl_xor_sync(0xffffffffu, gsc, o);
+    if (lane == 0) gscale[v] = gsc;
+}
+
+// Shared memory of the warp kernels: without the window's coefficients, and with them.
+size_t adj_fwd_bytes(int n, int k, int W, bool sm) {
+    return sizeof(double2) * 3 * (size_t)W * n + (sm ? sizeof(double2) * (size_t)W * (k + n) + 4 * (size_t)k : 0);
+}
+size_t adj_bwd_bytes(int n, int k, int W, bool sm) {
+    return sizeof(double2) * 6 * (size_t)n + sizeof(double) * (3 * (size_t)n + (n & 1)) + sizeof(float) * 3 * (size_t)W * n +
+           (sm ? (sizeof(double2) * (size_t)(k + n) + sizeof(double) * k) * W + 4 * (size_t)k : 0);
+}
+
 // Deterministic sums over vectors: g[a] = sum_v part[v][a] (a < n), in v order.
 __global__ void k_adj_reduce(const double *part, int nvec, int n, double *g) {
     int a = blockIdx.x * blockDim.x + threadIdx.x;
@@ -193,6 +469,9 @@ __global__ void k_adj_reduce(const double *part, int nvec, int n, double *g) {
     for (int v = 0; v < nvec; v++) s += part[(size_t)v * n + a];
     g[a] = s;
 }
+
+// Two CTAs per SM where the coefficients are staged.
+constexpr size_t kAdjShared = 112 * 1024;
 
 int lanes_adj(size_t lane_bytes) {
     int B = 64;
@@ -506,6 +785,14 @@ int launch_adj_prep(const DevTraj &T, const AdjPlan &P, cudaStream_t s) {
 int launch_adj_fwd(const DevTraj &T, const AdjPlan &P, const AbsJob &J, double2 *resp, double2 *ckpt,
                    cudaStream_t s) {
     const int nvec = 3 * J.nsamp;
+    if (P.sched1) {
+        const bool sm = adj_fwd_bytes(P.n, P.k, P.W, true) <= kAdjShared;
+        const size_t by = adj_fwd_bytes(P.n, P.k, P.W, sm);
+        auto kern = sm ? k_adj_fwd_warp<true> : k_adj_fwd_warp<false>;
+        if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)by)) return (int)e;
+        kern<<<J.nsamp, 96, by, s>>>(T, P, J, resp, ckpt);
+        return (int)cudaGetLastError();
+    }
     const size_t lb = sizeof(double2) * P.n;
     const int B = lanes_adj(lb);
     const size_t sm = lb * B;
@@ -518,12 +805,20 @@ int launch_adj_fwd(const DevTraj &T, const AdjPlan &P, const AbsJob &J, double2 
 int launch_adj_bwd(const DevTraj &T, const AdjPlan &P, const AbsJob &J, const double2 *G, const double2 *ckpt,
                    double *gshift_part, double *gscale_part, double *gshift, double *gscale, cudaStream_t s) {
     const int nvec = 3 * J.nsamp;
-    const size_t lb = (2 * sizeof(double2) + sizeof(double)) * P.n;
-    const int B = lanes_adj(lb);
-    const size_t sm = lb * B;
-    cudaError_t e = cudaFuncSetAttribute(k_adj_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e) return (int)e;
-    k_adj_bwd<<<(nvec + B - 1) / B, B, sm, s>>>(T, P, J, G, ckpt, gshift_part, gscale_part);
+    if (P.sched1) {
+        const bool sm = adj_bwd_bytes(P.n, P.k, P.W, true) <= kAdjShared;
+        const size_t by = adj_bwd_bytes(P.n, P.k, P.W, sm);
+        auto kern = sm ? k_adj_bwd_warp<true> : k_adj_bwd_warp<false>;
+        if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)by)) return (int)e;
+        kern<<<J.nsamp, 96, by, s>>>(T, P, J, G, ckpt, gshift_part, gscale_part);
+    } else {
+        const size_t lb = (2 * sizeof(double2) + sizeof(double)) * P.n;
+        const int B = lanes_adj(lb);
+        const size_t sm = lb * B;
+        cudaError_t e = cudaFuncSetAttribute(k_adj_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        if (e) return (int)e;
+        k_adj_bwd<<<(nvec + B - 1) / B, B, sm, s>>>(T, P, J, G, ckpt, gshift_part, gscale_part);
+    }
     k_adj_reduce<<<(P.n + 127) / 128, 128, 0, s>>>(gshift_part, nvec, P.n, gshift);
     k_adj_reduce<<<1, 1, 0, s>>>(gscale_part, nvec, 1, gscale);
     return (int)cudaGetLastError();
@@ -569,11 +864,50 @@ struct AdjRun {
     std::vector<double2> S;  // response sums (tmax)
 };
 
+// Schedules of the warp kernels.
+struct AdjSched {
+    DevBuf<uint32_t> s1, sW, parts;
+    DevBuf<int> iso;
+    int build(nise_ctx *c, const std::vector<int2> &pairs, AdjPlan &P) {
+        // one vector's state, its adjoint and gradient on a warp of three: up
+        // to 1600 sites; above, a thread per vector
+        P.W = 1;
+        if (P.n > NISE_SCHED_MAX_N || P.k > NISE_SCHED_MAX_K || adj_bwd_bytes(P.n, P.k, 1, false) > 220 * 1024 || P.ts < 1)
+            return NISE_OK;
+        std::vector<uint32_t> r1, rW, pt;
+        std::vector<int> is;
+        nise_step_schedule(pairs, P.n, P.ts, 1, r1);
+        nise_schedule_parts(pairs, P.n, pt, is);
+        P.nrow1 = (int)(r1.size() / 32);
+        // a window of four steps while one step's rows leave most lanes idle
+        // (a 256-site chain: 263 rows of 5 rotations per step, 293 of 17 per
+        // four) and its coefficients fit beside another CTA's
+        const int W = 4;
+        const bool narrow = (size_t)P.k * P.ts < 12 * (size_t)P.nrow1;
+        if (narrow && std::max(adj_fwd_bytes(P.n, P.k, W, true), adj_bwd_bytes(P.n, P.k, W, true)) <= kAdjShared) {
+            P.W = W;
+            nise_step_schedule(pairs, P.n, P.ts, W, rW);
+        } else {
+            rW = r1;
+        }
+        P.nrowW = (int)(rW.size() / 32);
+        P.niso = (int)is.size();
+        int rc;
+        if ((rc = s1.upload(c, r1)) || (rc = sW.upload(c, rW)) || (rc = parts.upload(c, pt)) || (rc = iso.upload(c, is)))
+            return rc;
+        P.sched1 = s1.p;
+        P.schedW = sW.p;
+        P.parts = parts.p;
+        P.iso = iso.p;
+        return NISE_OK;
+    }
+};
+
 // FP64 forward of the model; leaves the tables and checkpoints in the
 // caller's buffers for the backward sweep.
 int adj_forward(nise_ctx *c, const double *shift, double scale, int K, AdjRun &R, DevBuf<double> &dshift,
                 DevBuf<int2> &dpairs, DevBuf<double2> &U, DevBuf<double2> &rot, DevBuf<double> &jf,
-                DevBuf<double2> &ckpt, AdjPlan &P, AbsJob &J) {
+                DevBuf<double2> &ckpt, AdjSched &Q, AdjPlan &P, AbsJob &J) {
     const nise_params &p = c->p;
     if (!c->loaded) return nise_fail(c, NISE_ERR_STATE, "no trajectory loaded");
     if (!shift || !(scale == scale)) return nise_fail(c, NISE_ERR_ARG, "null shifts or invalid scale");
@@ -612,6 +946,7 @@ int adj_forward(nise_ctx *c, const double *shift, double scale, int K, AdjRun &R
     P.U = U.p;
     P.rot = rot.p;
     P.jf = jf.p;
+    if ((rc = Q.build(c, pairs, P))) return rc;
     memset(&J, 0, sizeof(J));
     J.begin = R.begin;
     J.nsamp = R.nsamp;
@@ -833,13 +1168,14 @@ extern "C" int nise_absorption_model(nise_ctx *c, const double *site_shift, doub
     DevBuf<double> dshift, jf;
     DevBuf<int2> dpairs;
     DevBuf<double2> U, rot, ckpt;
+    AdjSched Q;
     AdjPlan P;
     AbsJob J;
     Rk4Work W;
     const int model = adj_model(c);
     if (model < 0) return adj_unsupported(c);
     int rc = model ? adj_rk4_forward(c, site_shift, coupling_scale, 32, model == 2, R, W)
-                   : adj_forward(c, site_shift, coupling_scale, c->p.tmax1, R, dshift, dpairs, U, rot, jf, ckpt, P, J);
+                   : adj_forward(c, site_shift, coupling_scale, c->p.tmax1, R, dshift, dpairs, U, rot, jf, ckpt, Q, P, J);
     if (rc) return rc;
     cudaEventRecord(c->evk1, c->stream);
     cudaEventRecord(c->ev1, c->stream);
@@ -878,6 +1214,7 @@ extern "C" int nise_backward_absorption(nise_ctx *c, const double *site_shift, d
     DevBuf<double> dshift, jf;
     DevBuf<int2> dpairs;
     DevBuf<double2> U, rot, ckpt;
+    AdjSched Q;
     AdjPlan P;
     AbsJob J;
     const int K = 32;  // checkpoint interval (steps)
@@ -886,7 +1223,7 @@ extern "C" int nise_backward_absorption(nise_ctx *c, const double *site_shift, d
     const bool rk4 = model > 0;  // a polynomial model
     Rk4Work W;
     int rc = rk4 ? adj_rk4_forward(c, site_shift, coupling_scale, K, model == 2, R, W)
-                 : adj_forward(c, site_shift, coupling_scale, K, R, dshift, dpairs, U, rot, jf, ckpt, P, J);
+                 : adj_forward(c, site_shift, coupling_scale, K, R, dshift, dpairs, U, rot, jf, ckpt, Q, P, J);
     if (rc) return rc;
     // adjoint of the transform: dL/dOut_k = (dL/dspec_im + i dL/dspec_re) * 2 dt c_v,
     // dL/din_j = sum_k exp(+2 pi i jk/fft) dL/dOut_k, then through the input factors

@@ -210,6 +210,13 @@ struct AdjPlan {
     double scale, f;       // coupling scale, deltat*icm2ifs*2pi/ts
     double2 *U, *rot;
     double *jf;
+    // schedules of one time step and of a window of W (rotsched.h: rows of 32
+    // rotations), the rotations' packed sites and the sites without any; null
+    // above the size of the warp kernels
+    const uint32_t *sched1, *schedW, *parts;
+    int nrow1, nrowW, W;
+    const int *iso;
+    int niso;
 };
 int launch_adj_prep(const DevTraj &T, const AdjPlan &P, cudaStream_t s);
 int launch_adj_fwd(const DevTraj &T, const AdjPlan &P, const AbsJob &J, double2 *resp, double2 *ckpt,

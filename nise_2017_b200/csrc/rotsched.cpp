@@ -1,0 +1,43 @@
+// Schedule of the Trotter rotations of whole time steps (rotsched.h).
+#include "rotsched.h"
+
+#include <algorithm>
+
+int nise_step_schedule(const std::vector<int2> &pairs, int n, int ts, int steps, std::vector<uint32_t> &rows) {
+    const size_t K = pairs.size();
+    std::vector<int> last(n, 0);
+    std::vector<std::vector<uint32_t>> level;
+    for (int w = 0; w < steps; w++)
+        for (int s = 0; s < ts; s++)
+            for (size_t k = 0; k < K; k++) {
+                const int l = std::max(last[pairs[k].x], last[pairs[k].y]);
+                last[pairs[k].x] = last[pairs[k].y] = l + 1;
+                if ((int)level.size() == l) level.emplace_back();
+                level[l].push_back((uint32_t)k | (uint32_t)w << 20 | (uint32_t)(s == 0) << 30 |
+                                   (uint32_t)(s == ts - 1) << 31);
+            }
+    rows.clear();
+    for (const auto &l : level)
+        for (size_t q = 0; q < l.size(); q += 32)
+            for (size_t i = 0; i < 32; i++) rows.push_back(q + i < l.size() ? l[q + i] : NISE_SCHED_NONE);
+    return (int)level.size();
+}
+
+void nise_schedule_parts(const std::vector<int2> &pairs, int n, std::vector<uint32_t> &parts, std::vector<int> &iso) {
+    const int K = (int)pairs.size();
+    std::vector<int> first(n, -1), last(n, -1);
+    for (int k = 0; k < K; k++)
+        for (int a : {pairs[k].x, pairs[k].y}) {
+            if (first[a] < 0) first[a] = k;
+            last[a] = k;
+        }
+    parts.resize(K);
+    for (int k = 0; k < K; k++) {
+        const int a = pairs[k].x, b = pairs[k].y;
+        parts[k] = (uint32_t)a | (uint32_t)b << 14 | (uint32_t)(first[a] == k) << 28 | (uint32_t)(first[b] == k) << 29 |
+                   (uint32_t)(last[a] == k) << 30 | (uint32_t)(last[b] == k) << 31;
+    }
+    iso.clear();
+    for (int a = 0; a < n; a++)
+        if (first[a] < 0) iso.push_back(a);
+}

@@ -1,0 +1,41 @@
+// Schedule of the Trotter rotations of whole time steps (host only).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <vector>
+
+// One rotation of a schedule: which one (q, an index into the coupling list),
+// in which time step of the window (w), and whether that is the first or the
+// last sub-step of its time step.
+#define NISE_SCHED_Q(e) ((e) & 0xfffffu)
+#define NISE_SCHED_W(e) (((e) >> 20) & 0xfu)
+#define NISE_SCHED_FIRST(e) (((e) >> 30) & 1u)
+#define NISE_SCHED_LAST(e) ((e) >> 31)
+#define NISE_SCHED_NONE 0xfffffu
+#define NISE_SCHED_MAX_K 0xfffff
+
+// Rotation q's sites and its part in a sub-step: whether it is the first
+// (PRE) or the last (POST) to touch its first (A) or second (B) site.  The
+// half-step phase of a site belongs before its first and after its last
+// rotation of every sub-step (propagate.c:870-894).
+#define NISE_SCHED_A(p) ((p) & 0x3fffu)
+#define NISE_SCHED_B(p) (((p) >> 14) & 0x3fffu)
+#define NISE_SCHED_PRE_A(p) (((p) >> 28) & 1u)
+#define NISE_SCHED_PRE_B(p) (((p) >> 29) & 1u)
+#define NISE_SCHED_POST_A(p) (((p) >> 30) & 1u)
+#define NISE_SCHED_POST_B(p) ((p) >> 31)
+#define NISE_SCHED_MAX_N 0x3fff
+
+// The rotations of `steps` time steps of `ts` sub-steps each, in rows of 32
+// (one warp step each; NISE_SCHED_NONE fills a row up).  A rotation's level is
+// 1 + the highest level of the earlier ones that share a site with it, across
+// sub-step and step boundaries, so rotations that share a site keep the order
+// of propagate.c:876-888 and a row's rotations are disjoint.  A coupling list
+// with few disjoint neighbours (a chain: one rotation per level of a sub-step)
+// runs its sub-steps as a wavefront: n + 2 (ts steps - 1) levels instead of
+// n ts steps.  Returns the levels.
+int nise_step_schedule(const std::vector<int2> &pairs, int n, int ts, int steps, std::vector<uint32_t> &rows);
+// The packed sites and parts of every rotation; iso: the sites that no
+// rotation touches.
+void nise_schedule_parts(const std::vector<int2> &pairs, int n, std::vector<uint32_t> &parts, std::vector<int> &iso);
