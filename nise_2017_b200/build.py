@@ -38,6 +38,7 @@ CU_SOURCES = [
     "eigen_large.cu",
     "dia_tc.cu",
     "rk4.cu",
+    "propagators.cu",
 ]
 CPP_SOURCES = [
     "api.cpp",

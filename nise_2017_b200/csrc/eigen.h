@@ -31,3 +31,17 @@ int launch_eig_any(const EigJob &J, const long *frames_dev, long nframes, double
 // dropped when truncate), for the layout of launch_eig_any.
 int launch_build_u_any(int prec, const double *V, const double *w, long nfr, int n, double f, float thres,
                        int truncate, void *U, cudaStream_t s);
+
+// exp(-i H f) of the frames [f0, f0 + nfr) without eigenvectors
+// (propagators.cu), any n: U[t][a][c] in working precision (prec 0 FP32, 1
+// FP64), exactly symmetric, |U|^2 <= thres dropped when truncate; ws holds
+// propagator_ws_doubles(n, nfr) doubles.
+struct PropJob {
+    DevTraj T;
+    int n, singleshift, truncate;
+    long f0, nfr;
+    double f;
+    float thres;
+};
+size_t propagator_ws_doubles(int n, long frames);
+int launch_propagators(int prec, const PropJob &P, void *U, double *ws, cudaStream_t s);
