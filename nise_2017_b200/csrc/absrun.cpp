@@ -294,6 +294,7 @@ struct AbsRun {
     DevBuf<int> estatus;
     DevBuf<float> tcX;           // state columns of the tensor-core apply
     bool use_tc = false;
+    bool tc_starts = false; // its form with all start points in step
     bool stream_u = false;  // propagators built and applied chunk by chunk (tensor cores, batched)
     long FC = 1;
     bool truncated = false;
@@ -483,12 +484,15 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
             if (plain) Jt.nsamp = 1;
             use_tc = prec == NISE_FP32 && tc_dia_fits(Jt, N) &&
                      (p.kernel_config == 17 || (N > NISE_EIG_MAX_N && p.kernel_config != 16));
-            stream_u = use_tc && !plain;
-            if (N > (stream_u ? 2048 : 1024))
+            // all start points in step where every propagator can be held (8 GB)
+            tc_starts = use_tc && !plain && N <= 1024 && tc_dia_starts_pays(J, N, nf) &&
+                        r2 * (size_t)nf * N * N <= ((size_t)8 << 30);
+            stream_u = use_tc && !plain && !tc_starts;
+            if (N > (stream_u || tc_starts ? 2048 : 1024))
                 return nise_fail(c, NISE_ERR_UNSUPPORTED,
                                  "the eigen route (Threshold > 0, per-frame couplings, kernel_config 2) is limited to "
                                  "%d sites here (2048 with the tensor-core apply of a batched FP32 job)",
-                                 stream_u ? 2048 : 1024);
+                                 stream_u || tc_starts ? 2048 : 1024);
             // frames per eigensolver launch (one CTA per frame): a wave of
             // the 148 SMs, or as many as 1 GB of eigenvectors, QR workspace
             // (and streamed U) holds, at most 16 GB
@@ -515,7 +519,8 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
             }
             // propagate_vec_DIA: f = deltat*icm2ifs*twoPi*sign in float, one full step
             fe = prec == NISE_FP32 ? (double)J.f32_full : J.f;
-            if (use_tc && ((rc = tcX.alloc(c, (size_t)4 * tc_dia_columns(Jt) * N)) || (rc = derr.alloc(c, 1))))
+            const size_t cols = tc_starts ? (size_t)16 * nsamp : (size_t)tc_dia_columns(Jt);
+            if (use_tc && ((rc = tcX.alloc(c, 4 * cols * N)) || (rc = derr.alloc(c, 1))))
                 return rc;
             if (use_tc) cudaMemsetAsync(derr.p, 0, sizeof(int), c->stream);
         } else {
@@ -925,6 +930,7 @@ int AbsRun::run_main(cudaStream_t s, int cfg, double2 *dst) {
                 }
                 return er;
             }
+            if (tc_starts) return launch_abs_dia_tc_starts(T, Ue.p, f0, N, Js, r, tcX.p, derr.p, s);
             if (use_tc) return launch_abs_dia_tc(T, Ue.p, f0, N, Js, r, tcX.p, derr.p, s);
             return launch_abs_dia(pr, T, Ue.p, f0, N, Js, r, s);
         }

@@ -126,21 +126,11 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *m, uint32_t parity) 
     return false;
 }
 
-// Per-frame start and response: CTA per column of X (block 256 threads).
-// X planes: xr, xi [cols][n].
-__global__ void __launch_bounds__(256) k_tc_resp(DevTraj T, AbsJob J, int n, long t, int slots, float *xr, float *xi,
-                                                 double2 *resp) {
+// Start and response of vector (q, x) at frame t, t1 steps after its start:
+// one CTA of 256 threads; pr, pi its column of X.
+__device__ void tc_resp(const DevTraj &T, int n, long t, long t1, int tmax, long q, int x, float *pr, float *pi,
+                        double2 *resp) {
     __shared__ double red[2][8];
-    const int col = blockIdx.x, slot = col / 3, x = col % 3;
-    // the start point of this slot active on frame t, if any
-    const long tfirst = (long)J.begin * J.sample;
-    const long rel = t - tfirst;                 // frames since the first start
-    long q = rel / J.sample;                     // latest start point (relative) at or before t
-    q -= ((q % slots) - slot + slots) % slots;   // the latest one using this slot
-    if (q < 0 || q >= J.nsamp) return;
-    const long t1 = rel - q * J.sample;
-    if (t1 < 0 || t1 >= J.tmax) return;
-    float *pr = xr + (size_t)col * n, *pi = xi + (size_t)col * n;
     double re = 0, im = 0;
     for (int a = threadIdx.x; a < n; a += 256) {
         const float m = traj_mu(T, t, x, a);
@@ -167,18 +157,53 @@ __global__ void __launch_bounds__(256) k_tc_resp(DevTraj T, AbsJob J, int n, lon
             sr += red[0][w];
             si += red[1][w];
         }
-        resp[(size_t)(3 * q + x) * J.tmax + t1] = make_double2(sr, si);
+        resp[(size_t)(3 * q + x) * tmax + t1] = make_double2(sr, si);
     }
+}
+
+// Per-frame start and response: CTA per column of X (block 256 threads).
+// X planes: xr, xi [cols][n].
+__global__ void __launch_bounds__(256) k_tc_resp(DevTraj T, AbsJob J, int n, long t, int slots, float *xr, float *xi,
+                                                 double2 *resp) {
+    const int col = blockIdx.x, slot = col / 3, x = col % 3;
+    // the start point of this slot active on frame t, if any
+    const long tfirst = (long)J.begin * J.sample;
+    const long rel = t - tfirst;                 // frames since the first start
+    long q = rel / J.sample;                     // latest start point (relative) at or before t
+    q -= ((q % slots) - slot + slots) % slots;   // the latest one using this slot
+    if (q < 0 || q >= J.nsamp) return;
+    const long t1 = rel - q * J.sample;
+    if (t1 < 0 || t1 >= J.tmax) return;
+    tc_resp(T, n, t, t1, J.tmax, q, x, xr + (size_t)col * n, xi + (size_t)col * n, resp);
+}
+
+// The same with every start point at its own step t1: CTA per vector, start
+// point q's three columns at 16 q.
+__global__ void __launch_bounds__(256) k_tc_resp_starts(DevTraj T, AbsJob J, int n, int t1, float *xr, float *xi,
+                                                        double2 *resp) {
+    const int q = blockIdx.x / 3, x = blockIdx.x % 3;
+    const size_t col = (16 * (size_t)q + x) * n;
+    tc_resp(T, n, (long)(J.begin + q) * J.sample + t1, t1, J.tmax, q, x, xr + col, xi + col, resp);
 }
 
 // Y = U_t X for 128 rows per CTA; NC columns (a multiple of 16, <= 64).
 // Shared-memory tiles (1024-byte aligned, 128-byte swizzled rows of 32
 // tf32): A[c][p] = piece p of U_c (c = 0 real, 1 imaginary) for the CTA's 128
 // rows, B[c][p] = piece p of X_c for the NC columns, sites c0 .. c0 + 31.
+// The grid's second axis takes independent sets of columns, each NC x n
+// further in every plane, with propagators us further on.
 template <int NC>
 __global__ void __launch_bounds__(kTcThreads, 1)
-    k_tc_apply(const float2 *__restrict__ U, int n, const float *__restrict__ xr, const float *__restrict__ xi,
-               float *__restrict__ yr, float *__restrict__ yi, int *err) {
+    k_tc_apply(const float2 *__restrict__ U, size_t us, int n, const float *__restrict__ xr,
+               const float *__restrict__ xi, float *__restrict__ yr, float *__restrict__ yi, int *err) {
+    U += blockIdx.y * us;
+    {
+        const size_t off = blockIdx.y * (size_t)NC * n;
+        xr += off;
+        xi += off;
+        yr += off;
+        yi += off;
+    }
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *base = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     constexpr size_t kA = (size_t)kTcRows * 128, kB = (size_t)NC * 128;
@@ -334,11 +359,11 @@ size_t tc_apply_smem() {
 
 template <int NC>
 int run_tc_apply(const float2 *U, int n, const float *xr, const float *xi, float *yr, float *yi, int *err,
-                 cudaStream_t s) {
+                 cudaStream_t s, int sets = 1, size_t us = 0) {
     const size_t sm = tc_apply_smem<NC>();
     cudaError_t e = cudaFuncSetAttribute(k_tc_apply<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
     if (e != cudaSuccess) return (int)e;
-    k_tc_apply<NC><<<(n + kTcRows - 1) / kTcRows, kTcThreads, sm, s>>>(U, n, xr, xi, yr, yi, err);
+    k_tc_apply<NC><<<dim3((n + kTcRows - 1) / kTcRows, sets), kTcThreads, sm, s>>>(U, us, n, xr, xi, yr, yi, err);
     return (int)cudaGetLastError();
 }
 
@@ -392,6 +417,38 @@ int launch_abs_dia_tc_frames(const DevTraj &T, const void *U, long ufirst, int n
         case 48: rc = run_tc_apply<48>(Ut, n, cr, ci, nr, ni, err, s); break;
         default: rc = run_tc_apply<64>(Ut, n, cr, ci, nr, ni, err, s); break;
         }
+        if (rc) return rc;
+        std::swap(cr, nr);
+        std::swap(ci, ni);
+    }
+    return (int)cudaGetLastError();
+}
+
+// All start points step together, each through its own frames, with every
+// frame's propagator in U: tmax - 1 launches of (row tiles x start points) CTAs
+// instead of one launch of the row tiles per frame.  A column's arithmetic does
+// not depend on the other columns, so the responses are those of the
+// frame-by-frame form.  It reads a propagator once per start point that crosses
+// it, so it pays while its rounds of CTAs are fewer than the frames (200 sites,
+// 595 frames, 51 start points of 96 steps: frame by frame 595 x 68 us, 2 CTAs
+// at a time, 40.2 ms; now 95 x 69 us, 102 CTAs, 6.6 ms).  X holds 4 planes of 16 nsamp columns.
+bool tc_dia_starts_pays(const AbsJob &J, int n, long nf) {
+    const long ctas = (long)J.nsamp * ((n + kTcRows - 1) / kTcRows), sms = sm_count();
+    return J.nsamp <= 65535 && (J.tmax - 1) * ((ctas + sms - 1) / sms) < nf;
+}
+
+int launch_abs_dia_tc_starts(const DevTraj &T, const void *U, long f0, int n, const AbsJob &J, double2 *resp, float *X,
+                             int *err, cudaStream_t s) {
+    if (J.nsamp <= 0) return 0;
+    const size_t plane = (size_t)16 * J.nsamp * n;
+    cudaError_t e = cudaMemsetAsync(X, 0, sizeof(float) * 4 * plane, s);
+    if (e != cudaSuccess) return (int)e;
+    float *cr = X, *ci = cr + plane, *nr = ci + plane, *ni = nr + plane;
+    for (int t1 = 0; t1 < J.tmax; t1++) {
+        k_tc_resp_starts<<<3 * J.nsamp, 256, 0, s>>>(T, J, n, t1, cr, ci, resp);
+        if (t1 == J.tmax - 1) break;
+        const float2 *Ut = (const float2 *)U + (size_t)((long)J.begin * J.sample + t1 - f0) * n * n;
+        const int rc = run_tc_apply<16>(Ut, n, cr, ci, nr, ni, err, s, J.nsamp, (size_t)J.sample * n * n);
         if (rc) return rc;
         std::swap(cr, nr);
         std::swap(ci, ni);

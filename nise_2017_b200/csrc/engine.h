@@ -191,6 +191,11 @@ long tc_dia_first_frame(const AbsJob &J);
 long tc_dia_last_frame(const AbsJob &J);
 int launch_abs_dia_tc(const DevTraj &T, const void *U, long f0, int n, const AbsJob &J, double2 *resp, float *X,
                       int *err, cudaStream_t s);
+// All start points in step (16 columns of X each) with every propagator in U,
+// and whether that is the faster form.
+bool tc_dia_starts_pays(const AbsJob &J, int n, long nf);
+int launch_abs_dia_tc_starts(const DevTraj &T, const void *U, long f0, int n, const AbsJob &J, double2 *resp, float *X,
+                             int *err, cudaStream_t s);
 int launch_abs_dia_tc_frames(const DevTraj &T, const void *U, long ufirst, int n, const AbsJob &J, double2 *resp,
                              float *X, int *err, long ta, long tb, cudaStream_t s);
 // Linear absorption of the start points of J with the per-frame propagators
