@@ -12,6 +12,8 @@
 // the same test in the working precision, and shared by every start point
 // and polarisation that crosses the frame.  U is complex symmetric (V is
 // real orthogonal), so it is stored once and read along rows.
+#include <algorithm>
+
 #include "common.cuh"
 #include "engine.h"
 
@@ -69,77 +71,107 @@ __global__ void k_build_u(const double *V, const double *w, int n, double f, flo
 }
 
 // Linear absorption with per-frame propagators: CTA per start point, its
-// three polarisation vectors in shared memory, thread a owns site a.  The
-// response is taken before each step (absorption.c:119-145): float products,
-// double sums over sites (warp shuffles, then warps in order).  The step is
+// three polarisation vectors in shared memory.  The response is taken before
+// each step (absorption.c:119-145): float products, double sums.  The step is
 // c_a <- sum_b U_ab c_b in site order b, the reference's float accumulation
-// (propagate.c:109-119) in FP32 mode.
-template <typename R>
-__global__ void k_abs_dia(DevTraj T, const typename Vec2<R>::T *__restrict__ U, long f0, int n, AbsJob J,
-                          double2 *resp) {
+// (propagate.c:109-119) in FP32 mode, so its parallelism is rows x vectors: a
+// thread per row of VX vectors (one each while 3 n threads and three warps for
+// the responses fit a CTA, else all three).  Where two U_t fit shared memory
+// (STAGE) the next one is copied asynchronously while the sums run.  Bound by
+// the chain of a row's additions and the issue of its few warps.  48 sites, 94
+// start points, RunTimes 128: 1756 us with 64 threads that fetched U when
+// needed, 175 us now (216 with the sums split over 19 groups of rows: the
+// barriers of 1024 threads cost more than the shorter chains save, and another
+// rounding).
+template <typename R, int VX, bool STAGE>
+__global__ void __launch_bounds__(1024) k_abs_dia(DevTraj T, const typename Vec2<R>::T *__restrict__ U, long f0, int n,
+                                                  int rw, AbsJob J, double2 *resp) {
     typedef typename Vec2<R>::T R2;
     typedef Ar<R> A;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int a = threadIdx.x, lane = a & 31, warp = a >> 5, NW = blockDim.x >> 5;
-    double2 *red = (double2 *)smem_raw;          // [3][warps]
-    R2 *C = (R2 *)(red + 3 * NW);                // [3][n]
+    R2 *C = (R2 *)smem_raw, *D = C + 3 * n, *Us = D + 3 * n;  // [3][n] twice; [2][n][n] (STAGE)
+    const int work = VX == 1 ? 3 * n : n, a = threadIdx.x % n, x0 = VX == 1 ? threadIdx.x / n : 0, lane = threadIdx.x & 31;
+    const int x = (int)(threadIdx.x >> 5) - rw;  // the response warps: x = 0, 1, 2
+    const bool act = (int)threadIdx.x < work;
+    const size_t nn = (size_t)n * n;
     const int sl = blockIdx.x;
     const long ti = (long)(J.begin + sl) * J.sample;
-    for (int x = 0; x < 3; x++)
-        if (a < n) {
-            R2 z;
-            z.x = (R)traj_mu(T, ti, x, a);
-            z.y = 0;
-            C[x * n + a] = z;
-        }
-    __syncthreads();
+    const R2 *Ut = U + (size_t)(ti - f0) * nn;
+    for (int e = threadIdx.x; e < 3 * n; e += blockDim.x) {
+        C[e].x = (R)traj_mu(T, ti, e / n, e % n);
+        C[e].y = 0;
+    }
+    auto stage = [&](int t1) {
+        if (t1 < J.tmax - 1)
+            for (int e = threadIdx.x; e < (int)nn; e += blockDim.x)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                                 (uint32_t)__cvta_generic_to_shared(Us + (t1 & 1) * nn + e)),
+                             "l"(Ut + (size_t)t1 * nn + e), "n"(sizeof(R2)));
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (STAGE) stage(0);
     for (int t1 = 0; t1 < J.tmax; t1++) {
-        const long t = ti + t1;
-        for (int x = 0; x < 3; x++) {
+        if (STAGE) asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // U_t1 staged, C complete
+        if (STAGE) stage(t1 + 1);
+        if (x >= 0 && x < 3) {
+            const long t = ti + t1;
             double re = 0, im = 0;
-            if (a < n) {
-                R m = (R)traj_mu(T, t, x, a);
-                R2 z = C[x * n + a];
-                re = (double)A::mul(m, z.x);
-                im = (double)A::mul(m, z.y);
+            for (int i = lane; i < n; i += 32) {
+                const R m = (R)traj_mu(T, t, x, i);
+                re += (double)A::mul(m, C[x * n + i].x);
+                im += (double)A::mul(m, C[x * n + i].y);
             }
             for (int o = 16; o > 0; o >>= 1) {
                 re += __shfl_xor_sync(0xffffffffu, re, o);
                 im += __shfl_xor_sync(0xffffffffu, im, o);
             }
-            if (lane == 0) red[x * NW + warp] = make_double2(re, im);
-        }
-        __syncthreads();
-        if (a < 3) {
-            double sr = 0, si = 0;
-            for (int w = 0; w < NW; w++) {
-                sr += red[a * NW + w].x;
-                si += red[a * NW + w].y;
-            }
-            resp[(size_t)(3 * sl + a) * J.tmax + t1] = make_double2(sr, si);
+            if (lane == 0) resp[(size_t)(3 * sl + x) * J.tmax + t1] = make_double2(re, im);
         }
         if (t1 == J.tmax - 1) break;
-        R2 acc[3];
-        for (int x = 0; x < 3; x++) acc[x].x = acc[x].y = 0;
-        if (a < n) {
-            const R2 *Ut = U + (size_t)(t - f0) * n * n;
-            for (int b = 0; b < n; b++) {
-                R2 u = Ut[(size_t)b * n + a];  // = U[a][b]
+        if (act) {
+            const R2 *Ua = (STAGE ? Us + (t1 & 1) * nn : Ut + (size_t)t1 * nn) + a;
+            R2 acc[VX];
 #pragma unroll
-                for (int x = 0; x < 3; x++) {
-                    R2 z = C[x * n + b];
-                    acc[x].x = A::add(acc[x].x, A::sub(A::mul(u.x, z.x), A::mul(u.y, z.y)));
-                    acc[x].y = A::add(acc[x].y, A::add(A::mul(u.x, z.y), A::mul(u.y, z.x)));
+            for (int q = 0; q < VX; q++) acc[q].x = acc[q].y = 0;
+#pragma unroll 8
+            for (int b = 0; b < n; b++) {
+                const R2 u = Ua[(size_t)b * n];  // = U[a][b]
+#pragma unroll
+                for (int q = 0; q < VX; q++) {
+                    const R2 z = C[(x0 + q) * n + b];
+                    acc[q].x = A::add(acc[q].x, A::sub(A::mul(u.x, z.x), A::mul(u.y, z.y)));
+                    acc[q].y = A::add(acc[q].y, A::add(A::mul(u.x, z.y), A::mul(u.y, z.x)));
                 }
             }
+#pragma unroll
+            for (int q = 0; q < VX; q++) D[(x0 + q) * n + a] = acc[q];
         }
-        __syncthreads();
-        if (a < n)
-            for (int x = 0; x < 3; x++) C[x * n + a] = acc[x];
-        __syncthreads();
+        R2 *sw = C;
+        C = D;
+        D = sw;
     }
 }
 
+}  // namespace
+
+namespace {
+template <typename R>
+int run_abs_dia(const DevTraj &T, const typename Vec2<R>::T *U, long f0, int n, const AbsJob &J, double2 *resp,
+                cudaStream_t s) {
+    const bool one = 3 * n <= 928;  // a vector per thread
+    const int work = ((one ? 3 * n : n) + 31) / 32 * 32;
+    const bool own = work + 96 <= 1024;  // above 928 sites the first three warps take the responses too
+    const int threads = own ? work + 96 : work;
+    const size_t base = sizeof(typename Vec2<R>::T) * 6 * (size_t)n, all = base + sizeof(typename Vec2<R>::T) * 2 * n * n;
+    const bool stage = one && all <= 227 * 1024;
+    const size_t sm = stage ? all : base;
+    auto kern = stage ? k_abs_dia<R, 1, true> : one ? k_abs_dia<R, 1, false> : k_abs_dia<R, 3, false>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return (int)e;
+    kern<<<J.nsamp, threads, sm, s>>>(T, U, f0, n, own ? work / 32 : 0, J, resp);
+    return (int)cudaGetLastError();
+}
 }  // namespace
 
 size_t dia_build_smem(int n) { return sizeof(double) * ((size_t)n * n + 2 * n); }
@@ -164,19 +196,7 @@ int launch_build_u(int prec, const double *V, const double *w, long nfr, int n, 
 int launch_abs_dia(int prec, const DevTraj &T, const void *U, long f0, int n, const AbsJob &J, double2 *resp,
                    cudaStream_t s) {
     if (J.nsamp <= 0) return 0;
-    const int threads = ((n + 31) / 32) * 32;
-    const int nw = threads / 32;
-    if (threads > 1024) return (int)cudaErrorNotSupported;
-    if (prec == 0) {
-        size_t sm = sizeof(float2) * 3 * n + sizeof(double2) * 3 * nw;
-        cudaError_t e = cudaFuncSetAttribute(k_abs_dia<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return (int)e;
-        k_abs_dia<float><<<J.nsamp, threads, sm, s>>>(T, (const float2 *)U, f0, n, J, resp);
-    } else {
-        size_t sm = sizeof(double2) * 3 * n + sizeof(double2) * 3 * nw;
-        cudaError_t e = cudaFuncSetAttribute(k_abs_dia<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e != cudaSuccess) return (int)e;
-        k_abs_dia<double><<<J.nsamp, threads, sm, s>>>(T, (const double2 *)U, f0, n, J, resp);
-    }
-    return (int)cudaGetLastError();
+    if (n > 1024) return (int)cudaErrorNotSupported;
+    return prec == 0 ? run_abs_dia<float>(T, (const float2 *)U, f0, n, J, resp, s)
+                     : run_abs_dia<double>(T, (const double2 *)U, f0, n, J, resp, s);
 }

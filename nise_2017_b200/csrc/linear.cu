@@ -186,22 +186,90 @@ __device__ __forceinline__ double lin_weight(int tech, int ch, int v, int r) {
     }
 }
 
-// out[ch][t1] (+)= sum over start points, vectors and read-outs, in order.
-__global__ void k_lin_reduce(const double2 *part, int S, int nvec, int nread, int tmax, int tech, int nch,
-                             double2 *out, int first) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= nch * tmax) return;
-    const int ch = g / tmax, t1 = g % tmax;
-    double re = 0, im = 0;
-    for (int s = 0; s < S; s++)
-        for (int v = 0; v < nvec; v++)
-            for (int r = 0; r < nread; r++) {
-                const double w = lin_weight(tech, ch, v, r);
-                if (w == 0.0) continue;
-                double2 z = part[(((size_t)s * nvec + v) * nread + r) * tmax + t1];
-                re += w * z.x;
-                im += w * z.y;
+// The same for Sparse/Diagonal (propagate_vec_DIA, propagate.c:109-119): every
+// vector of a start point is multiplied by the same U_t, so a CTA takes VG of
+// them as the columns of X and a thread the row a of four columns: c_a <- sum_b
+// U_ab c_b in site order, the operations of dia_apply (U is symmetric: its rows
+// are read as columns, contiguous over the lanes), with 16 of them per element
+// of U.  nr more threads take the read-outs of the same X meanwhile.  Bound by
+// the latency of the sums over b.  CD on 40 sites in FP64 (21 start points, 120
+// vectors each, RunTimes 64): 8950 us with a thread per vector (40 CTAs), now
+// 976 us.
+template <typename R>
+__global__ void __launch_bounds__(1024) k_lin_dia(LinJob J, int VG, int nr) {
+    typedef typename Vec2<R>::T R2;
+    typedef Ar<R> A;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int n = J.n, groups = (J.nvec + VG - 1) / VG, s = blockIdx.x / groups, v0 = (blockIdx.x % groups) * VG;
+    const int nw = blockDim.x - nr, tid = threadIdx.x, tiles = n * (VG / 4);
+    R2 *X = (R2 *)smem_raw, *Y = X + (size_t)n * VG;  // [n][VG]
+    const long ti = (long)(J.begin + s) * J.sample;
+    for (int e = tid; e < n * VG; e += blockDim.x) {
+        const int v = v0 + e % VG;
+        X[e].x = v < J.nvec ? (R)lin_init(J, s, v, ti, e / VG) : (R)0;
+        X[e].y = 0;
+    }
+    __syncthreads();
+    for (int t1 = 0; t1 < J.tmax; t1++) {
+        const long tj = ti + t1;
+        if (tid >= nw) {
+            for (int e = tid - nw; e < VG * J.nread; e += nr) {
+                const int q = e % VG, r = e / VG, v = v0 + q;
+                if (v < J.nvec)
+                    J.part[(((size_t)s * J.nvec + v) * J.nread + r) * J.tmax + t1] = lin_read<R>(J, v, r, tj, X, VG, q);
             }
+        } else if (t1 < J.tmax - 1) {
+            const R2 *U = (const R2 *)J.Ud + (size_t)(tj - J.f0) * n * n;
+            for (int e = tid; e < tiles; e += nw) {
+                const int a = e % n, q0 = e / n * 4;
+                R2 acc[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) acc[q].x = acc[q].y = 0;
+#pragma unroll 8
+                for (int b = 0; b < n; b++) {
+                    const R2 u = U[(size_t)b * n + a];  // = U[a][b]
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const R2 z = X[b * VG + q0 + q];
+                        acc[q].x = A::add(acc[q].x, A::sub(A::mul(u.x, z.x), A::mul(u.y, z.y)));
+                        acc[q].y = A::add(acc[q].y, A::add(A::mul(u.x, z.y), A::mul(u.y, z.x)));
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < 4; q++) Y[a * VG + q0 + q] = acc[q];
+            }
+        }
+        __syncthreads();
+        R2 *sw = X;
+        X = Y;
+        Y = sw;
+    }
+}
+
+// out[ch][t1] (+)= sum over start points, vectors and read-outs: 32 rows of
+// threads over the terms (a warp's loads are contiguous in t1), then the rows
+// in order.
+__global__ void __launch_bounds__(1024) k_lin_reduce(const double2 *part, int S, int nvec, int nread, int tmax,
+                                                     int tech, int nch, double2 *out, int first) {
+    __shared__ double2 red[32][32];
+    const int t1 = blockIdx.x * 32 + threadIdx.x, ch = blockIdx.y, terms = S * nvec * nread;
+    double re = 0, im = 0;
+    if (t1 < tmax)
+        for (int e = threadIdx.y; e < terms; e += 32) {
+            const double w = lin_weight(tech, ch, e / nread % nvec, e % nread);
+            if (w == 0.0) continue;
+            const double2 z = part[(size_t)e * tmax + t1];
+            re += w * z.x;
+            im += w * z.y;
+        }
+    red[threadIdx.y][threadIdx.x] = make_double2(re, im);
+    __syncthreads();
+    if (threadIdx.y || t1 >= tmax) return;
+    for (int q = 1; q < 32; q++) {
+        re += red[q][threadIdx.x].x;
+        im += red[q][threadIdx.x].y;
+    }
+    const int g = ch * tmax + t1;
     if (first) out[g] = make_double2(re, im);
     else out[g] = make_double2(out[g].x + re, out[g].y + im);
 }
@@ -330,18 +398,31 @@ __global__ void k_lum_itime(DevTraj T, DevTraj T0, int n, int sample, int begin,
 
 template <typename R>
 int run_lin(const LinJob &J, double2 *out, int nch, int first, cudaStream_t st) {
-    size_t lane_b = singles_lane_bytes<R>(J.n, J.prop);
-    int B = 64;
-    while (B > 1 && (size_t)B * lane_b > 200 * 1024) B >>= 1;
-    size_t sm = lane_b * B;
+    const long nv = (long)J.S * J.nvec;
     int e;
-    if (sm > 48 * 1024 &&
-        (e = (int)cudaFuncSetAttribute(k_lin<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)))
-        return e;
-    long nv = (long)J.S * J.nvec;
-    k_lin<R><<<(unsigned)((nv + B - 1) / B), B, sm, st>>>(J);
-    int tot = nch * J.tmax;
-    k_lin_reduce<<<(tot + 127) / 128, 128, 0, st>>>(J.part, J.S, J.nvec, J.nread, J.tmax, J.tech, nch, out, first);
+    if (is_eigen_scheme(J.prop)) {
+        // columns per CTA: all of a start point's vectors, fewer where that
+        // leaves SMs without two CTAs
+        const size_t row = sizeof(typename Vec2<R>::T) * 2 * (size_t)J.n;
+        int VG = (int)std::min<long>(std::min(64, (J.nvec + 3) / 4 * 4), std::max<long>(4, nv / (2 * sm_count()) / 4 * 4));
+        while (VG > 4 && VG * row > 200 * 1024) VG -= 4;
+        const int tiles = J.n * (VG / 4), nr = (VG * J.nread + 31) / 32 * 32, nw = std::min((tiles + 31) / 32 * 32, 768);
+        if ((e = (int)cudaFuncSetAttribute(k_lin_dia<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(VG * row))))
+            return e;
+        k_lin_dia<R><<<(unsigned)(J.S * ((J.nvec + VG - 1) / VG)), nw + nr, VG * row, st>>>(J, VG, nr);
+    } else {
+        size_t lane_b = singles_lane_bytes<R>(J.n, J.prop);
+        int B = 64;
+        while (B > 1 && (size_t)B * lane_b > 200 * 1024) B >>= 1;
+        size_t sm = lane_b * B;
+        if (sm > 48 * 1024 &&
+            (e = (int)cudaFuncSetAttribute(k_lin<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)))
+            return e;
+        k_lin<R><<<(unsigned)((nv + B - 1) / B), B, sm, st>>>(J);
+    }
+    if ((e = (int)cudaGetLastError())) return e;
+    k_lin_reduce<<<dim3((J.tmax + 31) / 32, nch), dim3(32, 32), 0, st>>>(J.part, J.S, J.nvec, J.nread, J.tmax, J.tech,
+                                                                        nch, out, first);
     return (int)cudaGetLastError();
 }
 
