@@ -827,6 +827,354 @@ __global__ void __launch_bounds__(768, 1) k2d_doubles_duo(TwoD D, int vec_per_sa
     }
 }
 
+// Which vector of a start point: u < 9 -> fr for (p1,p2) = (u/3, u%3); else
+// ft1[t1] for (p0,p2).
+struct DblVec { int kind, pa, p2, t1; };
+__device__ __forceinline__ DblVec dbl_vec(int u, int T1) {
+    if (u < 9) return {0, u / 3, u % 3, 0};
+    const int w = u - 9, cmb = w / T1;
+    return {1, cmb / 3, cmb % 3, w % T1};
+}
+
+// Two single-precision operations per instruction, each rounded by itself.
+// The assembler contracts a two-wide product and sum into a fused multiply-add
+// whatever their rounding modifiers say, so the sum is written as a * one + b
+// with a one that it cannot see (a kernel argument): the same value and one
+// rounding.  The lane rate is that of the scalar operations; the two-wide form
+// halves the issue slots and the coefficient registers.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b, f32x2 one) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(one), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 both(float a) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(a));
+    return d;
+}
+
+// dipole_double (NISE_subs.c:485-509) of vector u: element (i, j), i <= j.
+template <typename R>
+__device__ __forceinline__ typename Vec2<R>::T dbl_init(const TwoD &D, int s, int u, int i, int j) {
+    typedef typename Vec2<R>::T R2;
+    typedef Ar<R> A;
+    const DblVec w = dbl_vec(u, D.T1);
+    const long tk = tk_of(D, s);
+    const R2 *src = (const R2 *)D.SE + ((size_t)s * D.T3 * nvec_se(D) + (w.kind == 0 ? w.pa : 3 + w.pa * D.T1 + w.t1)) * D.n;
+    R2 f;
+    if (i == j) {
+        const R o = (R)over_mu(D, tk, w.p2, i);
+        f.x = A::mul(o, src[i].x);
+        f.y = A::mul(o, src[i].y);
+    } else {
+        const R mi = (R)traj_mu(D.T, tk, w.p2, i), mj = (R)traj_mu(D.T, tk, w.p2, j);
+        f.x = A::add(A::mul(mi, src[j].x), A::mul(mj, src[i].x));
+        f.y = A::add(A::mul(mi, src[j].y), A::mul(mj, src[i].y));
+    }
+    return f;
+}
+
+// ------------------------------------------------ doubles, two vectors together
+// FP32, up to 64 sites: two doubles vectors of one start point share a warp (n <=
+// 32) or two warps, thread c the column c of both, with the operations of
+// k2d_doubles in its order, so the results are bitwise the same.  An element of
+// the circulant layout holds both vectors (re, re, im, im): one 16-byte load and
+// store serve two rotations, the two-wide instructions halve the issue slots of
+// their 24 operations, and coefficients, slot indices and synchronisation are
+// shared.
+//
+// The couplings run in the segments of k2d_doubles_duo (one first site a, one
+// warp of second sites b, the owner), with its ordering.  Coupling (a, b)
+// rotates |ac> (a register, the pivot row) and |bc> for every c, and in the owner
+// |aa> with |ab>.  The owner loads the next coupling's elements |b'c> before it
+// stores this one's; of those only |b'b>, which column b reads, is changed by
+// this coupling (by column b'), so that column alone reads its element again
+// after the __syncwarp, as column b' reads |aa>.  The records of 32 couplings are
+// staged in shared memory a chunk ahead, slot indices are read two couplings
+// ahead.  Bound by the issue and latency of the owners' steps: 93 instructions
+// per coupling and pair, half of the issue slots used (247 cycles per coupling of
+// five pairs).  64 sites, 10 start points, RunTimes 64 0 64: 498 ms with one
+// vector on two warps, 307 ms now; 24 sites, 12 start points, RunTimes 32 0 32
+// (whole spectrum): 38.2 against 21.0 ms with one vector per warp.  One warp for
+// both column halves of a pair (half the warps, 130 instructions in one stream)
+// measured 680 ms.
+struct DblPair { f32x2 re, im; };
+
+__device__ __forceinline__ DblPair pair_ld(const float4 *p) {
+    const ulonglong2 v = *(const ulonglong2 *)p;
+    return {v.x, v.y};
+}
+__device__ __forceinline__ void pair_st(float4 *p, DblPair v) { *(ulonglong2 *)p = make_ulonglong2(v.re, v.im); }
+
+// rot2 on two vectors: a - b is b * (-1) + a, rounded once.
+__device__ __forceinline__ void pair_rot(DblPair &x1, DblPair &x2, f32x2 co, f32x2 si, f32x2 one, f32x2 mone) {
+    DblPair y1, y2;
+    y1.re = add2(mul2(si, x2.im), mul2(co, x1.re), mone);
+    y1.im = add2(mul2(si, x2.re), mul2(co, x1.im), one);
+    y2.re = add2(mul2(si, x1.im), mul2(co, x2.re), mone);
+    y2.im = add2(mul2(si, x1.re), mul2(co, x2.im), one);
+    x1 = y1;
+    x2 = y2;
+}
+
+__device__ __forceinline__ DblPair pair_phase(DblPair z, float2 u, f32x2 one, f32x2 mone) {
+    const f32x2 ur = both(u.x), ui = both(u.y);
+    return {add2(mul2(z.im, ui), mul2(z.re, ur), mone), add2(mul2(z.im, ur), mul2(z.re, ui), one)};
+}
+
+// A warp's ring of coupling records: 64, of which 32 ahead.
+struct PairStage {
+    float4 c[64][2];  // (co, co, si, si), then at sqrt2
+    int row[64];      // b * n, the start of b's row of the slot table
+};
+
+// The owner's couplings [k, e) of a segment.
+template <bool ES>
+__device__ __forceinline__ void pair_owner(float4 *F, DblPair &piv, const PairStage *st, int k, int e, float4 *paa,
+                                           bool act, int c, int n, const unsigned short *cic, f32x2 one, f32x2 mone) {
+    const int cn = c * n;  // this column as a second site
+    int rowA = st->row[k & 63], rowB = st->row[(k + 1) & 63];
+    float4 *pA = F + cic[rowA], *pB = F + cic[rowB];
+    DblPair Q = pair_ld(pA);
+    int stale = -1;  // the row of the column whose element the last coupling changed
+#pragma unroll 2
+    for (; k < e; k++) {
+        const bool own = rowA == cn;
+        const ulonglong2 q = *(const ulonglong2 *)&st->c[k & 63][own];
+        DblPair X = {0, 0};
+        if (!ES) X = pair_ld(paa);
+        if (stale == cn) Q = pair_ld(pA);
+        const DblPair Qn = pair_ld(pB);
+        const int rowC = st->row[(k + 2) & 63];
+        float4 *pC = F + cic[rowC];
+        DblPair P = piv;
+        if (!ES) {
+            pair_rot(X, P, q.x, q.y, one, mone);
+            if (own) pair_st(paa, X);
+            P.re = own ? P.re : piv.re;
+            P.im = own ? P.im : piv.im;
+        }
+        pair_rot(P, Q, q.x, q.y, one, mone);
+        if (!ES || !own) {
+            piv = P;
+            if (act) pair_st(pA, Q);
+        }
+        stale = rowA;
+        rowA = rowB;
+        rowB = rowC;
+        pA = pB;
+        pB = pC;
+        Q = Qn;
+        __syncwarp();
+    }
+}
+
+// The other warp's: elements no other thread touches in the segment.
+__device__ __forceinline__ void pair_free(float4 *F, DblPair &piv, const PairStage *st, int k, int e, bool act,
+                                          const unsigned short *cic, f32x2 one, f32x2 mone) {
+    for (; k + 4 <= e; k += 4) {
+        float4 *p[4];
+        DblPair Q[4];
+        ulonglong2 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            p[u] = F + cic[st->row[(k + u) & 63]];
+            q[u] = *(const ulonglong2 *)&st->c[(k + u) & 63][0];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) Q[u] = pair_ld(p[u]);
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            pair_rot(piv, Q[u], q[u].x, q[u].y, one, mone);
+            if (act) pair_st(p[u], Q[u]);
+        }
+    }
+    for (; k < e; k++) {
+        float4 *p = F + cic[st->row[k & 63]];
+        const ulonglong2 q = *(const ulonglong2 *)&st->c[k & 63][0];
+        DblPair Q = pair_ld(p);
+        pair_rot(piv, Q, q.x, q.y, one, mone);
+        if (act) pair_st(p, Q);
+    }
+}
+
+template <bool TWO>
+__device__ __forceinline__ void pair_sync(int bar) {
+    if (TWO) duo_sync(bar);
+    else __syncwarp();
+}
+
+// One Trotter sub-step's couplings.
+template <bool TWO, bool ES>
+__device__ __forceinline__ void pair_couplings(float4 *F, const Dcoef<float> *cf, const TwoD &D, int half, int lane, int c,
+                                               const unsigned short *ci, PairStage *st, int bar, f32x2 one, f32x2 mone) {
+    const int n = D.n, K = D.K;
+    if (K == 0) return;
+    const int cc = min(c, n - 1);  // a column past the last reads the last one's elements and stores nothing
+    const unsigned short *cic = ci + cc;
+    Dcoef<float> gq;
+    int grow;
+    auto get = [&](int k) {  // past the list: its last record, never applied
+        gq = cf[min(k, K - 1)];
+        grow = D.pairs[min(k, K - 1)].y * n;
+    };
+    auto put = [&](int at) {
+        st->c[at][0] = make_float4(gq.co, gq.co, gq.si, gq.si);
+        st->c[at][1] = make_float4(gq.co2, gq.co2, gq.si2, gq.si2);
+        st->row[at] = grow;
+    };
+    get(lane);
+    put(lane);
+    get(32 + lane);
+    int a = -1;
+    bool act = false;
+    DblPair piv = {0, 0};
+    float4 *paa = F;
+    for (int g = 0; g < D.nsegs; g++) {
+        const int4 sg = D.segs[g];  // (a, first coupling, end, owner)
+        if (sg.x != a && act) pair_st(F + cic[a * n], piv);
+        pair_sync<TWO>(bar);
+        if (sg.x != a) {
+            a = sg.x;
+            act = c < n && c != a;
+            piv = pair_ld(F + cic[a * n]);
+            paa = F + ci[a * n + a];
+        }
+        for (int k = sg.y; k < sg.z;) {
+            if ((k & 31) == 0) {  // the next 32 records arrive, those after them start their way
+                put((k + 32 + lane) & 63);
+                get(k + 64 + lane);
+                __syncwarp();
+            }
+            const int e = min(sg.z, (k | 31) + 1);
+            if (!TWO || half == sg.w) pair_owner<ES>(F, piv, st, k, e, paa, act, c, n, cic, one, mone);
+            else pair_free(F, piv, st, k, e, act, cic, one, mone);
+            k = e;
+        }
+    }
+    if (act) pair_st(F + cic[a * n], piv);
+    pair_sync<TWO>(bar);
+}
+
+// CTA = P pairs of vectors of one start point, all at the same t3, each on one
+// warp (n <= 32) or two.  G, the pair's dipole_double_last, reuses the rings.
+template <bool TWO>
+__global__ void __launch_bounds__(512, 1) k2d_doubles_pair(TwoD D, int vec_per_sample, const Dcoef<float> *cf_all,
+                                                           float onef, float monef) {
+    typedef Ar<float> A;
+    constexpr int TW = TWO ? 2 : 1, T = 32 * TW;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int n = D.n, Wd = n / 2 + 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int pair = warp / TW, npairs = nwarps / TW, slots = n * Wd, bar = 1 + pair;
+    // the owner of most couplings is the second half: swapped in every other
+    // two pairs, so that the schedulers share those warps
+    const int half = TWO ? (warp & 1) ^ ((pair >> 1) & 1) : 0, c = lane + 32 * half, t = c;
+    float4 *F = (float4 *)smem_raw + (size_t)pair * slots;  // this pair's two vectors
+    PairStage *rings = (PairStage *)((float4 *)smem_raw + (size_t)npairs * slots);
+    PairStage *st = rings + warp;
+    float2 *G = (float2 *)(rings + pair * TW);  // [2][3][n]
+    float2 *Uh = (float2 *)(rings + nwarps);    // [slots]
+    float *mu = (float *)(Uh + slots), *ov = mu + 3 * n, *dg = ov + 3 * n;
+    unsigned short *ci = (unsigned short *)(dg + n);  // [n][n] circ(x, y)
+    const f32x2 one = both(onef), mone = both(monef);
+    const int vpc = 2 * npairs, cps = (vec_per_sample + vpc - 1) / vpc, s = blockIdx.x / cps;
+    const int u0 = (blockIdx.x % cps) * vpc + 2 * pair, nv = max(0, min(2, vec_per_sample - u0));
+    const long tk = tk_of(D, s);
+    const int NV = nvec_se(D);
+    for (int e = threadIdx.x; e < slots; e += blockDim.x) Uh[e] = make_float2(1, 0);  // unused slots: unit phase
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) ci[e] = (unsigned short)circ(e / n, e % n, n, Wd);
+    for (int e = t; e < slots; e += T) F[e] = make_float4(0, 0, 0, 0);
+    __syncthreads();
+    for (int h = 0; h < nv; h++)
+        for (int i = 0; i < n; i++)  // dipole_double (NISE_subs.c:485-509)
+            for (int j = i + t; j < n; j += T) {
+                const float2 f = dbl_init<float>(D, s, u0 + h, i, j);
+                float *z = (float *)(F + ci[i * n + j]) + h;
+                z[0] = f.x;
+                z[2] = f.y;
+            }
+    for (int t3 = 0; t3 < D.T3; t3++) {
+        const long tl = tk + t3;
+        __syncthreads();
+        for (int i = threadIdx.x; i < 3 * n; i += blockDim.x) {
+            mu[i] = traj_mu(D.T, tl, i / n, i % n);
+            ov[i] = over_mu(D, tl, i / n, i % n);
+        }
+        __syncthreads();
+        if (nv > 0 && D.ea) {  // EA projections and dot products (calc_2DIR.c:456-488), as k2d_doubles
+            if (c < n)
+                for (int p3 = 0; p3 < 3; p3++) {
+                    DblPair g = {0, 0};
+                    for (int j = 0; j < n; j++) {
+                        const f32x2 m = both(j == c ? ov[p3 * n + c] : mu[p3 * n + j]);
+                        const DblPair f = pair_ld(F + ci[j * n + c]);
+                        g.re = add2(mul2(m, f.re), g.re, one);
+                        g.im = add2(mul2(m, f.im), g.im, one);
+                    }
+                    for (int h = 0; h < 2; h++)
+                        G[(h * 3 + p3) * n + c] = make_float2(__uint_as_float((unsigned)(g.re >> (32 * h))),
+                                                              __uint_as_float((unsigned)(g.im >> (32 * h))));
+                }
+            pair_sync<TWO>(bar);
+            for (int h = 0, item = 0; h < nv; h++) {
+                const DblVec w = dbl_vec(u0 + h, D.T1);
+                for (int m = 0; m < 21; m++) {
+                    const int p0 = c_px[m][0], p1 = c_px[m][1], p3 = c_px[m][3];
+                    if (c_px[m][2] != w.p2 || (w.kind == 0 ? p1 : p0) != w.pa) continue;
+                    // rephasing (fr): right = conj(leftn_p0[t1]) for every t1; non-rephasing (ft1[t1]): conj(leftr_p1)
+                    const int reps = w.kind == 0 ? D.T1 : 1;
+                    for (int r = TWO ? (half ^ (item & 1)) : 0; r < reps; r += TW) {
+                        const float2 *rv = (const float2 *)D.SE +
+                                           (((size_t)s * D.T3 + t3) * NV + (w.kind == 0 ? 3 + p0 * D.T1 + r : p1)) * n;
+                        double a1 = 0, a2 = 0;
+#pragma unroll
+                        for (int q = lane; q < T; q += 32) {
+                            if (q >= n) continue;
+                            const float2 gq = G[(h * 3 + p3) * n + q];
+                            const float Rr = rv[q].x, Ri = -rv[q].y;
+                            a1 += (double)A::add(A::mul(gq.y, Rr), A::mul(gq.x, Ri));
+                            a2 += (double)A::sub(A::mul(gq.x, Rr), A::mul(Ri, gq.y));
+                        }
+                        for (int o = 16; o > 0; o >>= 1) {
+                            a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+                            a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+                        }
+                        if (lane == 0)
+                            (w.kind == 0 ? D.eaI : D.eaII)[(((size_t)s * D.T3 + t3) * 21 + m) * D.T1 +
+                                                           (w.kind == 0 ? r : w.t1)] = make_double2(a1, a2);
+                    }
+                    item += reps;
+                }
+            }
+        }
+        if (t3 == D.T3 - 1) break;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) dg[i] = traj_diag(D.T, tl, i, false);
+        __syncthreads();
+        doubles_half_phases<float>(D, Uh, dg, tl, n, Wd);
+        __syncthreads();
+        if (nv == 0) continue;
+        const Dcoef<float> *cf = D.rot_static ? cf_all : cf_all + (tl - D.f0) * D.K;
+        for (int e = t; e < slots; e += T)  // propagate.c:959-962
+            pair_st(F + e, pair_phase(pair_ld(F + e), Uh[e], one, mone));
+        for (int sub = 0; sub < D.ts; sub++) {
+            pair_sync<TWO>(bar);
+            if (D.es) pair_couplings<TWO, true>(F, cf, D, half, lane, c, ci, st, bar, one, mone);
+            else pair_couplings<TWO, false>(F, cf, D, half, lane, c, ci, st, bar, one, mone);
+            for (int e = t; e < slots; e += T) {  // propagate.c:1041-1044, and the next sub-step's first
+                DblPair z = pair_phase(pair_ld(F + e), Uh[e], one, mone);
+                if (sub + 1 < D.ts) z = pair_phase(z, Uh[e], one, mone);
+                pair_st(F + e, z);
+            }
+        }
+    }
+}
+
 // Coupling coefficients of the doubles Trotter step for the static coupling
 // frame: si = -sin(J f), co = sqrt(1-si^2), and the sqrt(2) pair
 // (propagate.c:970-993), float operations as the reference in FP32.
@@ -998,36 +1346,6 @@ __device__ void rk4_doubles_step(const TwoD &D, long t, typename Vec2<R>::T *F, 
 // the response's cancellation amplifies another order by 10^3), FP64 multiplies
 // matrices (k2d_doubles_sparse64).
 
-// Which vector of a start point: u < 9 -> fr for (p1,p2) = (u/3, u%3); else
-// ft1[t1] for (p0,p2).
-struct DblVec { int kind, pa, p2, t1; };
-__device__ __forceinline__ DblVec dbl_vec(int u, int T1) {
-    if (u < 9) return {0, u / 3, u % 3, 0};
-    const int w = u - 9, cmb = w / T1;
-    return {1, cmb / 3, cmb % 3, w % T1};
-}
-
-// dipole_double (NISE_subs.c:485-509) of vector u: element (i, j), i <= j.
-template <typename R>
-__device__ __forceinline__ typename Vec2<R>::T dbl_init(const TwoD &D, int s, int u, int i, int j) {
-    typedef typename Vec2<R>::T R2;
-    typedef Ar<R> A;
-    const DblVec w = dbl_vec(u, D.T1);
-    const long tk = tk_of(D, s);
-    const R2 *src = (const R2 *)D.SE + ((size_t)s * D.T3 * nvec_se(D) + (w.kind == 0 ? w.pa : 3 + w.pa * D.T1 + w.t1)) * D.n;
-    R2 f;
-    if (i == j) {
-        const R o = (R)over_mu(D, tk, w.p2, i);
-        f.x = A::mul(o, src[i].x);
-        f.y = A::mul(o, src[i].y);
-    } else {
-        const R mi = (R)traj_mu(D.T, tk, w.p2, i), mj = (R)traj_mu(D.T, tk, w.p2, j);
-        f.x = A::add(A::mul(mi, src[j].x), A::mul(mj, src[i].x));
-        f.y = A::add(A::mul(mi, src[j].y), A::mul(mj, src[i].y));
-    }
-    return f;
-}
-
 // EA projections and dot products of the CTA's vectors u0 .. u0 + nv - 1 at t3
 // (calc_2DIR.c:456-488): dipole_double_last into G[q][p3][n] (float sums in
 // site order), then a warp per dot product.  at(q, j, a) is element (j, a) of
@@ -1105,29 +1423,6 @@ template <typename R>
 __device__ __forceinline__ typename Vec2<R>::T dbl_half(typename Vec2<R>::T ph, R x, R y) {
     typedef Ar<R> A;
     return make_vec2<R>(A::sub(A::mul(ph.x, x), A::mul(ph.y, y)), A::add(A::mul(ph.x, y), A::mul(ph.y, x)));
-}
-
-// Two single-precision operations per instruction, each rounded by itself.
-// The assembler contracts a two-wide product and sum into a fused multiply-add
-// whatever their rounding modifiers say, so the sum is written as a * one + b
-// with a one that it cannot see (a kernel argument): the same value and one
-// rounding.  The lane rate is that of the scalar operations; the two-wide form
-// halves the issue slots and the coefficient registers.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b, f32x2 one) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(one), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 both(float a) {
-    f32x2 d;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(d) : "f"(a));
-    return d;
 }
 
 // FP32: every term of the reference's sum, in its order and roundings.
@@ -1698,21 +1993,35 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf) {
         size_t dsm = bytes(nwarps, use_tab);
         if (dsm > 220 * 1024) return (int)cudaErrorNotSupported;
         int vps = 9 + 9 * D.T1, cps = (vps + nwarps - 1) / nwarps;
-        // two warps per vector (k2d_doubles_duo, the same float operations)
-        // unless kernel_config 1 asks for one
+        // FP64: two warps per vector (k2d_doubles_duo) unless kernel_config 1 asks for one
         auto bytes_duo = [&](int pairs, bool tab) {
             return sizeof(R2) * ((size_t)slots * (1 + pairs) + 64 * (size_t)pairs) + sizeof(float) * 7 * D.n +
                    (tab ? sizeof(short) * D.n * D.n : 0);
         };
-        if (D.n > 32 && D.n <= 64 && c->p.kernel_config != 1) {
+        // FP32: pairs of vectors (k2d_doubles_pair, bitwise the one-warp kernel),
+        // on one warp up to 32 sites (several small CTAs per SM), on two above
+        // (as many as shared memory holds)
+        const int tw = D.n <= 32 ? 1 : 2;
+        auto bytes_pair = [&](int p) {
+            return sizeof(float4) * (size_t)slots * p + sizeof(PairStage) * p * tw + sizeof(float2) * slots +
+                   sizeof(float) * 7 * D.n + sizeof(short) * D.n * D.n;
+        };
+        if (sizeof(R) == 4 && D.n <= 64 && c->p.kernel_config != 1) {
+            int np = std::min(tw == 1 ? 4 : 8, (vps + 1) / 2);
+            while (np > 1 && bytes_pair(np) > 227 * 1024) np--;
+            auto kern = tw == 1 ? k2d_doubles_pair<false> : k2d_doubles_pair<true>;
+            if ((e = smem_attr(kern, bytes_pair(np)))) return e;
+            kern<<<D.S * ((vps + 2 * np - 1) / (2 * np)), 32 * tw * np, bytes_pair(np), st>>>(
+                D, vps, (const Dcoef<float> *)cf, 1.0f, -1.0f);
+        } else if (sizeof(R) == 8 && D.n > 32 && D.n <= 64 && c->p.kernel_config != 1) {
             int np = 11;  // 704 threads at most; named barriers 1..11
             while (np > 1 && bytes_duo(np, false) > 220 * 1024) np--;
             const int tab = bytes_duo(np, true) <= 220 * 1024;
             const size_t dsm2 = bytes_duo(np, tab);
             if (dsm2 > 220 * 1024) return (int)cudaErrorNotSupported;
             const int cps2 = (vps + np - 1) / np;
-            if ((e = smem_attr(k2d_doubles_duo<R>, dsm2))) return e;
-            k2d_doubles_duo<R><<<D.S * cps2, 64 * np, dsm2, st>>>(D, vps, cf, tab);
+            if ((e = smem_attr(k2d_doubles_duo<double>, dsm2))) return e;
+            k2d_doubles_duo<double><<<D.S * cps2, 64 * np, dsm2, st>>>(D, vps, (Dcoef<double> *)cf, tab);
         } else if (D.n <= 32) {
             if ((e = smem_attr(k2d_doubles<R, 1>, dsm))) return e;
             k2d_doubles<R, 1><<<D.S * cps, 32 * nwarps, dsm, st>>>(D, vps, cf, use_tab);
