@@ -27,6 +27,12 @@ struct DevTraj {
     float cut;               // Couplingcut
 };
 
+// Rows of a Trotter time step (nise_row_schedule) in device memory.
+struct RowPlan {
+    const uint2 *rows;
+    int nrow;
+};
+
 // Coefficient tables of one singles propagation scheme over the frames
 // [f0, f0 + nf) of a job (built by nise_singles_tables): the Trotter half
 // phases U[t][n] and rotations rot[t][K] (or [K] for static couplings), the

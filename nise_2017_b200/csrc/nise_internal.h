@@ -107,6 +107,8 @@ struct SinglesBufs {
     DevBuf<int2> pairs, ent;
     DevBuf<int4> segs;
     DevBuf<char> U, rot, rkval;
+    DevBuf<uint2> rows;
+    RowPlan row = {nullptr, 0};  // the Trotter step's rows of 32 (none above 65503 sites)
     const void *Us = nullptr;
 };
 

@@ -41,3 +41,34 @@ void nise_schedule_parts(const std::vector<int2> &pairs, int n, std::vector<uint
     for (int a = 0; a < n; a++)
         if (first[a] < 0) iso.push_back(a);
 }
+
+int nise_row_schedule(const std::vector<int2> &pairs, int n, int ts, int width, std::vector<uint2> &rows) {
+    std::vector<int> ready(n, 0);               // first row after the site's last operation
+    std::vector<std::vector<uint2>> row;
+    std::vector<int> next;                      // next[r]: a row >= r that may have room (path-compressed)
+    auto place = [&](int a, int b, uint32_t y) {
+        int r = std::max(ready[a], ready[b]);
+        while (r < (int)next.size() && next[r] != r) r = next[r] = next[r] < (int)next.size() ? next[next[r]] : next[r];
+        while (r >= (int)row.size()) {
+            next.push_back((int)row.size());
+            row.emplace_back();
+        }
+        row[r].push_back(make_uint2((uint32_t)a | (uint32_t)b << 16, y));
+        if ((int)row[r].size() == width) next[r] = r + 1;
+        ready[a] = ready[b] = r + 1;
+    };
+    for (int s = 0; s < ts; s++) {
+        for (int a = 0; a < n; a++) place(a, a, NISE_ROW_PHASE | (uint32_t)a);
+        for (size_t k = 0; k < pairs.size(); k++) place(pairs[k].x, pairs[k].y, (uint32_t)k);
+        for (int a = 0; a < n; a++) place(a, a, NISE_ROW_PHASE | (uint32_t)a);
+    }
+    const int nrow = (int)row.size();
+    rows.clear();
+    for (int r = 0; r < nrow + 2; r++)
+        for (int i = 0; i < width; i++) {
+            const uint32_t spare = (uint32_t)(n + i % 32);
+            rows.push_back(r < nrow && i < (int)row[r].size() ? row[r][i]
+                                                              : make_uint2(spare | spare << 16, NISE_ROW_PHASE | (uint32_t)n));
+        }
+    return nrow;
+}

@@ -39,3 +39,17 @@ int nise_step_schedule(const std::vector<int2> &pairs, int n, int ts, int steps,
 // The packed sites and parts of every rotation; iso: the sites that no
 // rotation touches.
 void nise_schedule_parts(const std::vector<int2> &pairs, int n, std::vector<uint32_t> &parts, std::vector<int> &iso);
+
+// Whole time steps as rows of `width` (a multiple of 32) independent operations
+// of one kind, y_a = c x_a + i s x_b, y_b = c x_b + i s x_a: a rotation with its
+// (co, si), or, with a = b, a site's half-step phase with its (cos, -sin) (the
+// same float operations in the same order as propagate.c:870-873).  One step is
+// `ts` times all phases, the rotations in order, all phases; every operation
+// goes to the first row after the rows of the earlier operations on its sites
+// that has room, so each site sees them in the reference's order.  x = a | b <<
+// 16; y = index into the rotation coefficients, or NISE_ROW_PHASE | site.  Idle
+// places rotate a spare site of their own, n + (place mod 32), by the phase at
+// index n, which the caller sets to (1, 0).  Two idle rows follow the last (a
+// kernel reads two rows ahead).  Returns the number of rows without them.
+#define NISE_ROW_PHASE 0x80000000u
+int nise_row_schedule(const std::vector<int2> &pairs, int n, int ts, int width, std::vector<uint2> &rows);

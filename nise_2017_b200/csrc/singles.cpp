@@ -15,6 +15,7 @@
 #include "eigen.h"
 #include "engine.h"
 #include "nise_internal.h"
+#include "rotsched.h"
 
 int nise_singles_tables(nise_ctx *c, const DevTraj &T, long fmin, long nf, int singleshift, bool doubles_u,
                         SinglesTab &S, SinglesBufs &B) {
@@ -64,6 +65,13 @@ int nise_singles_tables(nise_ctx *c, const DevTraj &T, long fmin, long nf, int s
         c->launches += 1 + P.rot_static;
         S.U = B.U.p;
         S.rot = B.rot.p;
+        if (N + 32 <= 0xffff && p.ts >= 1) {
+            std::vector<uint2> rows;
+            pairs.pop_back();
+            B.row.nrow = nise_row_schedule(pairs, N, p.ts, 32, rows);
+            if ((rc = B.rows.upload(c, rows))) return rc;
+            B.row.rows = B.rows.p;
+        }
     } else if (p.propagation == NISE_PROP_SPARSE || p.propagation == NISE_PROP_DIAGONAL) {
         // propagate_vector's Sparse scheme (DIA, or DIA_S when 0 < Threshold
         // <= 1) and time_evolution_mat's truncated sub-step propagator for the

@@ -45,6 +45,7 @@
 #include "eigen.h"
 #include "engine.h"
 #include "nise_internal.h"
+#include "rows.cuh"
 #include "schemes.cuh"
 
 namespace {
@@ -82,6 +83,14 @@ struct TwoD : SinglesTab {
     double *Rs;               // [S][12][T3][T1]
     const float *lt;          // [T3][T1]
 };
+
+template <typename R>
+__device__ __forceinline__ typename Vec2<R>::T make_vec2(R x, R y) {
+    typename Vec2<R>::T v;
+    v.x = x;
+    v.y = y;
+    return v;
+}
 
 __device__ __forceinline__ long tj_of(const TwoD &D, int s) { return (long)(D.s0 + s) * D.sample + D.T1; }
 __device__ __forceinline__ long tk_of(const TwoD &D, int s) { return tj_of(D, s) + D.T2; }
@@ -226,6 +235,104 @@ __global__ void k2d_se(TwoD D) {
     }
 }
 
+// ------------------------------------------------ singles, a warp per vector
+// k2d_gb1, k2d_gb3 and k2d_se for the Trotter scheme with the rotations of a step
+// spread over a warp (rows.cuh), the same operations.  64 sites, 10 start
+// points, RunTimes 64 0 64: 58.4, 38.7 and 34.8 ms with a thread per vector (the
+// chain of 1900 rotations a sub-step), now 2.0, 1.5 and 4.6 ms (115 cycles a row).
+template <typename R>
+__device__ __forceinline__ double2 rows_dot(const TwoD &D, long t, int x, const typename Vec2<R>::T *X, int lane) {
+    double pr = 0, pi = 0;
+    for (int i = lane; i < D.n; i += 32) {  // dot_mu's order: a residue's sites, then the residues
+        const R m = (R)traj_mu(D.T, t, x, i);
+        pr += (double)Ar<R>::mul(m, X[i].x);
+        pi += (double)Ar<R>::mul(m, X[i].y);
+    }
+    return resp_sum_warp(pr, pi, D.n);
+}
+
+template <typename R>
+__global__ void __launch_bounds__(256) k2d_gb1_rows(TwoD D, RowPlan Q, int stage) {
+    typedef typename Vec2<R>::T R2;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const uint2 *rows;
+    const R2 *rs;
+    R2 *X = rows_setup<R>(D, Q, stage, smem_raw, rows, rs);
+    const int n = D.n, lane = threadIdx.x & 31, P = (D.T1 + 1) / 2;
+    const int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (g >= D.S * 3 * P) return;
+    const int s = g / (3 * P), rem = g % (3 * P), x = rem / P, p = rem % P;
+    const long tj = tj_of(D, s);
+    for (int pass = 0; pass < 2; pass++) {
+        const int t1 = pass == 0 ? p : D.T1 - 1 - p;
+        if (pass == 1 && t1 == p) break;
+        for (int i = lane; i < n; i += 32) X[i] = make_vec2<R>((R)traj_mu(D.T, tj - t1, x, i), 0);
+        for (int tm = 0; tm < t1; tm++) rows_singles_step<R>(D, rows, Q.nrow, X, rs, lane, tj - t1 + tm - D.f0);
+        __syncwarp();
+        R2 *out = (R2 *)D.L + (((size_t)s * 3 + x) * D.T1 + t1) * n;
+        for (int i = lane; i < n; i += 32) out[i] = X[i];
+        if (D.gb)  // t1nr/t1ni (calc_2DIR.c:244-250) for every p1
+            for (int p1 = 0; p1 < 3; p1++) {
+                const double2 z = rows_dot<R>(D, tj, p1, X, lane);
+                if (lane == 0) D.gbt1[(((size_t)s * 3 + x) * 3 + p1) * D.T1 + t1] = z;
+            }
+        __syncwarp();
+    }
+}
+
+template <typename R>
+__global__ void __launch_bounds__(256) k2d_gb3_rows(TwoD D, RowPlan Q, int stage) {
+    typedef typename Vec2<R>::T R2;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const uint2 *rows;
+    const R2 *rs;
+    R2 *X = rows_setup<R>(D, Q, stage, smem_raw, rows, rs);
+    const int lane = threadIdx.x & 31, g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (g >= D.S * 3) return;
+    const int s = g / 3, x = g % 3;
+    const long tk = tk_of(D, s);
+    for (int i = lane; i < D.n; i += 32) X[i] = make_vec2<R>((R)traj_mu(D.T, tk, x, i), 0);
+    for (int t3 = 0; t3 < D.T3; t3++) {  // calc_2DIR.c:257-299
+        __syncwarp();
+        for (int p3 = 0; p3 < 3; p3++) {
+            const double2 z = rows_dot<R>(D, tk + t3, p3, X, lane);
+            if (lane == 0) D.gbt3[(((size_t)s * 3 + x) * 3 + p3) * D.T3 + t3] = z;
+        }
+        if (t3 < D.T3 - 1) rows_singles_step<R>(D, rows, Q.nrow, X, rs, lane, tk + t3 - D.f0);
+    }
+}
+
+template <typename R>
+__global__ void __launch_bounds__(256) k2d_se_rows(TwoD D, RowPlan Q, int stage) {
+    typedef typename Vec2<R>::T R2;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const uint2 *rows;
+    const R2 *rs;
+    R2 *X = rows_setup<R>(D, Q, stage, smem_raw, rows, rs);
+    const int n = D.n, NV = nvec_se(D), lane = threadIdx.x & 31, g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (g >= D.S * NV) return;
+    const int s = g / NV, v = g % NV;
+    const R2 *vec = v < 3 ? (const R2 *)D.Lr + ((size_t)s * 3 + v) * n
+                          : (const R2 *)D.L + (((size_t)s * 3 + (v - 3) / D.T1) * D.T1 + (v - 3) % D.T1) * n;
+    for (int i = lane; i < n; i += 32) X[i] = vec[i];
+    const long tk = tk_of(D, s);
+    for (int t3 = 0; t3 < D.T3; t3++) {  // calc_2DIR.c:372-443
+        __syncwarp();
+        R2 *snap = (R2 *)D.SE + (((size_t)s * D.T3 + t3) * NV + v) * n;
+        for (int i = lane; i < n; i += 32) snap[i] = X[i];
+        if (t3 < D.T3 - 1) rows_singles_step<R>(D, rows, Q.nrow, X, rs, lane, tk + t3 - D.f0);
+    }
+}
+
+template <typename R, typename Kern>
+int run_rows(Kern kern, const TwoD &D, const RowPlan &Q, long vectors, cudaStream_t st) {
+    const RowShape h = rows_shape<R>(D.n, D.K, D.rot_static, Q.nrow, vectors, sm_count());
+    if (!h.warps) return (int)cudaErrorNotSupported;
+    if (const int e = (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.bytes)) return e;
+    kern<<<(unsigned)((vectors + h.warps - 1) / h.warps), 32 * h.warps, h.bytes, st>>>(D, Q, h.stage);
+    return (int)cudaGetLastError();
+}
+
 // ---------------------------------------------------------------- doubles
 // Shared-memory layout of one doubles vector: the pair {x,y} lives at
 // circ(x,y): with d = (y-x) mod n, slot x*W + d when d < n-d (or d == n-d and
@@ -253,14 +360,6 @@ __device__ __forceinline__ void rot2(typename Vec2<R>::T &x1, typename Vec2<R>::
 
 // 16-byte (FP32) / 32-byte (FP64) records, one vector load each
 template <typename R> struct alignas(4 * sizeof(R)) Dcoef { R co, si, co2, si2; };
-
-template <typename R>
-__device__ __forceinline__ typename Vec2<R>::T make_vec2(R x, R y) {
-    typename Vec2<R>::T v;
-    v.x = x;
-    v.y = y;
-    return v;
-}
 
 // Warp per doubles vector; lane l owns columns c = l + 32*j (j < CPL).  One
 // Trotter sub-step of propagate_vec_coupling_S_doubles (propagate.c:956-1045):
@@ -1901,7 +2000,7 @@ int lanes_for2(size_t bytes_per_lane, int want) {
 }
 
 template <typename R>
-int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf) {
+int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf, const RowPlan &Q) {
     typedef typename Vec2<R>::T R2;
     cudaStream_t st = c->stream;
     int e;
@@ -1912,10 +2011,20 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf) {
     if ((e = smem_attr(k2d_gb1<R>, sm))) return e;
     if ((e = smem_attr(k2d_gb3<R>, sm))) return e;
     if ((e = smem_attr(k2d_se<R>, sm))) return e;
-    k2d_gb1<R><<<(D.S * 3 * P + B - 1) / B, B, sm, st>>>(D);
+    // Trotter: a warp per vector where its state and tables fit shared memory
+    const bool rows = Q.rows && rows_shape<R>(D.n, D.K, D.rot_static, Q.nrow, 1, 1).warps > 0;
+    if (rows) {
+        if ((e = run_rows<R>(k2d_gb1_rows<R>, D, Q, (long)D.S * 3 * P, st))) return e;
+    } else {
+        k2d_gb1<R><<<(D.S * 3 * P + B - 1) / B, B, sm, st>>>(D);
+    }
     c->launches++;
     if (D.gb) {
-        k2d_gb3<R><<<(D.S * 3 + B - 1) / B, B, sm, st>>>(D);
+        if (rows) {
+            if ((e = run_rows<R>(k2d_gb3_rows<R>, D, Q, (long)D.S * 3, st))) return e;
+        } else {
+            k2d_gb3<R><<<(D.S * 3 + B - 1) / B, B, sm, st>>>(D);
+        }
         c->launches++;
     }
     if (D.se || D.ea) {
@@ -1928,7 +2037,11 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf) {
             c->launches++;
         }
         int nv = D.S * (3 + 3 * D.T1);
-        k2d_se<R><<<(nv + B - 1) / B, B, sm, st>>>(D);
+        if (rows) {
+            if ((e = run_rows<R>(k2d_se_rows<R>, D, Q, nv, st))) return e;
+        } else {
+            k2d_se<R><<<(nv + B - 1) / B, B, sm, st>>>(D);
+        }
         c->launches++;
     }
     if (D.ea && is_eigen_scheme(D.prop)) {
@@ -2194,8 +2307,8 @@ extern "C" int nise_2dir(nise_ctx *c, double *R, int *sample_count) {
         // leftr_x = mu_x(tj) (calc_2DIR.c:303-304): host-free fill via a tiny copy kernel
         if ((rc = nise_cuda(c, launch_2d_leftr(D, prec, c->stream), "2DIR leftr"))) return rc;
         c->launches++;
-        int e = prec == NISE_FP32 ? run_chunk<float>(c, D, (Dcoef<float> *)dcoef.p)
-                                  : run_chunk<double>(c, D, (Dcoef<double> *)dcoef.p);
+        int e = prec == NISE_FP32 ? run_chunk<float>(c, D, (Dcoef<float> *)dcoef.p, SB.row)
+                                  : run_chunk<double>(c, D, (Dcoef<double> *)dcoef.p, SB.row);
         if ((rc = nise_cuda(c, e, "2DIR kernels"))) return rc;
         k2d_reduce<<<(unsigned)((12 * plane + 255) / 256), 256, 0, c->stream>>>((const double *)Rs.p, D.S, 12 * plane,
                                                                                dR.p, s0 == begin);

@@ -1,0 +1,44 @@
+"""Trotter steps scheduled as rows of independent operations, a warp per vector:
+the reference's float operations in its order on every site (propagate.c:821-899),
+so FP32 results equal the oracle's up to the order of the FP64 sums.
+
+No coupling at all, one, chains (few operations per row), dense couplings (full
+rows, more than one warp's worth of sites), static and per-frame coefficients.
+"""
+import pytest
+
+import helpers
+import nise_2017_b200 as nise
+import oracle
+from nise_2017_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+SUM_ORDER = 1e-10  # same float operations, FP64 sums in another order
+FP64 = 1e-11       # the same formulas in FP64
+
+
+def trajectory(tmp_path, n, geometry, ham, frames, seed):
+    static = ham == "Coupling"
+    return synth.write(synth.c0_spec(n_sites=n, frames=frames, geometry=geometry, spacing=6.0, seed=seed,
+                                     ham_type=synth.COUPLING if static else synth.FULL, dipole_frames=1 if static else 0,
+                                     mu_jitter=0.0 if static else 0.05), str(tmp_path))
+
+
+SYSTEMS = [(1, synth.CHAIN, "Full", 0.1), (2, synth.CHAIN, "Full", 0.1), (9, synth.CLUSTER, "Coupling", 1e6),
+           (16, synth.CHAIN, "Full", 0.1), (33, synth.CLUSTER, "Full", 0.1), (40, synth.CLUSTER, "Coupling", 0.1),
+           (70, synth.CLUSTER, "Coupling", 0.1)]
+
+
+@pytest.mark.parametrize("n, geometry, ham, cut", SYSTEMS[1:])
+def test_2d_singles(n, geometry, ham, cut, tmp_path):
+    files = trajectory(tmp_path, n, geometry, ham, 60, 600 + n)
+    kw = synth.c2_keywords(Singles=n, Length=60, RunTimes="5 0 5", Samplerate=23, HamiltonianType=ham, Couplingcut=cut,
+                           Technique="noEAIR", Trotter=3)
+    for precision, build, tol in ((nise.FP32, "f32a64", SUM_ORDER), (nise.FP64, "f64", FP64)):
+        with nise.Context(nise.params_from_keywords(kw, files, precision=precision)) as c:
+            c.load_files()
+            response, count = c.twodir()
+        want, wcount = oracle.twodir(oracle.params(kw, files), build)
+        assert count == wcount
+        assert helpers.rel2d(response, want) < tol
