@@ -39,6 +39,7 @@ CU_SOURCES = [
     "dia_tc.cu",
     "rk4.cu",
     "propagators.cu",
+    "trotter_rows.cu",
 ]
 CPP_SOURCES = [
     "api.cpp",

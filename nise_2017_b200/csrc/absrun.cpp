@@ -24,6 +24,7 @@
 #include "engine.h"
 #include "nise_b200.h"
 #include "nise_internal.h"
+#include "rotsched.h"
 
 namespace {
 
@@ -34,7 +35,9 @@ enum Scheme { SCHEME_TROTTER, SCHEME_RK4, SCHEME_TAYLOR, SCHEME_EIGEN };
 //            level-scheduled rotations with T threads per start point
 //            (k_abs_trotter_lv); 32 / 33 = warp per vector
 //            (k_abs_trotter_wv) with the rotation table in shared / global
-//            memory; all bitwise identical.
+//            memory; 34 = two vectors per warp; 35 / 36 = rows of 32 / 64
+//            operations of a whole step (k_abs_trotter_rows); all bitwise
+//            identical.
 //   Taylor:  3 = k_abs_taylor2 with 4 vectors per CTA, 8 = the sliced-ELL
 //            kernel with 8 (k_abs_taylor2 with 8 where it does not fit),
 //            -8 = k_abs_taylor2 with 8, 10 = the FP32 sliced-ELL kernel with
@@ -48,9 +51,27 @@ std::mutex g_tune_mu;
 // ~20 rotations per level) or the job has too few vectors to fill warps of
 // threads (a warp per vector then has the shorter critical path); thread per
 // vector for chains (one rotation per level) with many vectors.
+// rows[w]: rows of 32 (w = 0) and 64 operations per time step of `ops`, 0 where
+// they do not fit.
 int default_config(int scheme, int N, bool plain, bool cheb, int K, int nchk, int nvec, bool has4, bool rv,
-                   bool rot_static) {
+                   bool rot_static, const int rows[2], long ops) {
     if (scheme == SCHEME_TROTTER) {
+        // rows of operations, a warp per vector.  Per-frame couplings up to 128
+        // sites: 16-site chain, 1482 vectors, 0.67 ms against 1.02 (warp per
+        // level) and 1.85 (thread per vector); 64-site chain 0.84 against 2.4 and
+        // 8.0; 64 sites all coupled 3.2 against 3.9.  Static couplings: up to 100
+        // sites (64-site lattice, 2982 vectors, 3.1 against 3.9 ms for two
+        // vectors per warp), and up to 400 with few vectors (372 sites, 285
+        // vectors, 3.0 against 4.0 ms; with 1476 vectors 12.6 against 8.0; 547
+        // sites, 585 vectors, 5.8 against 5.6: full rows meet more bank
+        // conflicts than the levels' chunks, which are ordered against them).  Rows of 64 where they are fewer by a
+        // quarter (372 sites: 3.0 against 3.6; 64 sites: 0.95 against 0.78).
+        // Above about 860 operations per row and vector the SMs' warps are all
+        // busy and a thread per vector is faster (16-site chain, 7422 vectors:
+        // 1.9 against 2.2 ms).
+        const bool few = nvec < 8 * sm_count();
+        if (rows[0] && (rot_static ? N <= 100 || (few && N <= 400) : N <= 128) && (double)nvec * rows[0] < 860.0 * ops)
+            return rows[1] && rot_static && 4 * rows[1] < 3 * rows[0] ? 36 : 35;
         // a warp per two vectors once there are 8 or more vectors per SM (static
         // couplings; 1024-site lattice, 1185 vectors: 39.3 against 43.9 ms),
         // else a warp per vector (C4's 585-vector jobs: 18.6 against 25.5 ms at
@@ -264,6 +285,9 @@ struct AbsRun {
     DevBuf<char> U, rot;
     DevBuf<int> lvptr, lvchk;  // level bounds; the same split into chunks of at most 32
     int nlev = 0, nchk = 0;
+    DevBuf<uint32_t> row_ab[2];  // rows of 32 and of 64 operations
+    DevBuf<uint16_t> row_id[2];
+    RowPlan row[2] = {};
     TrotterPlan TP;
     // RK4
     DevBuf<int2> dent;
@@ -426,6 +450,19 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
         TP.pairs = dpairs.p;
         TP.U = U.p;
         TP.rot = rot.p;
+        // the whole step as rows, from the level order (every site's order is
+        // the same), for the sizes default_config takes them at, or on demand
+        const bool asked = p.kernel_config == 35 || p.kernel_config == 36;
+        const bool rows_ok = p.kernel_config == 0 && N <= (TP.rot_static ? 400 : 128);
+        if ((asked || rows_ok) && N + 64 <= NISE_ROW_MAX && TP.k <= NISE_ROW_MAX && p.ts >= 1)
+            for (int w = 0; w < 2; w++) {
+                std::vector<uint32_t> ab;
+                std::vector<uint16_t> id;
+                row[w].nrow = nise_row_schedule(lpairs, N, p.ts, 32 * (w + 1), ab, id);
+                if ((rc = row_ab[w].upload(c, ab)) || (rc = row_id[w].upload(c, id))) return rc;
+                row[w].ab = row_ab[w].p;
+                row[w].id = row_id[w].p;
+            }
     } else if (p.propagation == NISE_PROP_RK4) {
         scheme = SCHEME_RK4;
         std::vector<int2> pairs, ent;
@@ -827,14 +864,19 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
                 return rc;
         }
     }
+    int nrows[2] = {0, 0};
+    if (scheme == SCHEME_TROTTER)
+        for (int w = 0; w < 2; w++)
+            if (trotter_rows_fit(prec == NISE_FP32 ? 0 : 1, TP, row[w], 32 * (w + 1))) nrows[w] = row[w].nrow;
     config = default_config(scheme, N, plain, cheb, TP.k, nchk, plain ? 3 : nvec, dell4.p != nullptr,
                             scheme == SCHEME_TAYLOR && taylor_rv_fits(T, XP),
-                            scheme == SCHEME_TROTTER && TP.rot_static);
+                            scheme == SCHEME_TROTTER && TP.rot_static, nrows, (long)p.ts * (TP.k + 2L * N));
     if (p.kernel_config != 0) {  // forced by the caller
         const int k = p.kernel_config;
         if (scheme == SCHEME_EIGEN && (k == 2 || k == 16 || k == 17)) return NISE_OK;
         if (scheme == SCHEME_TROTTER &&
-            (k == 1 || k == 32 || k == 33 || (k == 34 && TP.rot_static) || k == 64 || k == 128 || k == 256))
+            (k == 1 || k == 32 || k == 33 || (k == 34 && TP.rot_static) || k == 64 || k == 128 || k == 256 ||
+             ((k == 35 || k == 36) && trotter_rows_fit(prec == NISE_FP32 ? 0 : 1, TP, row[k - 35], 32 * (k - 34)))))
             config = k == 1 ? 0 : k;
         else if (scheme == SCHEME_TAYLOR &&
                  (k == 3 || k == 8 || k == 9 || (k == 10 && cheb) || (k == 12 && dell4.p) || k == 13 || k == 14 ||
@@ -889,6 +931,8 @@ int AbsRun::run_main(cudaStream_t s, int cfg, double2 *dst) {
         case SCHEME_TROTTER:
             if (cfg == 32 || cfg == 33) return launch_abs_trotter_wv(pr, T, TP, Js, r, lvchk.p, nchk, cfg == 32, s);
             if (cfg == 34) return launch_abs_trotter_wv2(pr, T, TP, Js, r, lvchk.p, nchk, s);
+            if (cfg == 35 || cfg == 36)
+                return launch_abs_trotter_rows(pr, T, TP, row[cfg - 35], cfg == 36 ? 64 : 32, Js, r, s);
             if (cfg > 0) return launch_abs_trotter_lv(pr, T, TP, Js, r, lvptr.p, nlev, cfg, s);
             return launch_abs_trotter(pr, T, TP, Js, r, s);
         case SCHEME_RK4:
@@ -957,6 +1001,8 @@ int AbsRun::tune() {
     if (scheme == SCHEME_TROTTER) {
         cand = {0, 32, 33, 64, 128, 256};
         if (TP.rot_static) cand.push_back(34);
+        for (int w = 0; w < 2; w++)
+            if (trotter_rows_fit(prec == NISE_FP32 ? 0 : 1, TP, row[w], 32 * (w + 1))) cand.push_back(35 + w);
     } else {
         cand = {3, -8, 8, 13, 14};
         if (cheb) cand.push_back(10);

@@ -27,9 +27,11 @@ struct DevTraj {
     float cut;               // Couplingcut
 };
 
-// Rows of a Trotter time step (nise_row_schedule) in device memory.
+// Rows of a Trotter time step (nise_row_schedule) in device memory: the sites
+// and the coefficient of each place.
 struct RowPlan {
-    const uint2 *rows;
+    const unsigned int *ab;
+    const unsigned short *id;
     int nrow;
 };
 

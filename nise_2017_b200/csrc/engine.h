@@ -127,6 +127,11 @@ int launch_abs_trotter_wv(int prec, const DevTraj &T, const TrotterPlan &P, cons
 // bitwise identical to launch_abs_trotter_wv.
 int launch_abs_trotter_wv2(int prec, const DevTraj &T, const TrotterPlan &P, const AbsJob &J, double2 *resp,
                            const int *chk, int nchk, cudaStream_t s);
+// The same from rows of 32 or 64 operations (nise_row_schedule of P.pairs),
+// bitwise identical to all of these; whether one vector fits shared memory.
+bool trotter_rows_fit(int prec, const TrotterPlan &P, const RowPlan &Q, int width);
+int launch_abs_trotter_rows(int prec, const DevTraj &T, const TrotterPlan &P, const RowPlan &Q, int width,
+                            const AbsJob &J, double2 *resp, cudaStream_t s);
 int launch_prep_rk4(int prec, const DevTraj &T, const Rk4Plan &P, double fsub, float fsub32, cudaStream_t s);
 int launch_abs_rk4(int prec, const DevTraj &T, const Rk4Plan &P, const AbsJob &J, double2 *resp, cudaStream_t s);
 // The same with a thread per site row (rk4.cu; P.rows set, at most

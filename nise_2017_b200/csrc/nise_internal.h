@@ -1,6 +1,7 @@
 // Engine-internal host definitions shared by api.cpp and the 2D driver.
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 #include <memory>
 #include <string>
@@ -107,8 +108,9 @@ struct SinglesBufs {
     DevBuf<int2> pairs, ent;
     DevBuf<int4> segs;
     DevBuf<char> U, rot, rkval;
-    DevBuf<uint2> rows;
-    RowPlan row = {nullptr, 0};  // the Trotter step's rows of 32 (none above 65503 sites)
+    DevBuf<uint32_t> row_ab;
+    DevBuf<uint16_t> row_id;
+    RowPlan row = {nullptr, nullptr, 0};  // the Trotter step's rows of 32 (none above NISE_ROW_MAX couplings or sites)
     const void *Us = nullptr;
 };
 

@@ -42,7 +42,8 @@ void nise_schedule_parts(const std::vector<int2> &pairs, int n, std::vector<uint
         if (first[a] < 0) iso.push_back(a);
 }
 
-int nise_row_schedule(const std::vector<int2> &pairs, int n, int ts, int width, std::vector<uint2> &rows) {
+int nise_row_schedule(const std::vector<int2> &pairs, int n, int ts, int width, std::vector<uint32_t> &ab,
+                      std::vector<uint16_t> &id) {
     std::vector<int> ready(n, 0);               // first row after the site's last operation
     std::vector<std::vector<uint2>> row;
     std::vector<int> next;                      // next[r]: a row >= r that may have room (path-compressed)
@@ -63,12 +64,14 @@ int nise_row_schedule(const std::vector<int2> &pairs, int n, int ts, int width, 
         for (int a = 0; a < n; a++) place(a, a, NISE_ROW_PHASE | (uint32_t)a);
     }
     const int nrow = (int)row.size();
-    rows.clear();
+    ab.clear();
+    id.clear();
     for (int r = 0; r < nrow + 2; r++)
         for (int i = 0; i < width; i++) {
-            const uint32_t spare = (uint32_t)(n + i % 32);
-            rows.push_back(r < nrow && i < (int)row[r].size() ? row[r][i]
-                                                              : make_uint2(spare | spare << 16, NISE_ROW_PHASE | (uint32_t)n));
+            const uint32_t spare = (uint32_t)(n + i);
+            const bool op = r < nrow && i < (int)row[r].size();
+            ab.push_back(op ? row[r][i].x : spare | spare << 16);
+            id.push_back((uint16_t)(op ? row[r][i].y : NISE_ROW_PHASE | (uint32_t)n));
         }
     return nrow;
 }

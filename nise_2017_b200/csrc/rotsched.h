@@ -46,10 +46,12 @@ void nise_schedule_parts(const std::vector<int2> &pairs, int n, std::vector<uint
 // same float operations in the same order as propagate.c:870-873).  One step is
 // `ts` times all phases, the rotations in order, all phases; every operation
 // goes to the first row after the rows of the earlier operations on its sites
-// that has room, so each site sees them in the reference's order.  x = a | b <<
-// 16; y = index into the rotation coefficients, or NISE_ROW_PHASE | site.  Idle
-// places rotate a spare site of their own, n + (place mod 32), by the phase at
-// index n, which the caller sets to (1, 0).  Two idle rows follow the last (a
+// that has room, so each site sees them in the reference's order.  ab = a | b <<
+// 16; id = index into the rotation coefficients, or NISE_ROW_PHASE | site (six
+// bytes a place: the schedule of a 500-site lattice fits shared memory).  Idle
+// places rotate a spare site of their own, n + place, by the phase at index n, which the caller sets to (1, 0).  Two idle rows follow the last (a
 // kernel reads two rows ahead).  Returns the number of rows without them.
-#define NISE_ROW_PHASE 0x80000000u
-int nise_row_schedule(const std::vector<int2> &pairs, int n, int ts, int width, std::vector<uint2> &rows);
+#define NISE_ROW_PHASE 0x8000u
+#define NISE_ROW_MAX 0x7fff  // couplings, and sites
+int nise_row_schedule(const std::vector<int2> &pairs, int n, int ts, int width, std::vector<uint32_t> &ab,
+                      std::vector<uint16_t> &id);

@@ -1,4 +1,4 @@
-// One Trotter time step of a vector on a warp, from the rows of
+// One Trotter time step of a vector on a warp (or two), from the rows of
 // nise_row_schedule: the lanes apply the operations of a row (rotations and
 // half-step phases alike, both 2x2 on two sites of the state in shared memory), a
 // __syncwarp separates the rows.  Sub-steps overlap as far as the couplings
@@ -15,128 +15,129 @@
 
 // The coefficients of an entry, from the frame's rotations and phases.
 template <typename R>
-__device__ __forceinline__ typename Vec2<R>::T row_coef(uint32_t y, const typename Vec2<R>::T *rot,
+__device__ __forceinline__ typename Vec2<R>::T row_coef(unsigned y, const typename Vec2<R>::T *rot,
                                                         const typename Vec2<R>::T *ph) {
     return ((y & NISE_ROW_PHASE) ? ph : rot)[y & ~NISE_ROW_PHASE];
 }
 
-// X [n + 32] state (the last 32 spare), rot the rotations' (co, si), ph [n + 1]
-// the phases and (1, 0); I entries per lane and row.
-template <typename R, int I>
-__device__ __forceinline__ void rows_step(typename Vec2<R>::T *X, const uint2 *rows, int nrow, int lane,
+// The threads of a vector: one warp, or two on rows of 64 (a named barrier
+// separates the rows then; id 1 and up, 0 is __syncthreads).
+template <int TW> __device__ __forceinline__ void rows_sync(int bar) {
+    if (TW == 1) __syncwarp();
+    else asm volatile("bar.sync %0, 64;" ::"r"(bar) : "memory");
+}
+
+// X [n + 32 TW] state (the last ones spare), rot the rotations' (co, si), ph [n +
+// 1] the phases and (1, 0); thread th of the vector, rows of 32 TW places.
+template <typename R, int TW>
+__device__ __forceinline__ void rows_step(typename Vec2<R>::T *X, const RowPlan &Q, int th, int bar,
                                           const typename Vec2<R>::T *rot, const typename Vec2<R>::T *ph) {
     typedef typename Vec2<R>::T R2;
     typedef Ar<R> A;
-    uint2 e0[I], e1[I];
-    R2 c0[I];
-#pragma unroll
-    for (int i = 0; i < I; i++) {
-        e0[i] = rows[32 * i + lane];
-        e1[i] = rows[32 * (I + i) + lane];
-        c0[i] = row_coef<R>(e0[i].y, rot, ph);
-    }
-    const uint2 *next = rows + 64 * I + lane;
+    constexpr int W = 32 * TW;
+    const unsigned *ab = Q.ab + th;
+    const unsigned short *id = Q.id + th;
+    unsigned s0 = ab[0], y1 = id[W];
+    R2 c0 = row_coef<R>(id[0], rot, ph);
+    ab += W;
+    id += 2 * W;
 #pragma unroll 2
-    for (int r = 0; r < nrow; r++, next += 32 * I) {
-        R2 xa[I], xb[I], c1[I];
-#pragma unroll
-        for (int i = 0; i < I; i++) {
-            xa[i] = X[e0[i].x & 0xffff];
-            xb[i] = X[e0[i].x >> 16];
-        }
-        uint2 e2[I];
-#pragma unroll
-        for (int i = 0; i < I; i++) {
-            e2[i] = next[32 * i];
-            c1[i] = row_coef<R>(e1[i].y, rot, ph);
-        }
-#pragma unroll
-        for (int i = 0; i < I; i++) {  // propagate.c:883-886
-            R2 ya, yb;
-            ya.x = A::sub(A::mul(c0[i].x, xa[i].x), A::mul(c0[i].y, xb[i].y));
-            ya.y = A::add(A::mul(c0[i].x, xa[i].y), A::mul(c0[i].y, xb[i].x));
-            yb.x = A::sub(A::mul(c0[i].x, xb[i].x), A::mul(c0[i].y, xa[i].y));
-            yb.y = A::add(A::mul(c0[i].x, xb[i].y), A::mul(c0[i].y, xa[i].x));
-            X[e0[i].x & 0xffff] = ya;
-            X[e0[i].x >> 16] = yb;
-        }
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < I; i++) {
-            e0[i] = e1[i];
-            e1[i] = e2[i];
-            c0[i] = c1[i];
-        }
+    for (int r = 0; r < Q.nrow; r++, ab += W, id += W) {
+        R2 *pa = X + (s0 & 0xffff), *pb = X + (s0 >> 16);
+        const R2 xa = *pa, xb = *pb;
+        const unsigned s1 = ab[0], y2 = id[0];
+        const R2 c1 = row_coef<R>(y1, rot, ph);
+        R2 ya, yb;  // propagate.c:883-886
+        ya.x = A::sub(A::mul(c0.x, xa.x), A::mul(c0.y, xb.y));
+        ya.y = A::add(A::mul(c0.x, xa.y), A::mul(c0.y, xb.x));
+        yb.x = A::sub(A::mul(c0.x, xb.x), A::mul(c0.y, xa.y));
+        yb.y = A::add(A::mul(c0.x, xb.y), A::mul(c0.y, xa.x));
+        *pa = ya;
+        *pb = yb;
+        rows_sync<TW>(bar);
+        s0 = s1;
+        y1 = y2;
+        c0 = c1;
     }
 }
 
-// A warp's shared memory for rows_step: the state, the frame's phases and,
+// A vector's shared memory for rows_step: the state, the frame's phases and,
 // with per-frame couplings, its rotations.
-template <typename R> __host__ __device__ __forceinline__ size_t rows_warp_elems(int n, int K, bool rot_static) {
-    return (size_t)(n + 32) + (n + 1) + (rot_static ? 0 : K);
+template <typename R> __host__ __device__ __forceinline__ size_t rows_vec_elems(int n, int K, bool rot_static, int TW) {
+    return (size_t)(n + 32 * TW) + (n + 1) + (rot_static ? 0 : K);
 }
 
-// The step of a SinglesTab's Trotter tables through frame row fi; the warp's
+// The step of a SinglesTab's Trotter tables through frame row fi; the vector's
 // shared memory w (X first), rs the static rotations in shared memory.
-template <typename R>
-__device__ __forceinline__ void rows_singles_step(const SinglesTab &D, const uint2 *rows, int nrow, typename Vec2<R>::T *w,
-                                                  const typename Vec2<R>::T *rs, int lane, long fi) {
+template <typename R, int TW>
+__device__ __forceinline__ void rows_singles_step(const SinglesTab &D, const RowPlan &Q, typename Vec2<R>::T *w,
+                                                  const typename Vec2<R>::T *rs, int th, int bar, long fi) {
     typedef typename Vec2<R>::T R2;
+    constexpr int W = 32 * TW;
     const int n = D.n;
-    R2 *ph = w + n + 32, *rot = ph + n + 1;
+    R2 *ph = w + n + W, *rot = ph + n + 1;
     const R2 *U = (const R2 *)D.U + fi * n;
-    __syncwarp();
+    rows_sync<TW>(bar);
 #pragma unroll 2
-    for (int a = lane; a < n; a += 32) ph[a] = U[a];
+    for (int a = th; a < n; a += W) ph[a] = U[a];
     if (!D.rot_static) {
         const R2 *src = (const R2 *)D.rot + fi * D.K;
 #pragma unroll 4
-        for (int k = lane; k < D.K; k += 32) rot[k] = src[k];
+        for (int k = th; k < D.K; k += W) rot[k] = src[k];
         rs = rot;
     }
-    __syncwarp();
-    rows_step<R, 1>(w, rows, nrow, lane, rs, ph);
+    rows_sync<TW>(bar);
+    rows_step<R, TW>(w, Q, th, bar, rs, ph);
 }
 
-// A CTA of warps on rows_singles_step: the schedule (STAGE) and the static
-// rotations in shared memory, then the warps' parts.
-template <typename R>
-__device__ __forceinline__ typename Vec2<R>::T *rows_setup(const SinglesTab &D, const RowPlan &Q, bool stage,
-                                                           unsigned char *smem, const uint2 *&rows,
-                                                           const typename Vec2<R>::T *&rs) {
+// A CTA of vectors on rows_singles_step: the schedule (where `stage`; Q then
+// points to it) and the static rotations in shared memory, then the vectors' parts.
+template <typename R, int TW>
+__device__ __forceinline__ typename Vec2<R>::T *rows_setup(const SinglesTab &D, RowPlan &Q, bool stage,
+                                                           unsigned char *smem, const typename Vec2<R>::T *&rs) {
     typedef typename Vec2<R>::T R2;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ne = 32 * (Q.nrow + 2);
-    uint2 *es = (uint2 *)smem;
-    R2 *rsh = (R2 *)(smem + (stage ? sizeof(uint2) * (size_t)ne : 0));
+    constexpr int W = 32 * TW;
+    const int vec = threadIdx.x / W, th = threadIdx.x % W, ne = W * (Q.nrow + 2);
+    unsigned *as = (unsigned *)smem;
+    unsigned short *is = (unsigned short *)(as + ne);
+    R2 *rsh = (R2 *)(smem + (stage ? 6 * (size_t)ne : 0));
     const int Ks = D.rot_static ? D.K : 0;
-    if (stage)
-        for (int e = threadIdx.x; e < ne; e += blockDim.x) es[e] = Q.rows[e];
+    if (stage) {
+        for (int e = threadIdx.x; e < ne; e += blockDim.x) {
+            as[e] = Q.ab[e];
+            is[e] = Q.id[e];
+        }
+        Q.ab = as;
+        Q.id = is;
+    }
     for (int k = threadIdx.x; k < Ks; k += blockDim.x) rsh[k] = ((const R2 *)D.rot)[k];
-    R2 *w = rsh + Ks + warp * rows_warp_elems<R>(D.n, D.K, D.rot_static);
+    R2 *w = rsh + Ks + vec * rows_vec_elems<R>(D.n, D.K, D.rot_static, TW);
     R2 z;
     z.x = z.y = 0;
-    w[D.n + lane] = z;  // the spare sites
+    w[D.n + th] = z;  // the spare sites
     z.x = 1;
-    if (lane == 0) w[2 * D.n + 32] = z;  // their phase
+    if (th == 0) w[2 * D.n + W] = z;  // their phase
     __syncthreads();
-    rows = stage ? es : Q.rows;
     rs = rsh;
     return w;
 }
 
-// Launch shape: warps per CTA and shared memory; 0 warps if a vector does not fit.
+// Launch shape: vectors per CTA and shared memory; 0 vectors if one does not fit.
 struct RowShape {
-    int warps, stage;
+    int vecs, stage;
     size_t bytes;
 };
-template <typename R> inline RowShape rows_shape(int n, int K, bool rot_static, int nrow, long vectors, int sms) {
-    const size_t r2 = sizeof(typename Vec2<R>::T), ent = sizeof(uint2) * 32 * (size_t)(nrow + 2);
-    const size_t per = r2 * rows_warp_elems<R>(n, K, rot_static), rot = rot_static ? r2 * K : 0;
+template <typename R> inline RowShape rows_shape(int n, int K, bool rot_static, int nrow, int TW, long vectors, int sms) {
+    const size_t r2 = sizeof(typename Vec2<R>::T), ent = 192 * (size_t)TW * (nrow + 2), lim = 226 * 1024;
+    const size_t per = r2 * rows_vec_elems<R>(n, K, rot_static, TW), rot = rot_static ? r2 * K : 0;
+    const long want = std::min<long>(8 / TW, (vectors + sms - 1) / sms);
     RowShape s;
-    s.stage = ent + rot + per <= 220 * 1024 && ent <= 128 * 1024;
+    // the schedule is staged where that leaves the wanted vectors their place, or
+    // at least four of them (it is read again every step)
+    s.stage = ent + rot + std::min<long>(want, 4) * per <= lim;
     const size_t base = rot + (s.stage ? ent : 0);
-    s.warps = (int)std::min<long>(8, (vectors + sms - 1) / sms);
-    while (s.warps > 0 && base + s.warps * per > 220 * 1024) s.warps--;
-    s.bytes = base + s.warps * per;
+    s.vecs = (int)want;
+    while (s.vecs > 0 && base + s.vecs * per > lim) s.vecs--;
+    s.bytes = base + s.vecs * per;
     return s;
 }

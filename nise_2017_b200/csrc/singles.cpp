@@ -65,12 +65,14 @@ int nise_singles_tables(nise_ctx *c, const DevTraj &T, long fmin, long nf, int s
         c->launches += 1 + P.rot_static;
         S.U = B.U.p;
         S.rot = B.rot.p;
-        if (N + 32 <= 0xffff && p.ts >= 1) {
-            std::vector<uint2> rows;
+        if (N + 64 <= NISE_ROW_MAX && K <= NISE_ROW_MAX && p.ts >= 1) {
+            std::vector<uint32_t> ab;
+            std::vector<uint16_t> id;
             pairs.pop_back();
-            B.row.nrow = nise_row_schedule(pairs, N, p.ts, 32, rows);
-            if ((rc = B.rows.upload(c, rows))) return rc;
-            B.row.rows = B.rows.p;
+            B.row.nrow = nise_row_schedule(pairs, N, p.ts, 32, ab, id);
+            if ((rc = B.row_ab.upload(c, ab)) || (rc = B.row_id.upload(c, id))) return rc;
+            B.row.ab = B.row_ab.p;
+            B.row.id = B.row_id.p;
         }
     } else if (p.propagation == NISE_PROP_SPARSE || p.propagation == NISE_PROP_DIAGONAL) {
         // propagate_vector's Sparse scheme (DIA, or DIA_S when 0 < Threshold

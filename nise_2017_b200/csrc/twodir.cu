@@ -255,9 +255,8 @@ template <typename R>
 __global__ void __launch_bounds__(256) k2d_gb1_rows(TwoD D, RowPlan Q, int stage) {
     typedef typename Vec2<R>::T R2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const uint2 *rows;
     const R2 *rs;
-    R2 *X = rows_setup<R>(D, Q, stage, smem_raw, rows, rs);
+    R2 *X = rows_setup<R, 1>(D, Q, stage, smem_raw, rs);
     const int n = D.n, lane = threadIdx.x & 31, P = (D.T1 + 1) / 2;
     const int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (g >= D.S * 3 * P) return;
@@ -267,7 +266,7 @@ __global__ void __launch_bounds__(256) k2d_gb1_rows(TwoD D, RowPlan Q, int stage
         const int t1 = pass == 0 ? p : D.T1 - 1 - p;
         if (pass == 1 && t1 == p) break;
         for (int i = lane; i < n; i += 32) X[i] = make_vec2<R>((R)traj_mu(D.T, tj - t1, x, i), 0);
-        for (int tm = 0; tm < t1; tm++) rows_singles_step<R>(D, rows, Q.nrow, X, rs, lane, tj - t1 + tm - D.f0);
+        for (int tm = 0; tm < t1; tm++) rows_singles_step<R, 1>(D, Q, X, rs, lane, 0, tj - t1 + tm - D.f0);
         __syncwarp();
         R2 *out = (R2 *)D.L + (((size_t)s * 3 + x) * D.T1 + t1) * n;
         for (int i = lane; i < n; i += 32) out[i] = X[i];
@@ -284,9 +283,8 @@ template <typename R>
 __global__ void __launch_bounds__(256) k2d_gb3_rows(TwoD D, RowPlan Q, int stage) {
     typedef typename Vec2<R>::T R2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const uint2 *rows;
     const R2 *rs;
-    R2 *X = rows_setup<R>(D, Q, stage, smem_raw, rows, rs);
+    R2 *X = rows_setup<R, 1>(D, Q, stage, smem_raw, rs);
     const int lane = threadIdx.x & 31, g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (g >= D.S * 3) return;
     const int s = g / 3, x = g % 3;
@@ -298,7 +296,7 @@ __global__ void __launch_bounds__(256) k2d_gb3_rows(TwoD D, RowPlan Q, int stage
             const double2 z = rows_dot<R>(D, tk + t3, p3, X, lane);
             if (lane == 0) D.gbt3[(((size_t)s * 3 + x) * 3 + p3) * D.T3 + t3] = z;
         }
-        if (t3 < D.T3 - 1) rows_singles_step<R>(D, rows, Q.nrow, X, rs, lane, tk + t3 - D.f0);
+        if (t3 < D.T3 - 1) rows_singles_step<R, 1>(D, Q, X, rs, lane, 0, tk + t3 - D.f0);
     }
 }
 
@@ -306,9 +304,8 @@ template <typename R>
 __global__ void __launch_bounds__(256) k2d_se_rows(TwoD D, RowPlan Q, int stage) {
     typedef typename Vec2<R>::T R2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const uint2 *rows;
     const R2 *rs;
-    R2 *X = rows_setup<R>(D, Q, stage, smem_raw, rows, rs);
+    R2 *X = rows_setup<R, 1>(D, Q, stage, smem_raw, rs);
     const int n = D.n, NV = nvec_se(D), lane = threadIdx.x & 31, g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (g >= D.S * NV) return;
     const int s = g / NV, v = g % NV;
@@ -320,16 +317,16 @@ __global__ void __launch_bounds__(256) k2d_se_rows(TwoD D, RowPlan Q, int stage)
         __syncwarp();
         R2 *snap = (R2 *)D.SE + (((size_t)s * D.T3 + t3) * NV + v) * n;
         for (int i = lane; i < n; i += 32) snap[i] = X[i];
-        if (t3 < D.T3 - 1) rows_singles_step<R>(D, rows, Q.nrow, X, rs, lane, tk + t3 - D.f0);
+        if (t3 < D.T3 - 1) rows_singles_step<R, 1>(D, Q, X, rs, lane, 0, tk + t3 - D.f0);
     }
 }
 
 template <typename R, typename Kern>
 int run_rows(Kern kern, const TwoD &D, const RowPlan &Q, long vectors, cudaStream_t st) {
-    const RowShape h = rows_shape<R>(D.n, D.K, D.rot_static, Q.nrow, vectors, sm_count());
-    if (!h.warps) return (int)cudaErrorNotSupported;
+    const RowShape h = rows_shape<R>(D.n, D.K, D.rot_static, Q.nrow, 1, vectors, sm_count());
+    if (!h.vecs) return (int)cudaErrorNotSupported;
     if (const int e = (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.bytes)) return e;
-    kern<<<(unsigned)((vectors + h.warps - 1) / h.warps), 32 * h.warps, h.bytes, st>>>(D, Q, h.stage);
+    kern<<<(unsigned)((vectors + h.vecs - 1) / h.vecs), 32 * h.vecs, h.bytes, st>>>(D, Q, h.stage);
     return (int)cudaGetLastError();
 }
 
@@ -2012,7 +2009,7 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf, const RowPlan &Q) {
     if ((e = smem_attr(k2d_gb3<R>, sm))) return e;
     if ((e = smem_attr(k2d_se<R>, sm))) return e;
     // Trotter: a warp per vector where its state and tables fit shared memory
-    const bool rows = Q.rows && rows_shape<R>(D.n, D.K, D.rot_static, Q.nrow, 1, 1).warps > 0;
+    const bool rows = Q.ab && rows_shape<R>(D.n, D.K, D.rot_static, Q.nrow, 1, 1, 1).vecs > 0;
     if (rows) {
         if ((e = run_rows<R>(k2d_gb1_rows<R>, D, Q, (long)D.S * 3 * P, st))) return e;
     } else {

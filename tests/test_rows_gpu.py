@@ -42,3 +42,25 @@ def test_2d_singles(n, geometry, ham, cut, tmp_path):
         want, wcount = oracle.twodir(oracle.params(kw, files), build)
         assert count == wcount
         assert helpers.rel2d(response, want) < tol
+
+
+@pytest.mark.parametrize("n, geometry, ham, cut", SYSTEMS)
+def test_absorption_default_and_forced(n, geometry, ham, cut, tmp_path):
+    """The default configuration, rows of 32 and rows of 64 (35, 36) against the thread per vector (1)."""
+    files = trajectory(tmp_path, n, geometry, ham, 60, 700 + n)
+    kw = synth.c0_keywords(Singles=n, Length=60, RunTimes="9 0 0", Samplerate=13, HamiltonianType=ham, Couplingcut=cut)
+    for precision, build in ((nise.FP32, "f32a64"), (nise.FP64, "f64")):
+        got = {}
+        for config in (0, 1, 35, 36):
+            with nise.Context(nise.params_from_keywords(kw, files, precision=precision, kernel_config=config)) as c:
+                c.load_files()
+                re, im, count = c.absorption()
+            got[config] = re + 1j * im
+        ore, oim, ocount = oracle.absorption(oracle.params(kw, files), build)
+        assert count == ocount
+        assert helpers.rel(got[1], ore + 1j * oim) < 1e-11
+        for config in (0, 35, 36):
+            if precision == nise.FP32:
+                assert (got[config] == got[1]).all()
+            else:
+                assert helpers.rel(got[config], got[1]) < FP64
