@@ -35,6 +35,7 @@
 #include "eigen.h"
 #include "engine.h"
 #include "nise_internal.h"
+#include "rows.cuh"
 #include "schemes.cuh"
 
 namespace {
@@ -167,6 +168,34 @@ __global__ void k_lin(LinJob J) {
         const long tj = ti + t1;
         for (int r = 0; r < J.nread; r++) out[(size_t)r * J.tmax + t1] = lin_read<R>(J, v, r, tj, S, B, lane);
         if (t1 < J.tmax - 1) singles_step<R>(J, S, B, lane, tj);
+    }
+}
+
+// The same for the Trotter scheme with a warp per vector on rows of operations
+// (rows.cuh), the operations of trotter_apply; lane r takes read-out r.
+template <typename R>
+__global__ void __launch_bounds__(256) k_lin_rows(LinJob J, RowPlan Q, int stage) {
+    typedef typename Vec2<R>::T R2;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const R2 *rs;
+    R2 *X = rows_setup<R, 1>(J, Q, stage, smem_raw, rs);
+    const int lane = threadIdx.x & 31;
+    const long g = blockIdx.x * (long)(blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (g >= (long)J.S * J.nvec) return;
+    const int s = (int)(g / J.nvec), v = (int)(g % J.nvec);
+    const long ti = (long)(J.begin + s) * J.sample;
+    for (int i = lane; i < J.n; i += 32) {
+        R2 z;
+        z.x = (R)lin_init(J, s, v, ti, i);
+        z.y = 0;
+        X[i] = z;
+    }
+    double2 *out = J.part + ((size_t)s * J.nvec + v) * J.nread * J.tmax;
+    for (int t1 = 0; t1 < J.tmax; t1++) {
+        const long tj = ti + t1;
+        __syncwarp();
+        if (lane < J.nread) out[(size_t)lane * J.tmax + t1] = lin_read<R>(J, v, lane, tj, X, 1, 0);
+        if (t1 < J.tmax - 1) rows_singles_step<R, 1>(J, Q, X, rs, lane, 0, tj - J.f0);
     }
 }
 
@@ -397,7 +426,7 @@ __global__ void k_lum_itime(DevTraj T, DevTraj T0, int n, int sample, int begin,
 }
 
 template <typename R>
-int run_lin(const LinJob &J, double2 *out, int nch, int first, cudaStream_t st) {
+int run_lin(const LinJob &J, const RowPlan &Q, double2 *out, int nch, int first, cudaStream_t st) {
     const long nv = (long)J.S * J.nvec;
     int e;
     if (is_eigen_scheme(J.prop)) {
@@ -410,6 +439,14 @@ int run_lin(const LinJob &J, double2 *out, int nch, int first, cudaStream_t st) 
         if ((e = (int)cudaFuncSetAttribute(k_lin_dia<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(VG * row))))
             return e;
         k_lin_dia<R><<<(unsigned)(J.S * ((J.nvec + VG - 1) / VG)), nw + nr, VG * row, st>>>(J, VG, nr);
+    } else if (Q.ab && (double)nv * Q.nrow < 860.0 * J.ts * (J.K + 2.0 * J.n) &&
+               rows_shape<R>(J.n, J.K, J.rot_static, Q.nrow, 1, nv, sm_count()).vecs > 0) {
+        // Trotter: a warp per vector, until the vectors fill threads (the same
+        // line as for absorption)
+        const RowShape h = rows_shape<R>(J.n, J.K, J.rot_static, Q.nrow, 1, nv, sm_count());
+        if ((e = (int)cudaFuncSetAttribute(k_lin_rows<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.bytes)))
+            return e;
+        k_lin_rows<R><<<(unsigned)((nv + h.vecs - 1) / h.vecs), 32 * h.vecs, h.bytes, st>>>(J, Q, h.stage);
     } else {
         size_t lane_b = singles_lane_bytes<R>(J.n, J.prop);
         int B = 64;
@@ -658,8 +695,8 @@ extern "C" int nise_linear(nise_ctx *c, double *re_S, double *im_S, int max_chan
     for (int s0 = begin; s0 < end; s0 += chunk) {
         J.begin = s0;
         J.S = std::min(chunk, end - s0);
-        int e = p.precision == NISE_FP32 ? run_lin<float>(J, out.p, L.nch, s0 == begin, c->stream)
-                                         : run_lin<double>(J, out.p, L.nch, s0 == begin, c->stream);
+        int e = p.precision == NISE_FP32 ? run_lin<float>(J, SB.row, out.p, L.nch, s0 == begin, c->stream)
+                                         : run_lin<double>(J, SB.row, out.p, L.nch, s0 == begin, c->stream);
         if ((rc = nise_cuda(c, e, "linear technique kernels"))) return rc;
         c->launches += 2;
     }

@@ -64,3 +64,19 @@ def test_absorption_default_and_forced(n, geometry, ham, cut, tmp_path):
                 assert (got[config] == got[1]).all()
             else:
                 assert helpers.rel(got[config], got[1]) < FP64
+
+
+@pytest.mark.parametrize("tech", ["LD", "DOS", "CD"])
+@pytest.mark.parametrize("n, geometry, ham, cut", [SYSTEMS[1], SYSTEMS[3], SYSTEMS[4], SYSTEMS[5]])
+def test_linear_techniques(tech, n, geometry, ham, cut, tmp_path):
+    files = trajectory(tmp_path, n, geometry, ham, 40, 800 + n)
+    files.update(synth.write_positions(str(tmp_path), n, 40, seed=n))
+    kw = synth.c0_keywords(Singles=n, Length=40, RunTimes="7 0 0", Samplerate=15, HamiltonianType=ham, Couplingcut=cut,
+                           Technique=tech)
+    for precision, build in ((nise.FP32, "f32a64"), (nise.FP64, "f64")):
+        with nise.Context(nise.params_from_keywords(kw, files, precision=precision)) as c:
+            c.load_files()
+            re, im, count = c.linear()
+        want = oracle.linear(oracle.params(kw, files), build)
+        assert count == want[2]
+        assert helpers.rel(re + 1j * im, want[0] + 1j * want[1]) < SUM_ORDER
