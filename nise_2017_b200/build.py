@@ -40,6 +40,7 @@ CU_SOURCES = [
     "rk4.cu",
     "propagators.cu",
     "trotter_rows.cu",
+    "steps.cu",
 ]
 CPP_SOURCES = [
     "api.cpp",

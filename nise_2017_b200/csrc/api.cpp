@@ -708,17 +708,24 @@ extern "C" int nise_propagate(nise_ctx *c, const float *H, void *re, void *im, i
     cudaMemcpyAsync(dH.p, H, sizeof(float) * nvec * c->nn2, cudaMemcpyHostToDevice, c->stream);
     cudaMemcpyAsync(dr.p, re, rsz * nvec * N, cudaMemcpyHostToDevice, c->stream);
     cudaMemcpyAsync(di.p, im, rsz * nvec * N, cudaMemcpyHostToDevice, c->stream);
+    // a CTA per vector; a thread per vector where that does not fit
+    const double f64 = nise_f64(p, sign, p.ts);
+    const float f32 = nise_f32(p, sign, p.ts);
     int e;
-    if (p.propagation == NISE_PROP_COUPLING)
-        e = launch_step_coupling(prec, N, p.couplingcut, dH.p, dr.p, di.p, nvec, p.ts, nise_f64(p, sign, p.ts),
-                                 nise_f32(p, sign, p.ts), c->stream);
-    else if (p.propagation == NISE_PROP_RK4)
-        e = launch_step_rk4(prec, N, p.couplingcut, dH.p, dr.p, di.p, nvec, p.ts, nise_f64(p, sign, p.ts),
-                            nise_f32(p, sign, p.ts), c->stream);
-    else {
+    if (p.propagation == NISE_PROP_COUPLING) {
+        e = launch_step_coupling_cta(prec, N, p.couplingcut, dH.p, dr.p, di.p, nvec, p.ts, f64, f32, c->stream);
+        if (e == (int)cudaErrorNotSupported)
+            e = launch_step_coupling(prec, N, p.couplingcut, dH.p, dr.p, di.p, nvec, p.ts, f64, f32, c->stream);
+    } else if (p.propagation == NISE_PROP_RK4) {
+        e = launch_step_rk4_row(prec, N, p.couplingcut, dH.p, dr.p, di.p, nvec, p.ts, f64, f32, c->stream);
+        if (e == (int)cudaErrorNotSupported)
+            e = launch_step_rk4(prec, N, p.couplingcut, dH.p, dr.p, di.p, nvec, p.ts, f64, f32, c->stream);
+    } else {
         if (c->thres != 0 && !(c->thres > 1))
             return nise_fail(c, NISE_ERR_UNSUPPORTED, "Sparse with Threshold > 0 (truncated U) is not supported");
-        e = launch_step_taylor(prec, N, dH.p, dr.p, di.p, nvec, nise_f64(p, sign, 1), c->stream);
+        e = launch_step_taylor_cta(prec, N, dH.p, dr.p, di.p, nvec, nise_f64(p, sign, 1), c->stream);
+        if (e == (int)cudaErrorNotSupported)
+            e = launch_step_taylor(prec, N, dH.p, dr.p, di.p, nvec, nise_f64(p, sign, 1), c->stream);
     }
     if ((rc = nise_cuda(c, e, "propagate"))) return rc;
     cudaMemcpyAsync(re, dr.p, rsz * nvec * N, cudaMemcpyDeviceToHost, c->stream);

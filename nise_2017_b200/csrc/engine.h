@@ -178,6 +178,14 @@ int launch_step_coupling(int prec, int n, float cut, const float *H, void *re, v
 int launch_step_rk4(int prec, int n, float cut, const float *H, void *re, void *im, int nvec, int ts,
                     double fsub, float fsub32, cudaStream_t s);
 int launch_step_taylor(int prec, int n, const float *H, void *re, void *im, int nvec, double f, cudaStream_t s);
+// The same with a CTA per vector; cudaErrorNotSupported where a vector's tables
+// exceed shared memory (Trotter, above about 220 sites) or its rows a CTA (RK4
+// and the exact step, above 1024).
+int launch_step_coupling_cta(int prec, int n, float cut, const float *H, void *re, void *im, int nvec, int ts,
+                             double fsub, float fsub32, cudaStream_t s);
+int launch_step_rk4_row(int prec, int n, float cut, const float *H, void *re, void *im, int nvec, int ts, double fsub,
+                        float fsub32, cudaStream_t s);
+int launch_step_taylor_cta(int prec, int n, const float *H, void *re, void *im, int nvec, double f, cudaStream_t s);
 
 // Eigen route (diag.cu).  U[t][a][c] = sum_k V[t][a][k] V[t][c][k] exp(-i w[t][k] f)
 // for nfr frames, rounded to the working precision (prec 0 FP32, 1 FP64) and,
