@@ -47,31 +47,39 @@ typedef std::tuple<int, int, int, int, int> TuneKey;  // scheme, precision, site
 std::map<TuneKey, int> g_tuned;
 std::mutex g_tune_mu;
 
+struct RowCounts {
+    int n[2];
+};
+
+// Rows of operations, where they are the fastest Trotter kernel: 35 (a warp
+// per vector, rows of 32), 36 (two warps, rows of 64) or 0.  rows.n[w]: rows of 32
+// (w = 0) and 64 per time step of `ops` operations, 0 where they do not fit.
+// Per-frame couplings up to 128 sites: 16-site chain, 1482 vectors, 0.67 ms
+// against 1.02 (warp per level) and 1.85 (thread per vector); 64-site chain 0.84
+// against 2.4 and 8.0; 64 sites all coupled 3.2 against 3.9.  Static couplings:
+// up to 100 sites (64-site lattice, 2982 vectors, 3.1 against 3.9 ms for two
+// vectors per warp), and up to 400 with few vectors (372 sites, 285 vectors, 3.0
+// against 4.0 ms; with 1476 vectors 12.6 against 8.0; 547 sites, 585 vectors,
+// 5.8 against 5.6: full rows meet more bank conflicts than the levels' chunks,
+// which are ordered against them).  Rows of 64 where they are fewer by a quarter
+// (372 sites: 3.0 against 3.6; 64 sites: 1.18 against 0.78).  Above about 860
+// operations per row and vector the SMs' warps are all busy and a thread per
+// vector is faster (16-site chain, 7422 vectors: 1.9 against 2.2 ms).
+int default_rows(int N, bool rot_static, int nvec, RowCounts rows, long ops) {
+    const bool few = nvec < 8 * sm_count();
+    if (!rows.n[0] || !(rot_static ? N <= 100 || (few && N <= 400) : N <= 128) || (double)nvec * rows.n[0] >= 860.0 * ops)
+        return 0;
+    return rows.n[1] && rot_static && 4 * rows.n[1] < 3 * rows.n[0] ? 36 : 35;
+}
+
 // Trotter: the warp-per-vector kernel where the levels are wide (lattices:
 // ~20 rotations per level) or the job has too few vectors to fill warps of
 // threads (a warp per vector then has the shorter critical path); thread per
 // vector for chains (one rotation per level) with many vectors.
-// rows[w]: rows of 32 (w = 0) and 64 operations per time step of `ops`, 0 where
-// they do not fit.
 int default_config(int scheme, int N, bool plain, bool cheb, int K, int nchk, int nvec, bool has4, bool rv,
-                   bool rot_static, const int rows[2], long ops) {
+                   bool rot_static, RowCounts rows, long ops) {
     if (scheme == SCHEME_TROTTER) {
-        // rows of operations, a warp per vector.  Per-frame couplings up to 128
-        // sites: 16-site chain, 1482 vectors, 0.67 ms against 1.02 (warp per
-        // level) and 1.85 (thread per vector); 64-site chain 0.84 against 2.4 and
-        // 8.0; 64 sites all coupled 3.2 against 3.9.  Static couplings: up to 100
-        // sites (64-site lattice, 2982 vectors, 3.1 against 3.9 ms for two
-        // vectors per warp), and up to 400 with few vectors (372 sites, 285
-        // vectors, 3.0 against 4.0 ms; with 1476 vectors 12.6 against 8.0; 547
-        // sites, 585 vectors, 5.8 against 5.6: full rows meet more bank
-        // conflicts than the levels' chunks, which are ordered against them).  Rows of 64 where they are fewer by a
-        // quarter (372 sites: 3.0 against 3.6; 64 sites: 0.95 against 0.78).
-        // Above about 860 operations per row and vector the SMs' warps are all
-        // busy and a thread per vector is faster (16-site chain, 7422 vectors:
-        // 1.9 against 2.2 ms).
-        const bool few = nvec < 8 * sm_count();
-        if (rows[0] && (rot_static ? N <= 100 || (few && N <= 400) : N <= 128) && (double)nvec * rows[0] < 860.0 * ops)
-            return rows[1] && rot_static && 4 * rows[1] < 3 * rows[0] ? 36 : 35;
+        if (const int r = default_rows(N, rot_static, nvec, rows, ops)) return r;
         // a warp per two vectors once there are 8 or more vectors per SM (static
         // couplings; 1024-site lattice, 1185 vectors: 39.3 against 43.9 ms),
         // else a warp per vector (C4's 585-vector jobs: 18.6 against 25.5 ms at
@@ -85,11 +93,14 @@ int default_config(int scheme, int N, bool plain, bool cheb, int K, int nchk, in
     if (plain) return 8;
     (void)cheb;           // the Chebyshev kernel is a tuned alternative: fewer terms, more work per term
     // less than one wave of 8-vector CTAs: 4 vectors per CTA reach twice the
-    // SMs.  C4 jobs (585 vectors): the FP32 sliced-ELL kernel with 4 vectors
-    // up to 1024 sites (295 sites 1.96 against 2.31 ms for k_abs_taylor2 and
-    // 2.32 for the default), k_abs_taylor2 with 4 above (1440 sites 12.1
-    // against 15.8 and 25.0 ms)
-    if (nvec < 8 * sm_count()) return has4 && N <= 1024 ? 12 : 3;
+    // SMs.  Up to 1024 sites the FP32 sliced-ELL kernel with 4 vectors (285
+    // vectors, 229 sites: 1.23 ms against 1.59 for k_abs_taylor2 and 1.36 for
+    // the row-owner kernel), but from 300 sites on the row-owner kernel with
+    // the Chebyshev expansion, whose gathers are conflict-free, makes up for the
+    // idle SMs (285 vectors, 600 sites: 2.79 against 4.13 ms; 1024 sites, 585
+    // vectors: 4.67 against 6.56); above 1024 sites k_abs_taylor2 with 4 (1440
+    // sites, 585 vectors: 12.1 against 15.8 and 25.0)
+    if (nvec < 8 * sm_count() && !(rv && cheb && N >= 300)) return has4 && N <= 1024 ? 12 : 3;
     // whole waves of 8-vector CTAs: the row-owner kernel with the Chebyshev
     // expansion (FP32 lattices up to 1024 sites; on the 1024-site lattice,
     // 100 000 frames: 52.0 ms against 55.8 with the Taylor series and 69.7 on
@@ -288,6 +299,12 @@ struct AbsRun {
     DevBuf<uint32_t> row_ab[2];  // rows of 32 and of 64 operations
     DevBuf<uint16_t> row_id[2];
     RowPlan row[2] = {};
+    RowCounts rows_of(const TrotterPlan &P) const {
+        RowCounts r = {{0, 0}};
+        for (int w = 0; w < 2; w++)
+            if (trotter_rows_fit(prec == NISE_FP32 ? 0 : 1, P, row[w], 32 * (w + 1))) r.n[w] = row[w].nrow;
+        return r;
+    }
     TrotterPlan TP;
     // RK4
     DevBuf<int2> dent;
@@ -434,12 +451,47 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
         std::vector<int> hchk;
         rotation_chunks(hlv, hchk);
         nchk = (int)hchk.size() - 1;
-        std::vector<char> hflip;
-        bank_order(pairs, N, hchk, hperm, hflip);
         std::vector<int2> lpairs(pairs.size());
-        for (size_t q = 0; q < pairs.size(); q++) {
-            const int2 ab = pairs[hperm[q]];
-            lpairs[q] = hflip[q] ? make_int2(ab.y, ab.x) : ab;
+        auto in_order = [&](const std::vector<char> &flip) {
+            for (size_t q = 0; q < pairs.size(); q++) {
+                const int2 ab = pairs[hperm[q]];
+                lpairs[q] = !flip.empty() && flip[q] ? make_int2(ab.y, ab.x) : ab;
+            }
+        };
+        // The whole step as rows, from the level order (every site's order is
+        // the same), for the sizes default_config takes them at, or on demand.
+        const bool asked = p.kernel_config == 35 || p.kernel_config == 36;
+        const bool rows_ok = p.kernel_config == 0 && N <= (TP.rot_static ? 400 : 128);
+        auto build_rows = [&]() -> int {
+            for (int w = 0; w < 2; w++) {
+                if (w == 1 && !TP.rot_static && p.kernel_config != 36) break;  // never the default
+                std::vector<uint32_t> ab;
+                std::vector<uint16_t> id;
+                row[w].nrow = nise_row_schedule(lpairs, N, p.ts, 32 * (w + 1), ab, id);
+                int r;
+                if ((r = row_ab[w].upload(c, ab)) || (r = row_id[w].upload(c, id))) return r;
+                row[w].ab = row_ab[w].p;
+                row[w].id = row_id[w].p;
+            }
+            return NISE_OK;
+        };
+        const bool rows = (asked || rows_ok) && N + 64 <= NISE_ROW_MAX && TP.k <= NISE_ROW_MAX && p.ts >= 1;
+        in_order({});
+        if (rows && (rc = build_rows())) return rc;
+        // the warp kernels' bank order costs the host more than the levels, so
+        // not where the rows are taken anyway
+        const int cfg = rows ? default_rows(N, TP.rot_static, plain ? 3 : nvec, rows_of(TP), (long)p.ts * (TP.k + 2L * N)) : 0;
+        if (!asked && (!cfg || autotune)) {
+            std::vector<char> hflip;
+            bank_order(pairs, N, hchk, hperm, hflip);
+            in_order(hflip);
+            if (rows) {
+                for (int w = 0; w < 2; w++) {
+                    row_ab[w].free();
+                    row_id[w].free();
+                }
+                if ((rc = build_rows())) return rc;
+            }
         }
         if ((rc = dpairs.upload(c, lpairs.empty() ? std::vector<int2>(1) : lpairs)) ||
             (rc = U.alloc(c, r2 * (size_t)nf * N)) ||
@@ -450,19 +502,6 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
         TP.pairs = dpairs.p;
         TP.U = U.p;
         TP.rot = rot.p;
-        // the whole step as rows, from the level order (every site's order is
-        // the same), for the sizes default_config takes them at, or on demand
-        const bool asked = p.kernel_config == 35 || p.kernel_config == 36;
-        const bool rows_ok = p.kernel_config == 0 && N <= (TP.rot_static ? 400 : 128);
-        if ((asked || rows_ok) && N + 64 <= NISE_ROW_MAX && TP.k <= NISE_ROW_MAX && p.ts >= 1)
-            for (int w = 0; w < 2; w++) {
-                std::vector<uint32_t> ab;
-                std::vector<uint16_t> id;
-                row[w].nrow = nise_row_schedule(lpairs, N, p.ts, 32 * (w + 1), ab, id);
-                if ((rc = row_ab[w].upload(c, ab)) || (rc = row_id[w].upload(c, id))) return rc;
-                row[w].ab = row_ab[w].p;
-                row[w].id = row_id[w].p;
-            }
     } else if (p.propagation == NISE_PROP_RK4) {
         scheme = SCHEME_RK4;
         std::vector<int2> pairs, ent;
@@ -864,13 +903,10 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
                 return rc;
         }
     }
-    int nrows[2] = {0, 0};
-    if (scheme == SCHEME_TROTTER)
-        for (int w = 0; w < 2; w++)
-            if (trotter_rows_fit(prec == NISE_FP32 ? 0 : 1, TP, row[w], 32 * (w + 1))) nrows[w] = row[w].nrow;
     config = default_config(scheme, N, plain, cheb, TP.k, nchk, plain ? 3 : nvec, dell4.p != nullptr,
                             scheme == SCHEME_TAYLOR && taylor_rv_fits(T, XP),
-                            scheme == SCHEME_TROTTER && TP.rot_static, nrows, (long)p.ts * (TP.k + 2L * N));
+                            scheme == SCHEME_TROTTER && TP.rot_static,
+                            scheme == SCHEME_TROTTER ? rows_of(TP) : RowCounts{{0, 0}}, (long)p.ts * (TP.k + 2L * N));
     if (p.kernel_config != 0) {  // forced by the caller
         const int k = p.kernel_config;
         if (scheme == SCHEME_EIGEN && (k == 2 || k == 16 || k == 17)) return NISE_OK;

@@ -97,9 +97,11 @@ template <typename T> struct DevBuf {
         if (!h.empty()) cudaMemcpyAsync(p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice, s);
         return NISE_OK;
     }
-    ~DevBuf() {
+    void free() {
         if (p) cudaFreeAsync(p, s);
+        p = nullptr;
     }
+    ~DevBuf() { free(); }
 };
 
 // Device buffers behind a SinglesTab (and the eigen route's doubles sub-step
