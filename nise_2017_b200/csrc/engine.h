@@ -76,18 +76,17 @@ struct TaylorPlan {
     const void *ell4;
     const int *ell4_sptr, *ell4_rows;
     int ell4_nslices, ell4_nent;
-    // row-owner layout (k_abs_taylor_rv, FP32): 8-row slices of alternating
-    // parity, couplings in slot triples [group][row]: float4 of the three
-    // weights and the bits of the three neighbours' row indices (10 bits
-    // each); tptr [nslices + 1] first group of each slice, rows [nslices][8];
-    // wsl[s] the slices of each warp of launch shape s (24 or 32 warps,
-    // [warp][8], -1 = none), it[s] the most slices of a warp; no_rv keeps the
-    // 8-vector waves on k_abs_taylor3
-    const float4 *ell8_tri;
-    const int *ell8_tptr, *ell8_rows;
-    const int *ell8_wsl[2];
+    // row-owner layout (k_abs_taylor_rv, FP32), for each launch shape s (24 or
+    // 32 warps): 8-row slices of alternating parity dealt to the warps, couplings
+    // in slot triples [group][row], a warp's groups one after another: float4 of
+    // the three weights and the bits of the three neighbours' row indices (10
+    // bits each); rows [warp][8 slices][8]: the site (n: none), the slice's groups
+    // and, in a warp's first slice, its first group; it[s] the most slices of a
+    // warp; no_rv keeps the 8-vector waves on k_abs_taylor3
+    const float4 *ell8_tri[2];
+    const uint32_t *ell8_rows[2];
     int ell8_it[2];
-    int ell8_nslices, ell8_ntg;
+    int ell8_ntg;
     int rv_shape;
     int no_rv;
     int rv_cheb;           // with the Chebyshev tables: the row-owner kernel's Chebyshev form
@@ -95,6 +94,11 @@ struct TaylorPlan {
     int *err;              // device flag: 1 = a bounded wait for a staged frame gave up
 };
 #define NISE_CHEB_KMAX 40
+// A row word of the row-owner layout.
+#define NISE_RV_WORD(row, len, first) ((uint32_t)(row) | (uint32_t)(len) << 11 | (uint32_t)(first) << 20)
+#define NISE_RV_ROW(w) ((w) & 0x7ffu)
+#define NISE_RV_LEN(w) (((w) >> 11) & 0x1ffu)
+#define NISE_RV_FIRST(w) ((w) >> 20)
 
 // A batch of linear-absorption start points: vectors v = 3*(s-begin)+x for
 // samples s in [begin, begin+nsamp), polarisations x = 0..2.

@@ -19,7 +19,12 @@
 //    three weights and the three neighbours' 10-bit row indices, so one
 //    load (8 rows: one shared-memory wavefront) serves three slots;
 //  - the slices are dealt to the warps longest first (each warp's total
-//    slot count nearly equal: the CTA barrier waits for the slowest warp);
+//    slot count nearly equal: the CTA barrier waits for the slowest warp), and a
+//    warp's triples lie one after another in its order, so the triple loaded
+//    ahead at a slice's end is the next slice's first; one word per (warp,
+//    slice, row) holds the row and the slice's triples, where separate tables
+//    cost four more loads per slice and a longer chain to the first gather
+//    (1024-site lattice, 100 000 frames: 48.5 -> 45.7 ms);
 //  - the diagonal records of the frames the CTA's vectors need next are
 //    staged into shared memory with bulk copies (cp.async.bulk, completion on
 //    an mbarrier) one step ahead; the dipoles are static (read_coupling,
@@ -40,27 +45,23 @@ constexpr int kRvMaxIT = 8;       // slices per warp
 constexpr unsigned kRvSpin = 1u << 20;  // bound on the mbarrier waits
 
 struct RvLayout {
-    size_t cur, tri, tptr, rows, wsl, dg, red, mbar, total;
+    size_t cur, tri, rows, dg, red, mbar, total;
     int dgw;  // words per staged diagonal record (16-byte multiple)
 };
 
 __host__ __device__ inline size_t rv_al(size_t x) { return (x + 15) & ~(size_t)15; }
 
-// Shared-memory layout for n sites, ntg slot-triple groups (8 rows each), nsl
-// slices and nw warps.
-__host__ __device__ inline RvLayout rv_layout(int n, int ntg, int nsl, int nw) {
+// Shared-memory layout for n sites, ntg slot-triple groups (8 rows each) and
+// nw warps.
+__host__ __device__ inline RvLayout rv_layout(int n, int ntg, int nw) {
     RvLayout L;
     size_t o = 0;
     L.cur = o;
     o = rv_al(o + (size_t)2 * n * 64);
     L.tri = o;
     o = rv_al(o + (size_t)(ntg + 1) * 8 * 16);  // + one group of slack for the prefetch
-    L.tptr = o;
-    o = rv_al(o + (size_t)(nsl + 1) * 4);
     L.rows = o;
-    o = rv_al(o + (size_t)nsl * 8 * 4);
-    L.wsl = o;
-    o = rv_al(o + (size_t)nw * kRvMaxIT * 4);
+    o = rv_al(o + (size_t)nw * kRvMaxIT * 8 * 4);
     L.dgw = (n + 6) & ~3;  // a record shifted by up to 3 words, rounded up to 4 words
     L.dg = o;
     o = rv_al(o + (size_t)kRvSlots * L.dgw * 4);
@@ -147,27 +148,24 @@ __device__ __forceinline__ void rv_stage(const DevTraj &T, const AbsJob &J, int 
 // Each vector uses its own frame's c, R and coefficients.
 template <int IT, int NT, bool CHEB>
 __global__ void __launch_bounds__(NT, 1)
-    k_abs_taylor_rv(DevTraj T, TaylorPlan P, AbsJob J, double2 *resp, int v0, int nvec, const int *__restrict__ wsl_g) {
+    k_abs_taylor_rv(DevTraj T, TaylorPlan P, AbsJob J, double2 *resp, int v0, int nvec, const float4 *__restrict__ tri_g,
+                    const uint32_t *__restrict__ rows_g) {
     constexpr int NW = NT / 32;
     extern __shared__ __align__(16) unsigned char sm[];
-    const int n = P.n, nsl = P.ell8_nslices, ntg = P.ell8_ntg;
-    const RvLayout L = rv_layout(n, ntg, nsl, NW);
+    const int n = P.n, ntg = P.ell8_ntg;
+    const RvLayout L = rv_layout(n, ntg, NW);
     float4 *cur = (float4 *)(sm + L.cur);  // [2][n][4]
     float4 *tri = (float4 *)(sm + L.tri);
-    int *tptr = (int *)(sm + L.tptr);
-    int *rows = (int *)(sm + L.rows);
-    int *wsl = (int *)(sm + L.wsl);
+    uint32_t *rows = (uint32_t *)(sm + L.rows);  // [warp][slice][8]
     float *dg = (float *)(sm + L.dg);
     double *red = (double *)(sm + L.red);
     uint64_t *mbar = (uint64_t *)(sm + L.mbar);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int r = lane >> 2, c = lane & 3;
 
-    for (int e = tid; e < 8 * ntg; e += NT) tri[e] = P.ell8_tri[e];
+    for (int e = tid; e < 8 * ntg; e += NT) tri[e] = tri_g[e];
     for (int e = tid; e < 8; e += NT) tri[8 * ntg + e] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int e = tid; e <= nsl; e += NT) tptr[e] = P.ell8_tptr[e];
-    for (int e = tid; e < 8 * nsl; e += NT) rows[e] = P.ell8_rows[e];
-    for (int e = tid; e < NW * kRvMaxIT; e += NT) wsl[e] = wsl_g[e];
+    for (int e = tid; e < NW * kRvMaxIT * 8; e += NT) rows[e] = rows_g[e];
     if (tid == 0) {
         mbar_init(&mbar[0], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -194,10 +192,8 @@ __global__ void __launch_bounds__(NT, 1)
     float d0[IT], d1[IT];
     __syncthreads();
     // site of this lane's row in its it-th slice (n: none)
-    auto site = [&](int it) {
-        const int sl = wsl[warp * kRvMaxIT + it];
-        return sl >= 0 ? rows[8 * sl + r] : n;
-    };
+    const uint32_t *wrow = rows + warp * kRvMaxIT * 8 + r;
+    auto site = [&](int it) { return (int)NISE_RV_ROW(wrow[8 * it]); };
 #pragma unroll
     for (int it = 0; it < IT; it++) {
         const int i = site(it);
@@ -313,21 +309,20 @@ __global__ void __launch_bounds__(NT, 1)
             const float4 *src = cur + (size_t)((k - 1) & 1) * n * 4;
             float4 *dst = cur + (size_t)(k & 1) * n * 4;
             const char *srcc = (const char *)(src + c);
+            const float4 *tp = tri + 8 * NISE_RV_FIRST(wrow[0]) + r;
+            float4 w = *tp;
 #pragma unroll
             for (int it = 0; it < IT; it++) {
-                const int sl = wsl[warp * kRvMaxIT + it];
-                if (sl < 0) continue;
-                const int i = rows[8 * sl + r];
+                const uint32_t wd = wrow[8 * it];
+                const int i = NISE_RV_ROW(wd);
                 const float4 own = i < n ? src[(size_t)i * 4 + c] : make_float4(0.f, 0.f, 0.f, 0.f);
                 float a0 = d0[it] * own.x, b0 = d0[it] * own.y;
                 float a1 = d1[it] * own.z, b1 = d1[it] * own.w;
                 // slot triples; the next triple is loaded one iteration ahead
-                // (past the slice it is unused; one group of slack)
-                const int p1 = tptr[sl + 1];
-                int p = tptr[sl];
-                float4 w = tri[8 * p + r];
-                for (; p < p1; p++) {
-                    const float4 nw = tri[8 * (p + 1) + r];
+                // (past the warp's last it is unused; one group of slack)
+                for (int q = NISE_RV_LEN(wd); q > 0; q--) {
+                    tp += 8;
+                    const float4 nw = *tp;
                     const uint32_t ix = __float_as_uint(w.w);
                     const float4 za = *(const float4 *)(srcc + ((ix & 0x3ffu) << 6));
                     const float4 zb = *(const float4 *)(srcc + (((ix >> 10) & 0x3ffu) << 6));
@@ -380,21 +375,21 @@ __global__ void __launch_bounds__(NT, 1)
 }
 
 template <int IT, int NT, bool CHEB>
-int run_rv1(const DevTraj &T, const TaylorPlan &P, const AbsJob &J, double2 *resp, int v0, int nvec, const int *wsl,
-            cudaStream_t s) {
-    const size_t smem = rv_layout(P.n, P.ell8_ntg, P.ell8_nslices, NT / 32).total;
+int run_rv1(const DevTraj &T, const TaylorPlan &P, const AbsJob &J, double2 *resp, int v0, int nvec, cudaStream_t s) {
+    const size_t smem = rv_layout(P.n, P.ell8_ntg, NT / 32).total;
+    const int sh = P.rv_shape;
     cudaError_t e =
         cudaFuncSetAttribute(k_abs_taylor_rv<IT, NT, CHEB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    k_abs_taylor_rv<IT, NT, CHEB><<<(nvec + kRvG - 1) / kRvG, NT, smem, s>>>(T, P, J, resp, v0, nvec, wsl);
+    k_abs_taylor_rv<IT, NT, CHEB><<<(nvec + kRvG - 1) / kRvG, NT, smem, s>>>(T, P, J, resp, v0, nvec,
+                                                                               P.ell8_tri[sh], P.ell8_rows[sh]);
     return (int)cudaGetLastError();
 }
 
 template <int IT, int NT>
-int run_rv(const DevTraj &T, const TaylorPlan &P, const AbsJob &J, double2 *resp, int v0, int nvec, const int *wsl,
-           cudaStream_t s) {
-    if (P.cheb_coef) return run_rv1<IT, NT, true>(T, P, J, resp, v0, nvec, wsl, s);
-    return run_rv1<IT, NT, false>(T, P, J, resp, v0, nvec, wsl, s);
+int run_rv(const DevTraj &T, const TaylorPlan &P, const AbsJob &J, double2 *resp, int v0, int nvec, cudaStream_t s) {
+    if (P.cheb_coef) return run_rv1<IT, NT, true>(T, P, J, resp, v0, nvec, s);
+    return run_rv1<IT, NT, false>(T, P, J, resp, v0, nvec, s);
 }
 
 }  // namespace
@@ -404,10 +399,10 @@ int run_rv(const DevTraj &T, const TaylorPlan &P, const AbsJob &J, double2 *resp
 const int kRvWarps[2] = {24, 32};
 
 bool taylor_rv_fits(const DevTraj &T, const TaylorPlan &P) {
-    if (!P.ell8_tri || !P.err || !T.mu_static || T.full || !P.static_j || P.n > 1024) return false;
+    if (!P.err || !T.mu_static || T.full || !P.static_j || P.n > 1024) return false;
     const int sh = P.rv_shape;
-    if (sh < 0 || sh > 1 || !P.ell8_wsl[sh] || P.ell8_it[sh] > kRvMaxIT) return false;
-    return rv_layout(P.n, P.ell8_ntg, P.ell8_nslices, kRvWarps[sh]).total <= 227 * 1024;
+    if (sh < 0 || sh > 1 || !P.ell8_tri[sh] || P.ell8_it[sh] > kRvMaxIT) return false;
+    return rv_layout(P.n, P.ell8_ntg, kRvWarps[sh]).total <= 227 * 1024;
 }
 
 int launch_abs_taylor_rv(const DevTraj &T, const TaylorPlan &P, const AbsJob &J, double2 *resp, int v0, int nvec,
@@ -415,13 +410,12 @@ int launch_abs_taylor_rv(const DevTraj &T, const TaylorPlan &P, const AbsJob &J,
     if (nvec <= 0) return 0;
     if (!taylor_rv_fits(T, P)) return (int)cudaErrorNotSupported;
     const int sh = P.rv_shape, it = P.ell8_it[sh];
-    const int *wsl = P.ell8_wsl[sh];
     if (sh == 0) {
-        if (it <= 4) return run_rv<4, 768>(T, P, J, resp, v0, nvec, wsl, s);
-        if (it <= 6) return run_rv<6, 768>(T, P, J, resp, v0, nvec, wsl, s);
-        return run_rv<8, 768>(T, P, J, resp, v0, nvec, wsl, s);
+        if (it <= 4) return run_rv<4, 768>(T, P, J, resp, v0, nvec, s);
+        if (it <= 6) return run_rv<6, 768>(T, P, J, resp, v0, nvec, s);
+        return run_rv<8, 768>(T, P, J, resp, v0, nvec, s);
     }
-    if (it <= 4) return run_rv<4, 1024>(T, P, J, resp, v0, nvec, wsl, s);
-    if (it <= 6) return run_rv<6, 1024>(T, P, J, resp, v0, nvec, wsl, s);
-    return run_rv<8, 1024>(T, P, J, resp, v0, nvec, wsl, s);
+    if (it <= 4) return run_rv<4, 1024>(T, P, J, resp, v0, nvec, s);
+    if (it <= 6) return run_rv<6, 1024>(T, P, J, resp, v0, nvec, s);
+    return run_rv<8, 1024>(T, P, J, resp, v0, nvec, s);
 }
