@@ -1442,13 +1442,28 @@ __device__ void rk4_doubles_step(const TwoD &D, long t, typename Vec2<R>::T *F, 
 // the response's cancellation amplifies another order by 10^3), FP64 multiplies
 // matrices (k2d_doubles_sparse64).
 
+// The molecular polarisations a vector takes part in, at most three of the 21
+// (-1: none); list [nv][3], all threads of the CTA, no synchronisation.  Once per
+// CTA: every warp looking through 21 x nv pairs at every t3 was a fifth of
+// k2d_doubles_sparse32 at 12 sites (10.9 -> 8.7 ms without).
+__device__ __forceinline__ void dbl_list(const TwoD &D, int u0, int nv, short *list) {
+    for (int q = threadIdx.x; q < nv; q += blockDim.x) {
+        const DblVec w = dbl_vec(u0 + q, D.T1);
+        int k = 0;
+        for (int m = 0; m < 21; m++)
+            if (c_px[m][2] == w.p2 && c_px[m][w.kind == 0 ? 1 : 0] == w.pa) list[3 * q + k++] = (short)m;
+        while (k < 3) list[3 * q + k++] = -1;
+    }
+}
+
 // EA projections and dot products of the CTA's vectors u0 .. u0 + nv - 1 at t3
 // (calc_2DIR.c:456-488): dipole_double_last into G[q][p3][n] (float sums in
 // site order), then a warp per dot product.  at(q, j, a) is element (j, a) of
-// vector q; mu and ov [3][n] hold the frame's dipoles.
+// vector q; mu and ov [3][n] hold the frame's dipoles; list the molecular
+// polarisations of each vector (dbl_list).
 template <typename R, typename At>
 __device__ __forceinline__ void dbl_ea(const TwoD &D, int s, int t3, int u0, int nv, typename Vec2<R>::T *G,
-                                       const R *mu, const R *ov, At at) {
+                                       const R *mu, const R *ov, const short *list, At at) {
     typedef typename Vec2<R>::T R2;
     typedef Ar<R> A;
     const int n = D.n, NV = nvec_se(D), lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -1465,11 +1480,11 @@ __device__ __forceinline__ void dbl_ea(const TwoD &D, int s, int t3, int u0, int
         G[e].y = gi;
     }
     __syncthreads();
-    for (int qm = 0, item = 0; qm < 21 * nv; qm++) {
-        const int q = qm / 21, m = qm % 21;
+    for (int qm = 0, item = 0; qm < 3 * nv; qm++) {
+        const int q = qm / 3, m = list[qm];
+        if (m < 0) continue;
         const DblVec w = dbl_vec(u0 + q, D.T1);
         const int p0 = c_px[m][0], p1 = c_px[m][1], p3 = c_px[m][3];
-        if (c_px[m][2] != w.p2 || (w.kind == 0 ? p1 : p0) != w.pa) continue;
         const int reps = w.kind == 0 ? D.T1 : 1;
         // the products of all matching (q, m) are dealt to the warps in turn
         for (int r = (warp - item % nw + nw) % nw; r < reps; r += nw) {
@@ -1531,9 +1546,10 @@ __device__ __forceinline__ typename Vec2<R>::T dbl_half(typename Vec2<R>::T ph, 
 // vector: a thread carries 8 vectors of one start point, kept in pairs for the
 // two-wide instructions, and the lanes of a warp read the same F{t,v} (four
 // broadcast 16-byte loads per term).  g is sqrt2 for t = v where p != q (peeled
-// off the loop) and for t != v where p = q (those outputs come last, so that a
-// warp seldom holds both kinds).  Small N: NG groups of 8 vectors per CTA, so
-// that the outputs fill 8 warps.  TRUNC: the Threshold truncates, so zero
+// off the loop) and for t != v where p = q (those outputs have warps of their
+// own: a warp with both kinds runs both in sequence and the others wait for it;
+// 12 sites, 912 CTAs: 11.1 -> 10.9 ms).  Small N: NG groups of 8 vectors per CTA,
+// so that the outputs fill 4 warps.  TRUNC: the Threshold truncates, so zero
 // elements are skipped; else the list is full.
 constexpr int kSpVG = 8;
 
@@ -1590,6 +1606,9 @@ __global__ void __launch_bounds__(256, 3) k2d_doubles_sparse32(TwoD D, int vec_p
     float2 *ph = G + 3 * VC * n;                                     // [n]
     float *mu = (float *)(ph + n), *ov = mu + 3 * n;                 // [3][n] each
     short2 *pq = (short2 *)(ov + 3 * n);                             // [N2] the outputs: p < q, then p = q
+    short *list = (short *)(pq + N2);                                // [VC][3]
+    dbl_list(D, u0, nv, list);
+    const int offp = (NG * noff + 31) & ~31;  // the outputs p = q start on a warp of their own
     const f32x2 one = both(onef);
     // element {j, a} of vector q
     auto at = [&](int q, int j, int a) {
@@ -1618,7 +1637,7 @@ __global__ void __launch_bounds__(256, 3) k2d_doubles_sparse32(TwoD D, int vec_p
             U = Ush;
         }
         __syncthreads();
-        if (D.ea) dbl_ea<float>(D, s, t3, u0, nv, G, mu, ov, [&](int q, int j, int a) {
+        if (D.ea) dbl_ea<float>(D, s, t3, u0, nv, G, mu, ov, list, [&](int q, int j, int a) {
             const size_t o = at(q, j, a);
             return make_float2(Fr[o], Fi[o]);
         });
@@ -1634,9 +1653,10 @@ __global__ void __launch_bounds__(256, 3) k2d_doubles_sparse32(TwoD D, int vec_p
         for (int sub = 0; sub < D.ts; sub++) {
             for (int e = tid; e < VC * n; e += blockDim.x) half(e);
             __syncthreads();
-            for (int e = tid; e < NG * N2; e += blockDim.x) {
-                const bool off = e < NG * noff;
-                const int eo = off ? e : e - NG * noff, per = off ? noff : n, grp = eo / per;
+            for (int e = tid; e < offp + NG * n; e += blockDim.x) {
+                const bool off = e < offp;
+                if (off && e >= NG * noff) continue;
+                const int eo = off ? e : e - offp, per = off ? noff : n, grp = eo / per;
                 const short2 o2 = pq[(off ? 0 : noff) + eo % per];
                 const int p = o2.x, q = o2.y;
                 const float *fr = Fr + grp * gp, *fi = Fi + grp * gp;
@@ -1730,6 +1750,8 @@ __global__ void __launch_bounds__(256) k2d_doubles_sparse64(TwoD D, int vec_per_
     double2 *G = dF + VC * n;                                      // [VC][3][n]
     double2 *ph = G + 3 * VC * n;                                  // [n]
     double *mu = (double *)(ph + n), *ov = mu + 3 * n;             // [3][n] each
+    short *list = (short *)(ov + 3 * n);                           // [VC][3]
+    dbl_list(D, u0, nv, list);
     const double g = (double)1.41421356237f, corr = 1.0 - 0.5 * g * g;
     for (int e = tid; e < nv * N2; e += blockDim.x) {
         const int q = e / N2;
@@ -1750,7 +1772,7 @@ __global__ void __launch_bounds__(256) k2d_doubles_sparse64(TwoD D, int vec_per_
             U = Ush;
         }
         __syncthreads();
-        if (D.ea) dbl_ea<double>(D, s, t3, u0, nv, G, mu, ov, [&](int q, int j, int a) { return F[q * mat + (size_t)j * n + a]; });
+        if (D.ea) dbl_ea<double>(D, s, t3, u0, nv, G, mu, ov, list, [&](int q, int j, int a) { return F[q * mat + (size_t)j * n + a]; });
         if (t3 == D.T3 - 1) break;
         __syncthreads();
         for (int e = tid; e < nv * n; e += blockDim.x) {
@@ -2046,9 +2068,11 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf, const RowPlan &Q) {
         void *ws = nullptr;
         if (sizeof(R) == 4) {
             const int NG = std::max(1, std::min(128 / N2, (vps + kSpVG - 1) / kSpVG)), VC = NG * kSpVG;
-            const size_t small = sizeof(float2) * (3 * (size_t)VC + 1) * n + sizeof(float) * 6 * n + sizeof(short2) * N2;
+            const size_t small = sizeof(float2) * (3 * (size_t)VC + 1) * n + sizeof(float) * 6 * n + sizeof(short2) * N2 +
+                                 sizeof(short) * 3 * VC;
             const size_t all = sizeof(float) * 4 * VC * N2 + sizeof(float2) * n * n + small;
-            const int ctas = D.S * ((vps + VC - 1) / VC), threads = std::min(256, (NG * N2 + 31) / 32 * 32);
+            const int ctas = D.S * ((vps + VC - 1) / VC), offp = (NG * n * (n - 1) / 2 + 31) & ~31,
+                      threads = std::min(256, (offp + NG * n + 31) / 32 * 32);
             const bool sm = all <= 227 * 1024;  // up to 53 sites
             auto kern = sm ? (D.trunc ? k2d_doubles_sparse32<true, true> : k2d_doubles_sparse32<true, false>)
                            : (D.trunc ? k2d_doubles_sparse32<false, true> : k2d_doubles_sparse32<false, false>);
@@ -2059,7 +2083,7 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf, const RowPlan &Q) {
             // vectors per CTA: enough 4-column tiles for 256 threads
             const int tiles = n * ((n + 3) / 4), VC = std::min(vps, std::max(1, (256 + tiles - 1) / tiles));
             const size_t mat = (size_t)n * n;
-            const size_t small = sizeof(double2) * (size_t)(4 * VC + 1) * n + sizeof(double) * 6 * n;
+            const size_t small = sizeof(double2) * (size_t)(4 * VC + 1) * n + sizeof(double) * 6 * n + sizeof(short) * 3 * VC;
             const size_t all = sizeof(double2) * mat * (1 + 2 * VC) + small;
             const int ctas = D.S * ((vps + VC - 1) / VC);
             if (all <= 227 * 1024) {  // up to 68 sites
