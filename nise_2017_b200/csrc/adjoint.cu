@@ -32,6 +32,11 @@
 
 namespace {
 
+// The kernels on one matrix per rotation keep sites, and the rotations of a frame,
+// the even ones before the odd ones: the sub-steps that overlap on a chain are two
+// sites apart, and neighbours in shared memory meet no bank conflict.
+__host__ __device__ __forceinline__ int adj_pos(int a, int n) { return (a >> 1) + (a & 1) * ((n + 1) >> 1); }
+
 // FP64 tables for frames [f0, f0+nf): U[t][a] = (cos(h f/2), -sin(h f/2)),
 // rot[t][k] = (co, si) with si = -sin(s J f), co = sqrt(1 - si^2), and
 // jf[t][k] = J f (the derivative of the angle with respect to s).
@@ -55,7 +60,17 @@ __global__ void k_adj_prep(DevTraj T, AdjPlan P) {
         double jf = (double)traj_coupling(T, P.f0 + t, ab.x, ab.y) * P.f;
         double si = -sin(P.scale * jf);
         P.rot[g] = make_double2(sqrt(1.0 - si * si), si);
-        P.jf[g] = jf;
+        if (P.mat) {
+            // jf q_a conj(q_b), q the half phases after the rotation
+            const uint32_t p = P.parts[k];
+            const double ha = NISE_SCHED_POST_A(p) ? (double)traj_diag_raw(T, P.f0 + t, ab.x) + P.shift[ab.x] : 0.0;
+            const double hb = NISE_SCHED_POST_B(p) ? (double)traj_diag_raw(T, P.f0 + t, ab.y) + P.shift[ab.y] : 0.0;
+            double s, c;
+            sincos(0.5 * (hb - ha) * P.f, &s, &c);
+            P.je[t * P.k + adj_pos(k, P.k)] = make_double2(jf * c, jf * s);
+        } else {
+            P.jf[g] = jf;
+        }
     }
 }
 
@@ -202,7 +217,8 @@ __global__ void k_adj_bwd(DevTraj T, AdjPlan P, AbsJob J, const double2 *G, cons
 // it), so what counts is the number of rows.
 // 256-site chain, 244 start points, RunTimes 128, with a thread per vector (23
 // warps in all, 1275 rotations in sequence per step): forward 32.4 ms, backward
-// 50.2 ms; now 3.6 and 5.6 ms (157 instructions per row, 4.3 cycles each).
+// 50.2 ms; now 3.6 and 5.6 ms (157 instructions per row, 4.3 cycles each;
+// less with one matrix per rotation, below, where those fit).
 struct AdjCoef {
     uint32_t e, p;
     double2 cs, ua, ub;
@@ -215,14 +231,12 @@ __device__ __forceinline__ double2 cmul_conj(double2 u, double2 z) {
     return make_double2(z.x * u.x + z.y * u.y, z.y * u.x - z.x * u.y);
 }
 
-__device__ __forceinline__ AdjCoef adj_coef(const AdjPlan &P, uint32_t e, const uint32_t *parts, const double2 *rot,
-                                            const double2 *U) {
+__device__ __forceinline__ AdjCoef adj_coef(const AdjPlan &P, uint2 r, const double2 *rot, const double2 *U) {
     AdjCoef c;
-    c.e = e;
-    c.p = 0;
-    const uint32_t q = NISE_SCHED_Q(e), w = NISE_SCHED_W(e);
+    c.e = r.y;
+    c.p = r.x;
+    const uint32_t q = NISE_SCHED_Q(c.e), w = NISE_SCHED_W(c.e);
     if (q != NISE_SCHED_NONE) {
-        c.p = parts[q];
         c.cs = rot[(size_t)w * P.k + q];
         c.ua = U[(size_t)w * P.n + NISE_SCHED_A(c.p)];
         c.ub = U[(size_t)w * P.n + NISE_SCHED_B(c.p)];
@@ -244,10 +258,6 @@ __global__ void __launch_bounds__(96) k_adj_fwd_warp(DevTraj T, AdjPlan P, AbsJo
     const int n = P.n, lane = threadIdx.x & 31, x = threadIdx.x >> 5, v = 3 * blockIdx.x + x;
     double2 *X = (double2 *)smem_raw + (size_t)x * P.W * n, *snap = X + n;  // [3][X, W - 1 snapshots][n]
     double2 *rsh = (double2 *)smem_raw + 3 * (size_t)P.W * n, *ush = rsh + (SM ? (size_t)P.W * P.k : 0);
-    uint32_t *psh = (uint32_t *)(ush + (SM ? (size_t)P.W * n : 0));
-    const uint32_t *parts = SM ? psh : P.parts;
-    if (SM)
-        for (int e = threadIdx.x; e < P.k; e += blockDim.x) psh[e] = P.parts[e];
     const long ti = (long)(J.begin + blockIdx.x) * J.sample;
     for (int a = lane; a < n; a += 32) X[a] = make_double2((double)traj_mu(T, ti, x, a), 0.0);
     double2 *ck = ckpt + (size_t)v * P.nck * n;
@@ -272,7 +282,7 @@ __global__ void __launch_bounds__(96) k_adj_fwd_warp(DevTraj T, AdjPlan P, AbsJo
             for (int a = lane; a < n; a += 32) ck[(size_t)(t1 / P.K) * n + a] = X[a];
         if (t1 == J.tmax - 1) break;
         const int steps = J.tmax - 1 - t1 >= P.W ? P.W : 1;
-        const uint32_t *rows = steps == P.W ? P.schedW : P.sched1;
+        const uint2 *rows = steps == P.W ? P.schedW : P.sched1;
         const int nrow = steps == P.W ? P.nrowW : P.nrow1;
         const long fi = ti + t1 - P.f0;
         const double2 *rot = P.rot + fi * P.k, *U = P.U + fi * n;
@@ -283,11 +293,12 @@ __global__ void __launch_bounds__(96) k_adj_fwd_warp(DevTraj T, AdjPlan P, AbsJo
             rot = rsh;
             U = ush;
         }
-        AdjCoef c = adj_coef(P, nrow > 0 ? rows[lane] : NISE_SCHED_NONE, parts, rot, U);
-        uint32_t e1 = nrow > 1 ? rows[32 + lane] : NISE_SCHED_NONE;
+        rows += lane;
+        AdjCoef c = adj_coef(P, rows[0], rot, U);
+        uint2 e1 = rows[32];
         for (int r = 0; r < nrow; r++) {
-            const AdjCoef nx = adj_coef(P, e1, parts, rot, U);
-            e1 = r + 2 < nrow ? rows[(size_t)(r + 2) * 32 + lane] : NISE_SCHED_NONE;
+            const AdjCoef nx = adj_coef(P, e1, rot, U);
+            e1 = rows[(size_t)(r + 2) * 32];
             if (NISE_SCHED_Q(c.e) != NISE_SCHED_NONE) {
                 const int a = NISE_SCHED_A(c.p), b = NISE_SCHED_B(c.p);
                 double2 xa = X[a], xb = X[b];
@@ -345,10 +356,6 @@ __global__ void __launch_bounds__(96) k_adj_bwd_warp(DevTraj T, AdjPlan P, AbsJo
     double2 *ush = rsh + (SM ? (size_t)P.W * P.k : 0);
     double *jsh = (double *)(ush + (SM ? (size_t)P.W * n : 0));
     float *mu = (float *)(jsh + (SM ? (size_t)P.W * P.k : 0)) + (size_t)x * P.W * n;  // [3][W][n]
-    uint32_t *psh = (uint32_t *)((float *)(jsh + (SM ? (size_t)P.W * P.k : 0)) + 3 * (size_t)P.W * n);
-    const uint32_t *parts = SM ? psh : P.parts;
-    if (SM)
-        for (int e = threadIdx.x; e < P.k; e += blockDim.x) psh[e] = P.parts[e];
     const long ti = (long)(J.begin + blockIdx.x) * J.sample;
     const double2 *ck = ckpt + (size_t)v * P.nck * n;
     const double hf = 0.5 * P.f;
@@ -361,7 +368,7 @@ __global__ void __launch_bounds__(96) k_adj_bwd_warp(DevTraj T, AdjPlan P, AbsJo
     }
     for (int t2 = J.tmax - 1; t2 > 0;) {  // the window [t1, t2), whole windows at multiples of W
         const int steps = t2 % P.W == 0 ? P.W : 1, t1 = t2 - steps;
-        const uint32_t *rows = steps == P.W ? P.schedW : P.sched1;
+        const uint2 *rows = steps == P.W ? P.schedW : P.sched1;
         const int nrow = steps == P.W ? P.nrowW : P.nrow1;
         const long fi = ti + t1 - P.f0;
         const double2 *rot = P.rot + fi * P.k, *U = P.U + fi * n;
@@ -376,11 +383,12 @@ __global__ void __launch_bounds__(96) k_adj_bwd_warp(DevTraj T, AdjPlan P, AbsJo
             __syncthreads();
         }
         __syncwarp();
-        AdjCoef c = adj_coef(P, nrow > 0 ? rows[(size_t)(nrow - 1) * 32 + lane] : NISE_SCHED_NONE, parts, rot, U);
-        uint32_t e1 = nrow > 1 ? rows[(size_t)(nrow - 2) * 32 + lane] : NISE_SCHED_NONE;
-        for (int r = nrow - 1; r >= 0; r--) {
-            const AdjCoef nx = adj_coef(P, e1, parts, rot, U);
-            e1 = r - 2 >= 0 ? rows[(size_t)(r - 2) * 32 + lane] : NISE_SCHED_NONE;
+        rows += (long)(nrow - 1) * 32 + lane;
+        AdjCoef c = adj_coef(P, rows[0], rot, U);
+        uint2 e1 = rows[-32];
+        for (int r = nrow - 1; r >= 0; r--, rows -= 32) {
+            const AdjCoef nx = adj_coef(P, e1, rot, U);
+            e1 = rows[-64];
             const uint32_t q = NISE_SCHED_Q(c.e);
             if (q != NISE_SCHED_NONE) {
                 const int a = NISE_SCHED_A(c.p), b = NISE_SCHED_B(c.p), w = NISE_SCHED_W(c.e);
@@ -454,11 +462,256 @@ __global__ void __launch_bounds__(96) k_adj_bwd_warp(DevTraj T, AdjPlan P, AbsJo
 
 // Shared memory of the warp kernels: without the window's coefficients, and with them.
 size_t adj_fwd_bytes(int n, int k, int W, bool sm) {
-    return sizeof(double2) * 3 * (size_t)W * n + (sm ? sizeof(double2) * (size_t)W * (k + n) + 4 * (size_t)k : 0);
+    return sizeof(double2) * 3 * (size_t)W * n + (sm ? sizeof(double2) * (size_t)W * (k + n) : 0);
 }
 size_t adj_bwd_bytes(int n, int k, int W, bool sm) {
     return sizeof(double2) * 6 * (size_t)n + sizeof(double) * (3 * (size_t)n + (n & 1)) + sizeof(float) * 3 * (size_t)W * n +
-           (sm ? (sizeof(double2) * (size_t)(k + n) + sizeof(double) * k) * W + 4 * (size_t)k : 0);
+           (sm ? (sizeof(double2) * (size_t)(k + n) + sizeof(double) * k) * W : 0);
+}
+
+// The same sweeps on one complex 2x2 matrix per rotation and frame, the rotation
+// with the half phases that belong to it: M = D_post R D_pre, built for a window in
+// shared memory (four planes, so that neighbouring rotations meet no bank
+// conflict they need not), shared by the three polarisations and the ts sub-steps.
+// A row is then two loads of the state, 16 multiply-adds without a branch and two
+// stores, and the next row's matrix is in flight meanwhile.  Backward M^H = M^-1
+// takes both the state and its adjoint back.  The derivative terms need no state
+// between the factors of M: a phase's (l x y) is the same on both of its sides, and
+// a rotation's is Im(jf q_a conj(q_b) (conj(l_a) y_b - l_b conj(y_a))), q the phases
+// after it.  Taken where a window's matrices leave room for two CTAs per SM (256-site
+// chain, 244 start points: forward 3.6 -> 2.0 ms, backward 5.6 -> 4.0 ms against the
+// kernels above; even and odd sites apart, see adj_pos, are 10 % of it).
+__device__ __forceinline__ void adj_mats(const AdjPlan &P, long fi, int steps, double2 *M) {
+    const double2 one = make_double2(1, 0);
+    const int plane = P.W * P.k + 1;  // the identity last, for idle places
+    if (threadIdx.x < 4) M[threadIdx.x * plane + plane - 1] = make_double2(threadIdx.x % 3 == 0, 0);
+#pragma unroll 2
+    for (int e = threadIdx.x; e < steps * P.k; e += blockDim.x) {
+        const int w = e / P.k, q = e - w * P.k, o = w * P.k + adj_pos(q, P.k);
+        const uint32_t p = P.parts[q];
+        const double2 cs = P.rot[fi * P.k + e], *U = P.U + (fi + w) * P.n;
+        const double2 ua = U[NISE_SCHED_A(p)], ub = U[NISE_SCHED_B(p)];
+        const double2 pa = NISE_SCHED_PRE_A(p) ? ua : one, pb = NISE_SCHED_PRE_B(p) ? ub : one;
+        const double2 qa = NISE_SCHED_POST_A(p) ? ua : one, qb = NISE_SCHED_POST_B(p) ? ub : one;
+        const double2 aa = cmul(pa, qa), ab = cmul(pb, qa), ba = cmul(pa, qb), bb = cmul(pb, qb);
+        M[o] = make_double2(cs.x * aa.x, cs.x * aa.y);
+        M[plane + o] = make_double2(-cs.y * ab.y, cs.y * ab.x);
+        M[2 * plane + o] = make_double2(-cs.y * ba.y, cs.y * ba.x);
+        M[3 * plane + o] = make_double2(cs.x * bb.x, cs.x * bb.y);
+    }
+}
+
+struct AdjMat {
+    double2 aa, ab, ba, bb;
+};
+
+// A schedule entry's matrix: the low bits of e index the planes.
+__device__ __forceinline__ AdjMat adj_mat(const double2 *M, int plane, uint32_t e) {
+    M += NISE_SCHED_Q(e);
+    return AdjMat{M[0], M[plane], M[2 * plane], M[3 * plane]};
+}
+
+// m x + k y, and with the conjugates of m and k
+__device__ __forceinline__ double2 mad2(double2 m, double2 x, double2 k, double2 y) {
+    return make_double2(m.x * x.x - m.y * x.y + k.x * y.x - k.y * y.y, m.x * x.y + m.y * x.x + k.x * y.y + k.y * y.x);
+}
+__device__ __forceinline__ double2 mad2c(double2 m, double2 x, double2 k, double2 y) {
+    return make_double2(m.x * x.x + m.y * x.y + k.x * y.x + k.y * y.y, m.x * x.y - m.y * x.x + k.x * y.y - k.y * y.x);
+}
+
+size_t adj_mat_fwd_bytes(int n, int k, int W) {
+    return sizeof(double2) * (4 * ((size_t)W * k + 1) + 3 * ((size_t)W * n + 1));
+}
+size_t adj_mat_bwd_bytes(int n, int k, int W) {
+    return sizeof(double2) * (4 * ((size_t)W * k + 1) + W + 6 * ((size_t)n + 1)) + sizeof(double) * 3 * ((size_t)n + 1) +
+           sizeof(float) * 3 * (size_t)W * n;
+}
+
+__global__ void __launch_bounds__(96) k_adj_fwd_mat(DevTraj T, AdjPlan P, AbsJob J, double2 *resp, double2 *ckpt) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int n = P.n, lane = threadIdx.x & 31, x = threadIdx.x >> 5, v = 3 * blockIdx.x + x, plane = P.W * P.k + 1;
+    // [X n, the idle places' site, W - 1 snapshots of n]
+    double2 *M = (double2 *)smem_raw, *X = M + 4 * (size_t)plane + (size_t)x * (P.W * n + 1), *snap = X + n + 1;
+    if (lane == 0) X[n] = make_double2(0, 0);
+    const long ti = (long)(J.begin + blockIdx.x) * J.sample;
+    for (int a = lane; a < n; a += 32) X[adj_pos(a, n)] = make_double2((double)traj_mu(T, ti, x, a), 0.0);
+    double2 *ck = ckpt + (size_t)v * P.nck * n;
+    auto respond = [&](int t1, const double2 *Z) {
+        double re = 0, im = 0;
+        for (int a = lane; a < n; a += 32) {
+            const double m = (double)traj_mu(T, ti + t1, x, a);
+            const double2 z = Z[adj_pos(a, n)];
+            re += m * z.x;
+            im += m * z.y;
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            re += __shfl_xor_sync(0xffffffffu, re, o);
+            im += __shfl_xor_sync(0xffffffffu, im, o);
+        }
+        if (lane == 0) resp[(size_t)v * J.tmax + t1] = make_double2(re, im);
+    };
+    __syncwarp();
+    int t1 = 0;
+    while (true) {
+        respond(t1, X);
+        if (t1 % P.K == 0)
+            for (int a = lane; a < n; a += 32) ck[(size_t)(t1 / P.K) * n + a] = X[adj_pos(a, n)];
+        if (t1 == J.tmax - 1) break;
+        const int steps = J.tmax - 1 - t1 >= P.W ? P.W : 1;
+        const uint2 *rows = (steps == P.W ? P.schedW : P.sched1) + lane;
+        const int nrow = steps == P.W ? P.nrowW : P.nrow1;
+        const long fi = ti + t1 - P.f0;
+        __syncthreads();
+        adj_mats(P, fi, steps, M);
+        __syncthreads();
+        uint2 c = rows[0], c1 = rows[32];
+        AdjMat m = adj_mat(M, plane, c.y);
+#pragma unroll 2
+        for (int r = 0; r < nrow; r++, rows += 32) {
+            double2 *A = X + NISE_SCHED_A(c.x), *B = X + NISE_SCHED_B(c.x);
+            const double2 xa = *A, xb = *B;
+            const AdjMat m1 = adj_mat(M, plane, c1.y);
+            const uint2 c2 = rows[64];
+            const double2 ya = mad2(m.aa, xa, m.ab, xb), yb = mad2(m.ba, xa, m.bb, xb);
+            *A = ya;
+            *B = yb;
+            const int w = NISE_SCHED_W(c.y);
+            const bool last = NISE_SCHED_LAST(c.y) && w < steps - 1;
+            if (last && NISE_SCHED_POST_A(c.x)) A[(w + 1) * n + 1] = ya;
+            if (last && NISE_SCHED_POST_B(c.x)) B[(w + 1) * n + 1] = yb;
+            __syncwarp();
+            m = m1;
+            c = c1;
+            c1 = c2;
+        }
+        for (int i = lane; i < P.niso; i += 32) {
+            const int a = P.iso[i], o = adj_pos(a, n);
+            double2 z = X[o];
+            for (int w = 0; w < steps; w++) {
+                const double2 u = P.U[(fi + w) * n + a];
+                for (int s = 0; s < 2 * P.ts; s++) z = cmul(u, z);
+                if (w < steps - 1) snap[(size_t)w * n + o] = z;
+            }
+            X[o] = z;
+        }
+        __syncwarp();
+        for (int w = 0; w < steps - 1; w++) respond(t1 + w + 1, snap + (size_t)w * n);
+        __syncwarp();
+        t1 += steps;
+    }
+    for (int a = lane; a < n; a += 32) ck[(size_t)(P.nck - 1) * n + a] = X[adj_pos(a, n)];
+}
+
+__global__ void __launch_bounds__(96) k_adj_bwd_mat(DevTraj T, AdjPlan P, AbsJob J, const double2 *G,
+                                                    const double2 *ckpt, double *gshift, double *gscale) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int n = P.n, lane = threadIdx.x & 31, x = threadIdx.x >> 5, v = 3 * blockIdx.x + x, plane = P.W * P.k + 1,
+              n1 = n + 1;  // the idle places' site last
+    double2 *M = (double2 *)smem_raw, *Gw = M + 4 * (size_t)plane, *X = Gw + P.W + 2 * (size_t)x * n1, *L = X + n1;
+    double *gs0 = (double *)(Gw + P.W + 6 * (size_t)n1), *gs = gs0 + (size_t)x * n1;
+    float *mu = (float *)(gs0 + 3 * (size_t)n1) + (size_t)x * P.W * n;  // [3][W][n]
+    if (lane == 0) {
+        X[n] = L[n] = make_double2(0, 0);
+        gs[n] = 0;
+    }
+    const long ti = (long)(J.begin + blockIdx.x) * J.sample;
+    const double2 *ck = ckpt + (size_t)v * P.nck * n;
+    const double hf = 0.5 * P.f;
+    double gsc = 0;
+    for (int a = lane; a < n; a += 32) {
+        const double m = (double)traj_mu(T, ti + J.tmax - 1, x, a);
+        const int o = adj_pos(a, n);
+        X[o] = ck[(size_t)(P.nck - 1) * n + a];
+        L[o] = make_double2(m * G[J.tmax - 1].x, m * G[J.tmax - 1].y);
+        gs[o] = 0;
+    }
+    for (int t2 = J.tmax - 1; t2 > 0;) {  // the window [t1, t2), whole windows at multiples of W
+        const int steps = t2 % P.W == 0 ? P.W : 1, t1 = t2 - steps;
+        const int nrow = steps == P.W ? P.nrowW : P.nrow1;
+        const uint2 *rows = (steps == P.W ? P.schedW : P.sched1) + (long)(nrow - 1) * 32 + lane;
+        const long fi = ti + t1 - P.f0;
+        const double2 *je = P.je + fi * P.k;
+        for (int w = 0; w < steps; w++)
+            for (int a = lane; a < n; a += 32) mu[w * n + adj_pos(a, n)] = traj_mu(T, ti + t1 + w, x, a);
+        __syncthreads();
+        if (threadIdx.x < steps) Gw[threadIdx.x] = G[t1 + threadIdx.x];
+        adj_mats(P, fi, steps, M);
+        __syncthreads();
+        auto jcoef = [&](uint32_t e) { return je[(int)NISE_SCHED_Q(e) == plane - 1 ? 0 : NISE_SCHED_Q(e)]; };
+        uint2 c = rows[0], c1 = rows[-32];
+        AdjMat m = adj_mat(M, plane, c.y);
+        double2 j = jcoef(c.y);
+#pragma unroll 2
+        for (int r = nrow - 1; r >= 0; r--, rows -= 32) {
+            const int a = NISE_SCHED_A(c.x), b = NISE_SCHED_B(c.x);
+            const double2 ya = X[a], yb = X[b], la = L[a], lb = L[b];
+            const double ga0 = gs[a], gb0 = gs[b];
+            const AdjMat m1 = adj_mat(M, plane, c1.y);
+            const double2 j1 = jcoef(c1.y);
+            const uint2 c2 = rows[-64];
+            const double2 xa = mad2c(m.aa, ya, m.ba, yb), xb = mad2c(m.ab, ya, m.bb, yb);
+            double2 ka = mad2c(m.aa, la, m.ba, lb), kb = mad2c(m.ab, la, m.bb, lb);
+            X[a] = xa;
+            X[b] = xb;
+            const double dx = la.x * yb.x + la.y * yb.y - lb.x * ya.x - lb.y * ya.y;
+            const double dy = la.x * yb.y - la.y * yb.x + lb.x * ya.y - lb.y * ya.x;
+            gsc += j.x * dy + j.y * dx;
+            double ga = 0, gb = 0;
+            if (NISE_SCHED_POST_A(c.x)) ga = la.x * ya.y - la.y * ya.x;
+            if (NISE_SCHED_POST_B(c.x)) gb = lb.x * yb.y - lb.y * yb.x;
+            if (NISE_SCHED_PRE_A(c.x)) ga += ka.x * xa.y - ka.y * xa.x;
+            if (NISE_SCHED_PRE_B(c.x)) gb += kb.x * xb.y - kb.y * xb.x;
+            const int w = NISE_SCHED_W(c.y);
+            if (NISE_SCHED_FIRST(c.y) && w > 0) {  // back at the start of step t1 + w
+                const double2 g = Gw[w];
+                if (NISE_SCHED_PRE_A(c.x)) {
+                    const double d = (double)mu[(size_t)w * n + a];
+                    ka = make_double2(ka.x + d * g.x, ka.y + d * g.y);
+                }
+                if (NISE_SCHED_PRE_B(c.x)) {
+                    const double d = (double)mu[(size_t)w * n + b];
+                    kb = make_double2(kb.x + d * g.x, kb.y + d * g.y);
+                }
+            }
+            L[a] = ka;
+            L[b] = kb;
+            gs[a] = ga0 + hf * ga;
+            gs[b] = gb0 + hf * gb;
+            __syncwarp();
+            m = m1;
+            j = j1;
+            c = c1;
+            c1 = c2;
+        }
+        for (int i = lane; i < P.niso; i += 32) {
+            const int a = P.iso[i], o = adj_pos(a, n);
+            double2 z = X[o], l = L[o];
+            double ga = 0;
+            for (int w = steps - 1; w >= 0; w--) {
+                const double2 u = P.U[(fi + w) * n + a];
+                for (int s = 0; s < 2 * P.ts; s++) adj_unphase(u, hf, z, l, ga);
+                if (w > 0) {
+                    const double d = (double)mu[(size_t)w * n + o];
+                    l = make_double2(l.x + d * Gw[w].x, l.y + d * Gw[w].y);
+                }
+            }
+            X[o] = z;
+            L[o] = l;
+            gs[o] += ga;
+        }
+        __syncwarp();
+        for (int a = lane; a < n; a += 32) {
+            const int o = adj_pos(a, n);
+            if (t1 % P.K == 0) X[o] = ck[(size_t)(t1 / P.K) * n + a];
+            const double m0 = (double)mu[o];
+            L[o] = make_double2(L[o].x + m0 * Gw[0].x, L[o].y + m0 * Gw[0].y);
+        }
+        __syncwarp();
+        t2 = t1;
+    }
+    for (int a = lane; a < n; a += 32) gshift[(size_t)v * n + a] = gs[adj_pos(a, n)];
+    for (int o = 16; o > 0; o >>= 1) gsc += __shfl_xor_sync(0xffffffffu, gsc, o);
+    if (lane == 0) gscale[v] = gsc;
 }
 
 // Deterministic sums over vectors: g[a] = sum_v part[v][a] (a < n), in v order.
@@ -470,8 +723,8 @@ __global__ void k_adj_reduce(const double *part, int nvec, int n, double *g) {
     g[a] = s;
 }
 
-// Two CTAs per SM where the coefficients are staged.
-constexpr size_t kAdjShared = 112 * 1024;
+// Two CTAs per SM where the coefficients are staged (228 KB, 1 KB of it each CTA's).
+constexpr size_t kAdjShared = 113 * 1024;
 
 int lanes_adj(size_t lane_bytes) {
     int B = 64;
@@ -787,8 +1040,8 @@ int launch_adj_fwd(const DevTraj &T, const AdjPlan &P, const AbsJob &J, double2 
     const int nvec = 3 * J.nsamp;
     if (P.sched1) {
         const bool sm = adj_fwd_bytes(P.n, P.k, P.W, true) <= kAdjShared;
-        const size_t by = adj_fwd_bytes(P.n, P.k, P.W, sm);
-        auto kern = sm ? k_adj_fwd_warp<true> : k_adj_fwd_warp<false>;
+        const size_t by = P.mat ? adj_mat_fwd_bytes(P.n, P.k, P.W) : adj_fwd_bytes(P.n, P.k, P.W, sm);
+        auto kern = P.mat ? k_adj_fwd_mat : sm ? k_adj_fwd_warp<true> : k_adj_fwd_warp<false>;
         if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)by)) return (int)e;
         kern<<<J.nsamp, 96, by, s>>>(T, P, J, resp, ckpt);
         return (int)cudaGetLastError();
@@ -807,8 +1060,8 @@ int launch_adj_bwd(const DevTraj &T, const AdjPlan &P, const AbsJob &J, const do
     const int nvec = 3 * J.nsamp;
     if (P.sched1) {
         const bool sm = adj_bwd_bytes(P.n, P.k, P.W, true) <= kAdjShared;
-        const size_t by = adj_bwd_bytes(P.n, P.k, P.W, sm);
-        auto kern = sm ? k_adj_bwd_warp<true> : k_adj_bwd_warp<false>;
+        const size_t by = P.mat ? adj_mat_bwd_bytes(P.n, P.k, P.W) : adj_bwd_bytes(P.n, P.k, P.W, sm);
+        auto kern = P.mat ? k_adj_bwd_mat : sm ? k_adj_bwd_warp<true> : k_adj_bwd_warp<false>;
         if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)by)) return (int)e;
         kern<<<J.nsamp, 96, by, s>>>(T, P, J, G, ckpt, gshift_part, gscale_part);
     } else {
@@ -866,7 +1119,8 @@ struct AdjRun {
 
 // Schedules of the warp kernels.
 struct AdjSched {
-    DevBuf<uint32_t> s1, sW, parts;
+    DevBuf<uint2> s1, sW;
+    DevBuf<uint32_t> parts;
     DevBuf<int> iso;
     int build(nise_ctx *c, const std::vector<int2> &pairs, AdjPlan &P) {
         // one vector's state, its adjoint and gradient on a warp of three: up
@@ -884,19 +1138,46 @@ struct AdjSched {
         // four) and its coefficients fit beside another CTA's
         const int W = 4;
         const bool narrow = (size_t)P.k * P.ts < 12 * (size_t)P.nrow1;
-        if (narrow && std::max(adj_fwd_bytes(P.n, P.k, W, true), adj_bwd_bytes(P.n, P.k, W, true)) <= kAdjShared) {
+        auto mat = [&](int w) {
+            return P.k > 0 && std::max(adj_mat_fwd_bytes(P.n, P.k, w), adj_mat_bwd_bytes(P.n, P.k, w)) <= kAdjShared;
+        };
+        if (narrow && (mat(W) || std::max(adj_fwd_bytes(P.n, P.k, W, true), adj_bwd_bytes(P.n, P.k, W, true)) <= kAdjShared)) {
             P.W = W;
             nise_step_schedule(pairs, P.n, P.ts, W, rW);
         } else {
             rW = r1;
         }
+        P.mat = mat(P.W);
         P.nrowW = (int)(rW.size() / 32);
         P.niso = (int)is.size();
+        // the rotation's packed sites beside each entry, two idle rows on either
+        // side (the kernels read two rows ahead, in both directions).  With `mat`
+        // the entry names the matrix and idle places turn site n by the
+        // identity at W k
+        auto words = [&](const std::vector<uint32_t> &e) {
+            const uint2 idle = P.mat ? make_uint2((uint32_t)P.n | (uint32_t)P.n << 14, (uint32_t)(P.W * P.k))
+                                     : make_uint2(0, NISE_SCHED_NONE);
+            std::vector<uint2> w(64, idle);
+            for (uint32_t x : e) {
+                const uint32_t q = NISE_SCHED_Q(x);
+                if (q == NISE_SCHED_NONE)
+                    w.push_back(idle);
+                else if (P.mat)
+                    w.push_back(make_uint2((pt[q] & 0xf0000000u) | (uint32_t)adj_pos(NISE_SCHED_A(pt[q]), P.n) |
+                                               (uint32_t)adj_pos(NISE_SCHED_B(pt[q]), P.n) << 14,
+                                           x - q + NISE_SCHED_W(x) * P.k + adj_pos(q, P.k)));
+                else
+                    w.push_back(make_uint2(pt[q], x));
+            }
+            w.insert(w.end(), 64, idle);
+            return w;
+        };
         int rc;
-        if ((rc = s1.upload(c, r1)) || (rc = sW.upload(c, rW)) || (rc = parts.upload(c, pt)) || (rc = iso.upload(c, is)))
+        if ((rc = s1.upload(c, words(r1))) || (rc = sW.upload(c, words(rW))) || (rc = parts.upload(c, pt)) ||
+            (rc = iso.upload(c, is)))
             return rc;
-        P.sched1 = s1.p;
-        P.schedW = sW.p;
+        P.sched1 = s1.p + 64;
+        P.schedW = sW.p + 64;
         P.parts = parts.p;
         P.iso = iso.p;
         return NISE_OK;
@@ -937,16 +1218,17 @@ int adj_forward(nise_ctx *c, const double *shift, double scale, int K, AdjRun &R
     P.scale = scale;
     P.f = nise_f64(p, 1, p.ts);
     std::vector<double> hs(shift, shift + N);
+    if ((rc = Q.build(c, pairs, P))) return rc;
     if ((rc = dshift.upload(c, hs)) || (rc = dpairs.upload(c, pairs.empty() ? std::vector<int2>(1) : pairs)) ||
         (rc = U.alloc(c, (size_t)R.nf * N)) || (rc = rot.alloc(c, (size_t)R.nf * (P.k ? P.k : 1))) ||
-        (rc = jf.alloc(c, (size_t)R.nf * (P.k ? P.k : 1))) || (rc = ckpt.alloc(c, (size_t)nvec * P.nck * N)))
+        (rc = jf.alloc(c, (size_t)R.nf * (P.k ? P.k : 1) * (P.mat ? 2 : 1))) || (rc = ckpt.alloc(c, (size_t)nvec * P.nck * N)))
         return rc;
     P.shift = dshift.p;
     P.pairs = dpairs.p;
     P.U = U.p;
     P.rot = rot.p;
     P.jf = jf.p;
-    if ((rc = Q.build(c, pairs, P))) return rc;
+    P.je = (double2 *)jf.p;
     memset(&J, 0, sizeof(J));
     J.begin = R.begin;
     J.nsamp = R.nsamp;

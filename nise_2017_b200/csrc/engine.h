@@ -232,11 +232,15 @@ struct AdjPlan {
     double scale, f;       // coupling scale, deltat*icm2ifs*2pi/ts
     double2 *U, *rot;
     double *jf;
+    double2 *je;           // with `mat`, in place of jf: jf with the phases after the rotation
     // schedules of one time step and of a window of W (rotsched.h: rows of 32
-    // rotations), the rotations' packed sites and the sites without any; null
-    // above the size of the warp kernels
-    const uint32_t *sched1, *schedW, *parts;
+    // rotations, {packed sites, entry}, two idle rows before and after), the
+    // rotations' packed sites and the sites without any; null above the size of the
+    // warp kernels.  mat: the kernels on one matrix per rotation
+    const uint2 *sched1, *schedW;
+    const uint32_t *parts;
     int nrow1, nrowW, W;
+    bool mat;
     const int *iso;
     int niso;
 };
