@@ -132,11 +132,13 @@ typedef struct {
                                       per CTA, 10 the sliced-ELL Chebyshev kernel (FP32), 15 the
                                       row-owner Chebyshev kernel (FP32), 12 the sliced-ELL Taylor
                                       kernel with 4 vectors per CTA (FP32);
-                                      2 the eigen route (explicit per-frame propagators, up to
-                                      2048 sites batched in FP32, else 1024), 16 / 17 its
-                                      propagators applied per start point / on the tensor cores;
+                                      2 the eigen route (every frame diagonalised, its
+                                      propagator up to 2048 sites batched in FP32, else 1024),
+                                      16 / 17 explicit per-frame propagators applied per start
+                                      point / on the tensor cores;
                                       2D techniques, Trotter doubles: 1 one warp per doubles
-                                      vector (else two warps per vector for 32 < N <= 64,
+                                      vector (else, up to 64 sites, two vectors together in
+                                      FP32 and two warps per vector for 32 < N in FP64,
                                       bitwise the same result) */
     char positionFName[256];       /* Positionfile (TransitionDipole / ExtendedDipole; CD) */
     char pbcFName[256];            /* PBCfile: periodic box per frame (optional) */

@@ -1,4 +1,4 @@
-// Eigen-route exact propagator for linear absorption: Propagation Diagonal,
+// Exact propagators of linear absorption, built and applied: Propagation Diagonal,
 // and Propagation Sparse where the static-coupling Taylor route does not
 // apply (HamiltonianType Full, or a Threshold that truncates U).
 //
@@ -7,11 +7,11 @@
 // frame and applies it (propagate_vec_DIA, propagate.c:60-125), or applies
 // only the elements with |U_ab|^2 > Threshold (propagate_vec_DIA_S,
 // :185-258; Threshold pre-scaled by (f/ts)^2 at input, readinput.c:264-267).
-// Here every frame is diagonalised once (FP64 Jacobi, eigen.cu), U is built
-// once per frame in FP64 and rounded to the working precision, truncated by
-// the same test in the working precision, and shared by every start point
-// and polarisation that crosses the frame.  U is complex symmetric (V is
-// real orthogonal), so it is stored once and read along rows.
+// Here U is built once per frame in FP64 (propagators.cu; with kernel_config 2
+// from an eigendecomposition, eigen.cu and k_build_u), rounded to the working
+// precision, truncated by the same test in the working precision, and shared
+// by every start point and polarisation that crosses the frame.  U is complex
+// symmetric, so it is stored once and read along rows.
 #include <algorithm>
 
 #include "common.cuh"

@@ -1,7 +1,8 @@
 // Batched FP64 symmetric eigensolver for per-frame Hamiltonians.
 //
 // Replaces the reference's LAPACK ssyev_ calls (diagonalizeLPD,
-// propagate.c:1185-1221) used by propagate_t2_DIA and the exact propagators.
+// propagate.c:1185-1221) used by propagate_t2_DIA, luminescence's Boltzmann
+// weights and, with kernel_config 2, the exact propagators (else propagators.cu).
 // One CTA diagonalises one frame with the parallel (Brent-Luk round-robin)
 // cyclic Jacobi method in shared memory: every round applies N/2 disjoint
 // rotations to both sides of A at once, block by block, and accumulates the

@@ -3,8 +3,9 @@
 //
 // Replaces the reference's LAPACK ssyev_ (diagonalizeLPD,
 // propagate.c:1185-1221) and its naive N^3 transform to the site basis
-// (propagate_vec_DIA, propagate.c:89-106) for the exact propagators of
-// Propagation Sparse / Diagonal and the t2 step.  One CTA per frame, the
+// (propagate_vec_DIA, propagate.c:89-106) for the t2 step, luminescence's
+// Boltzmann weights and, with kernel_config 2, the exact propagators of
+// Propagation Sparse / Diagonal (else propagators.cu).  One CTA per frame, the
 // matrix in global memory:
 //
 //  1. Householder tridiagonalisation, A = Q T Q^T (Golub & Van Loan,

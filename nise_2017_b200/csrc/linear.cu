@@ -18,10 +18,11 @@
 //   Lum    3 vectors rho mu_x(ti), rho the equilibrium density matrix at the
 //          Temperature (below); read-out mu_x(tj); channels total, x, y, z
 //
-// One thread propagates one vector (the [site][lane] shared-memory layout and
-// the singles_step of the 2D kernels, so every vector sees the reference's
-// single-precision operations in FP32 mode) and writes its read-outs of every
-// t1 to a per-vector array; a second kernel sums them per channel in a fixed
+// A warp or two propagate a vector on rows of operations (Trotter, k_lin_rows), a
+// group of threads on a frame's propagator (Sparse and Diagonal, k_lin_dia), else a
+// thread (k_lin: RK4, and Trotter tables too large for rows); every vector sees the
+// reference's single-precision operations in FP32 mode.  The read-outs of every
+// t1 go to a per-vector array; a second kernel sums them per channel in a fixed
 // order (FP64 sums, as the absorption path).  Products keep the reference's
 // float operand order; the scalings by -0.5, 2 and 1/2 are exact.
 //

@@ -28,8 +28,13 @@
 //   k2d_gb3      mut3_x: mu_x(tk) propagated through t3; GB t3 dots
 //   k2d_t2       t2 eigen steps (propagate_t2_DIA) of leftr_x and leftn_x[t1]
 //   k2d_se       SE t3 propagation of leftr_x and leftn_x[t1], snapshots per t3
+//                (each a warp per vector on rows of operations where Trotter tables
+//                fit, k2d_*_rows, else a thread per vector)
 //   k2d_doubles  doubles (two-exciton) Trotter propagation of fr / ft1[t1],
-//                dipole_double_last projections and EA dot products per t3
+//                dipole_double_last projections and EA dot products per t3;
+//                FP32 up to 64 sites two vectors together (k2d_doubles_pair), FP64 of
+//                33 to 64 sites two warps per vector (k2d_doubles_duo)
+//   k2d_doubles_sparse32/64, k2d_doubles_seq  the same for Sparse/Diagonal and RK4
 //   k2d_response GB + SE + EA contributions per (start point, t3, t1) with the
 //                21 molecular-frame weights and the lifetime factors
 // followed by a deterministic sum over start points.
