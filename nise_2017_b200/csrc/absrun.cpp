@@ -346,6 +346,13 @@ struct AbsRun {
     long vec_steps = 0;
     double alg_bytes = 0;  // every frame read once (diagonal or full record) and the dipoles
 
+    // the tuned configuration of this job's key, else `otherwise`
+    int tuned(const TrotterPlan &P, int otherwise = 0) const {
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        const auto it = g_tuned.find(TuneKey(scheme, prec, N, scheme == SCHEME_TROTTER ? P.k : 0,
+                                             scheme == SCHEME_TROTTER ? P.rot_static : 0));
+        return it != g_tuned.end() ? it->second : otherwise;
+    }
     int plan(nise_ctx *ctx, bool autotune);
     int enqueue(cudaStream_t s, bool events);
     // The static-coupling series kernels wave by wave, each wave after the
@@ -772,7 +779,10 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
                 ell4_nslices = ns4;
                 ell4_nent = sp4[ns4];
             }
-            if (prec == NISE_FP32) {
+            // (where its kernel may run: not for the sizes and vectors that
+            // default_config gives to the 4-vector kernels)
+            const bool any = autotune || p.kernel_config != 0 || tuned(TP);
+            if (prec == NISE_FP32 && N <= 1024 && (any || plain || nvec >= 8 * sm_count() || N >= 300)) {
                 // Row-owner layout: 8-row slices whose rows alternate in parity, so
                 // that the two rows of a quarter-warp are of different parity, and
                 // slot triples.  A slot is free of bank conflicts where they gather
@@ -880,7 +890,7 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
                 // its slices' order
                 const int shapes[2] = {24, 32};
                 ell8_ntg = ntg;
-                for (int sh = 0; sh < 2 && N <= 1024 && ntg < 4096; sh++) {
+                for (int sh = 0; sh < (any ? 2 : 1) && ntg < 4096; sh++) {
                     const int nw = shapes[sh];
                     std::vector<int> order(ns8), load(nw, 0), cnt(nw, 0), wl(nw * 8, -1);
                     for (int sl = 0; sl < ns8; sl++) order[sl] = sl;
@@ -973,12 +983,7 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
         else return nise_fail(c, NISE_ERR_ARG, "kernel_config %d does not apply to this scheme", k);
         return NISE_OK;
     }
-    {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        auto it = g_tuned.find(TuneKey(scheme, prec, N, scheme == SCHEME_TROTTER ? TP.k : 0,
-                                       scheme == SCHEME_TROTTER ? TP.rot_static : 0));
-        if (it != g_tuned.end()) config = it->second;
-    }
+    config = tuned(TP, config);
     if (autotune && (scheme == SCHEME_TROTTER || scheme == SCHEME_TAYLOR) && !plain)
         if ((rc = tune())) return rc;
     return NISE_OK;
