@@ -990,7 +990,7 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
 }
 
 // exp(-i H f) from its Taylor polynomials (1987 frames of 48 sites: 0.50 ms
-// against 4.9 by eigenvectors; 595 frames of 200 sites: 10.8 against 70.7), or,
+// against 4.9 by eigenvectors; 595 frames of 200 sites: 8.1 against 70.7), or,
 // where the caller asked for it, from every frame's eigenvectors.
 int AbsRun::build_u(long q, long m, void *dst, cudaStream_t s) {
     const int pr = prec == NISE_FP32 ? 0 : 1;

@@ -22,8 +22,9 @@
 // are polynomials in H, hence symmetric: only tiles on and above the diagonal
 // are computed, the others mirrored, and both operands of a product are read
 // along rows.  A thread holds 4 x 4 results; the tile is N / ceil(N / 64)
-// rounded up to 4, so little of it is padding.  Bound by the FP64 pipe: 48
-// sites, 1987 frames 0.50 ms (Jacobi 4.8 ms); 200 sites, 595 frames 10.8 ms
+// rounded up to 4, so little of it is padding.  Bound by operand loads (L2, then
+// shared memory: 8 values for 16 multiply-adds) with two CTAs per SM to hide them: 48
+// sites, 1987 frames 0.50 ms (Jacobi 4.8 ms); 200 sites, 595 frames 8.1 ms
 // (Householder and QR 69.3 ms, then 1.4 ms for U).
 #include <algorithm>
 
@@ -96,6 +97,83 @@ __device__ void pu_gemm(const PuTile &Q, double *out, const double *A, const Lin
     __syncthreads();
 }
 
+// The same with the next step's operands loaded while this one's are multiplied:
+// with several tiles a third of the time was the wait for them (200 sites, 595
+// frames: 10.8 -> 8.1 ms).  A single tile has few steps and other CTAs beside it, and
+// is faster without (CD, 40 sites, FP64, whole job: 1.09 against 1.12 ms).
+__device__ void pu_gemm_ahead(const PuTile &Q, double *out, const double *A, const Lin B, const Lin E) {
+    constexpr int F = 6;  // elements a thread has in flight
+    const int n = Q.n, tid = threadIdx.x, cx = tid % Q.tx * 4, cy = tid / Q.tx * 4;
+    const bool act = tid < Q.tx * Q.tx;
+    int pos[F];
+    double fa[F], f1[F], f2[F];
+#pragma unroll
+    for (int u = 0; u < F; u++) {
+        const int e = tid + u * blockDim.x;
+        pos[u] = e < kPuK * Q.tile ? e / Q.tile << 8 | e % Q.tile : -1;
+    }
+    auto fetch = [&](int k0, int i0, int j0) {
+#pragma unroll
+        for (int u = 0; u < F; u++) {
+            const int k = k0 + (pos[u] >> 8), q = pos[u] & 255;
+            const bool in = pos[u] >= 0 && k < n;
+            const size_t r = (size_t)k * n;
+            fa[u] = in && i0 + q < n ? A[r + i0 + q] : 0.0;
+            f1[u] = in && j0 + q < n && B.m1 ? B.m1[r + j0 + q] : 0.0;
+            f2[u] = in && j0 + q < n && B.m2 ? B.m2[r + j0 + q] : 0.0;
+        }
+    };
+    for (int ti = 0; ti < Q.nt; ti++)
+        for (int tj = ti; tj < Q.nt; tj++) {
+            const int i0 = ti * Q.tile, j0 = tj * Q.tile;
+            double acc[4][4] = {};
+            fetch(0, i0, j0);
+            for (int k0 = 0; k0 < n; k0 += kPuK) {
+                __syncthreads();
+#pragma unroll
+                for (int u = 0; u < F; u++)
+                    if (pos[u] >= 0) {
+                        const int kk = pos[u] >> 8, q = pos[u] & 255;
+                        double v = k0 + kk == j0 + q && k0 + kk < n ? B.c0 : 0.0;
+                        if (B.m1) v = fma(B.c1, f1[u], v);
+                        if (B.m2) v = fma(B.c2, f2[u], v);
+                        Q.As[kk][q] = fa[u];
+                        Q.Bs[kk][q] = v;
+                    }
+                for (int e = tid + F * (int)blockDim.x; e < kPuK * Q.tile; e += blockDim.x) {
+                    const int kk = e / Q.tile, q = e % Q.tile, k = k0 + kk;
+                    Q.As[kk][q] = k < n && i0 + q < n ? A[(size_t)k * n + i0 + q] : 0.0;
+                    Q.Bs[kk][q] = k < n && j0 + q < n ? B.at(k, j0 + q, n) : 0.0;
+                }
+                __syncthreads();
+                if (k0 + kPuK < n) fetch(k0 + kPuK, i0, j0);
+                if (!act) continue;
+#pragma unroll
+                for (int kk = 0; kk < kPuK; kk++) {
+                    const double2 a0 = *(const double2 *)&Q.As[kk][cy], a1 = *(const double2 *)&Q.As[kk][cy + 2];
+                    const double2 b0 = *(const double2 *)&Q.Bs[kk][cx], b1 = *(const double2 *)&Q.Bs[kk][cx + 2];
+                    const double a[4] = {a0.x, a0.y, a1.x, a1.y}, b[4] = {b0.x, b0.y, b1.x, b1.y};
+#pragma unroll
+                    for (int p = 0; p < 4; p++)
+#pragma unroll
+                        for (int q = 0; q < 4; q++) acc[p][q] = fma(a[p], b[q], acc[p][q]);
+                }
+            }
+            if (act)
+#pragma unroll
+                for (int p = 0; p < 4; p++)
+#pragma unroll
+                    for (int q = 0; q < 4; q++) {
+                        const int i = i0 + cy + p, j = j0 + cx + q;
+                        if (i >= n || j >= n || i > j) continue;
+                        const double v = acc[p][q] + E.at(i, j, n);
+                        out[(size_t)i * n + j] = v;
+                        out[(size_t)j * n + i] = v;
+                    }
+        }
+    __syncthreads();
+}
+
 // Largest value over the CTA (every thread gets it).
 __device__ double pu_max(double v, double *red) {
     for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -107,8 +185,8 @@ __device__ double pu_max(double v, double *red) {
     return v;
 }
 
-template <typename R>
-__global__ void __launch_bounds__(256) k_propagators(PropJob P, int tx, int nt, typename Vec2<R>::T *U, double *ws) {
+template <typename R, bool AHEAD>
+__global__ void __launch_bounds__(256, 2) k_propagators(PropJob P, int tx, int nt, typename Vec2<R>::T *U, double *ws) {
     typedef typename Vec2<R>::T R2;
     __shared__ __align__(16) double As[kPuK][64], Bs[kPuK][64];
     __shared__ double red[8];
@@ -117,6 +195,7 @@ __global__ void __launch_bounds__(256) k_propagators(PropJob P, int tx, int nt, 
     const PuTile Q = {n, tx, nt, 4 * tx, As, Bs};
     double *A = ws + blockIdx.x * kPuMat * nn, *X = A + nn, *Y = X + nn, *Z = Y + nn, *C = Z + nn, *S = C + nn;
     const Lin zero = {0, 0, 0, nullptr, nullptr};
+    const auto gemm = AHEAD ? pu_gemm_ahead : pu_gemm;
     for (long fr = blockIdx.x; fr < P.nfr; fr += gridDim.x) {
         const long t = P.f0 + fr;
         // H - c, its Gershgorin bound, and the scaling
@@ -150,9 +229,9 @@ __global__ void __launch_bounds__(256) k_propagators(PropJob P, int tx, int nt, 
         const double g = ldexp(P.f, -s);
         for (int e = tid; e < n * n; e += blockDim.x) A[e] *= g;
         __syncthreads();
-        pu_gemm(Q, X, A, {0, 1, 0, A, nullptr}, zero);
-        pu_gemm(Q, Y, X, {0, 1, 0, X, nullptr}, zero);
-        pu_gemm(Q, Z, X, {0, 1, 0, Y, nullptr}, zero);
+        gemm(Q, X, A, {0, 1, 0, A, nullptr}, zero);
+        gemm(Q, Y, X, {0, 1, 0, X, nullptr}, zero);
+        gemm(Q, Z, X, {0, 1, 0, Y, nullptr}, zero);
         // reciprocal factorials with alternating signs: cc[j] = (-1)^j / (2j)!, sc[j] = (-1)^j / (2j+1)!
         double cc[9], sc[9];
         cc[0] = sc[0] = 1;
@@ -163,21 +242,21 @@ __global__ void __launch_bounds__(256) k_propagators(PropJob P, int tx, int nt, 
         }
         double *Sn = r > 0.2 ? S : X, *f1 = Y, *f2 = Z;
         if (r > 0.2) {
-            pu_gemm(Q, S, Z, {cc[6], cc[7], cc[8], X, Y}, {cc[3], cc[4], cc[5], X, Y});
-            pu_gemm(Q, C, Z, {0, 1, 0, S, nullptr}, {cc[0], cc[1], cc[2], X, Y});
-            pu_gemm(Q, S, Z, {sc[6], sc[7], sc[8], X, Y}, {sc[3], sc[4], sc[5], X, Y});
+            gemm(Q, S, Z, {cc[6], cc[7], cc[8], X, Y}, {cc[3], cc[4], cc[5], X, Y});
+            gemm(Q, C, Z, {0, 1, 0, S, nullptr}, {cc[0], cc[1], cc[2], X, Y});
+            gemm(Q, S, Z, {sc[6], sc[7], sc[8], X, Y}, {sc[3], sc[4], sc[5], X, Y});
             // X is only read where it is written, by the same thread
-            pu_gemm(Q, X, Z, {0, 1, 0, S, nullptr}, {sc[0], sc[1], sc[2], X, Y});
-            pu_gemm(Q, Sn, A, {0, 1, 0, X, nullptr}, zero);
+            gemm(Q, X, Z, {0, 1, 0, S, nullptr}, {sc[0], sc[1], sc[2], X, Y});
+            gemm(Q, Sn, A, {0, 1, 0, X, nullptr}, zero);
         } else {
-            pu_gemm(Q, C, Z, {cc[3], cc[4], cc[5], X, Y}, {cc[0], cc[1], cc[2], X, Y});
-            pu_gemm(Q, S, Z, {sc[3], sc[4], sc[5], X, Y}, {sc[0], sc[1], sc[2], X, Y});
-            pu_gemm(Q, Sn, A, {0, 1, 0, S, nullptr}, zero);
+            gemm(Q, C, Z, {cc[3], cc[4], cc[5], X, Y}, {cc[0], cc[1], cc[2], X, Y});
+            gemm(Q, S, Z, {sc[3], sc[4], sc[5], X, Y}, {sc[0], sc[1], sc[2], X, Y});
+            gemm(Q, Sn, A, {0, 1, 0, S, nullptr}, zero);
         }
         double *Cn = C;
         for (int q = 0; q < s; q++) {
-            pu_gemm(Q, f1, Cn, {0, 2, 0, Cn, nullptr}, {-1, 0, 0, nullptr, nullptr});
-            pu_gemm(Q, f2, Sn, {0, 2, 0, Cn, nullptr}, zero);
+            gemm(Q, f1, Cn, {0, 2, 0, Cn, nullptr}, {-1, 0, 0, nullptr, nullptr});
+            gemm(Q, f2, Sn, {0, 2, 0, Cn, nullptr}, zero);
             double *sw = Cn;
             Cn = f1;
             f1 = sw;
@@ -229,7 +308,9 @@ size_t propagator_ws_doubles(int n, long frames) { return (size_t)pu_shape(n, fr
 int launch_propagators(int prec, const PropJob &P, void *U, double *ws, cudaStream_t s) {
     if (P.nfr <= 0) return 0;
     const PuShape q = pu_shape(P.n, P.nfr);
-    if (prec == 0) k_propagators<float><<<q.ctas, q.threads, 0, s>>>(P, q.tx, q.nt, (float2 *)U, ws);
-    else k_propagators<double><<<q.ctas, q.threads, 0, s>>>(P, q.tx, q.nt, (double2 *)U, ws);
+    if (prec == 0)
+        (q.nt > 1 ? k_propagators<float, true> : k_propagators<float, false>)<<<q.ctas, q.threads, 0, s>>>(P, q.tx, q.nt, (float2 *)U, ws);
+    else
+        (q.nt > 1 ? k_propagators<double, true> : k_propagators<double, false>)<<<q.ctas, q.threads, 0, s>>>(P, q.tx, q.nt, (double2 *)U, ws);
     return (int)cudaGetLastError();
 }
