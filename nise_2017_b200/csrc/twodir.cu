@@ -1149,6 +1149,7 @@ __device__ __forceinline__ void pair_couplings(float4 *F, const Dcoef<float> *cf
         }
         for (int k = sg.y; k < sg.z;) {
             if ((k & 31) == 0) {  // the next 32 records arrive, those after them start their way
+                __syncwarp();     // in place of the 32 that a slower lane of pair_free may still read
                 put((k + 32 + lane) & 63);
                 get(k + 64 + lane);
                 __syncwarp();
