@@ -1815,6 +1815,13 @@ static int run_taylor3(const DevTraj &T, const TaylorPlan &P, const AbsJob &J, d
     return run_taylor3_tail<R, IT1>(T, P, J, resp, main, nvec - main, s);
 }
 
+// Whether the row-owner waves and the 1-vector CTAs beside them both fit shared
+// memory.  A neighbour takes 5.3 bytes in the row-owner's slot triples and 8 in
+// the 1-vector kernel's sliced ELL, so either can be the limit.
+bool taylor_rv_runs(const DevTraj &T, const TaylorPlan &P) {
+    return P.ell && P.ell_nslices <= 16 * 32 && taylor3_smem(P, 4, 1) <= kMaxSmem && taylor_rv_fits(T, P);
+}
+
 int launch_abs_taylor_part(const DevTraj &T, const TaylorPlan &P, const AbsJob &J, double2 *resp, int v0, int nvec,
                            bool one, cudaStream_t s) {
     if (nvec <= 0) return 0;
@@ -1849,9 +1856,8 @@ int launch_abs_taylor(int prec, const DevTraj &T, const TaylorPlan &P, const Abs
         }
     }
     if (P.cheb_coef && P.rv_cheb) {  // the row-owner kernel with the Chebyshev expansion (FP32)
-        if (prec != 0 || !P.ell || !taylor_rv_fits(T, P)) return (int)cudaErrorNotSupported;
+        if (prec != 0 || !taylor_rv_runs(T, P)) return (int)cudaErrorNotSupported;
         const int it = (P.ell_nslices + 15) / 16;
-        if (it > 32 || taylor3_smem(P, 4) > 220 * 1024) return (int)cudaErrorNotSupported;
         const int nvec = 3 * J.nsamp;
         switch (it <= 1 ? 1 : it <= 2 ? 2 : it <= 4 ? 4 : it <= 8 ? 8 : it <= 16 ? 16 : 32) {
         case 1: return run_taylor3<float, 1>(T, P, J, resp, nvec, s, kernels);

@@ -966,7 +966,7 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
         }
     }
     config = default_config(scheme, N, plain, cheb, TP.k, nchk, plain ? 3 : nvec, dell4.p != nullptr,
-                            scheme == SCHEME_TAYLOR && taylor_rv_fits(T, XP),
+                            scheme == SCHEME_TAYLOR && taylor_rv_runs(T, XP),
                             scheme == SCHEME_TROTTER && TP.rot_static,
                             scheme == SCHEME_TROTTER ? rows_of(TP) : RowCounts{{0, 0}}, (long)p.ts * (TP.k + 2L * N));
     if (p.kernel_config != 0) {  // forced by the caller
@@ -1144,7 +1144,7 @@ int AbsRun::tune() {
 // Kernels of the job on stream s: tables, propagation, response sum.
 bool AbsRun::waves_apply() const {
     return c->nchunks > 0 && scheme == SCHEME_TAYLOR && !plain && (config == 15 || config == 8) &&
-           prec == NISE_FP32 && taylor_rv_fits(T, XP) && nvec > sm_count();
+           prec == NISE_FP32 && taylor_rv_runs(T, XP) && nvec > sm_count();
 }
 
 int AbsRun::enqueue_waves(cudaStream_t s) {

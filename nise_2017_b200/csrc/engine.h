@@ -151,6 +151,8 @@ int launch_prep_taylor(int prec, const DevTraj &T, TaylorPlan &P, double rowabs_
 int launch_abs_taylor_rv(const DevTraj &T, const TaylorPlan &P, const AbsJob &J, double2 *resp, int v0, int nvec,
                          cudaStream_t s);
 bool taylor_rv_fits(const DevTraj &T, const TaylorPlan &P);
+// The same for a job: its last vectors on 1-vector CTAs fit too.
+bool taylor_rv_runs(const DevTraj &T, const TaylorPlan &P);
 // Vectors [v0, v0 + nvec) of an FP32 static-coupling job: on the row-owner
 // kernel (whole CTAs of 8), or on 1-vector CTAs of the sliced-ELL Taylor
 // kernel (one).
