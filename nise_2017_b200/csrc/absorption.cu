@@ -1883,7 +1883,9 @@ int launch_abs_taylor(int prec, const DevTraj &T, const TaylorPlan &P, const Abs
         default: return run_cheb3<32>(T, P, J, resp, nvec, s);
         }
     }
-    if (!P.only_v2 && P.static_j && P.ell && vec_per_cta > 4 && taylor3_smem(P, prec == 0 ? 4 : 8) <= 220 * 1024) {
+    // (the row-owner waves and the 1-vector CTAs need no 8-vector tables)
+    if (!P.only_v2 && P.static_j && P.ell && vec_per_cta > 4 &&
+        (taylor3_smem(P, prec == 0 ? 4 : 8) <= 220 * 1024 || (prec == 0 && !P.no_rv && taylor_rv_runs(T, P)))) {
         int nvec = 3 * J.nsamp;
         int it = (P.ell_nslices + 15) / 16;  // 16 warps, one slice (4 rows) per warp instruction
         int IT = it <= 1 ? 1 : it <= 2 ? 2 : it <= 4 ? 4 : it <= 8 ? 8 : it <= 16 ? 16 : 32;

@@ -91,16 +91,17 @@ int default_config(int scheme, int N, bool plain, bool cheb, int K, int nchk, in
     // one start point per launch (3 vectors): the sliced-ELL kernel, which
     // gives every vector its own CTA when there are fewer vectors than SMs
     if (plain) return 8;
-    (void)cheb;           // the Chebyshev kernel is a tuned alternative: fewer terms, more work per term
-    // less than one wave of 8-vector CTAs: 4 vectors per CTA reach twice the
-    // SMs.  Up to 1024 sites the FP32 sliced-ELL kernel with 4 vectors (285
-    // vectors, 229 sites: 1.23 ms against 1.59 for k_abs_taylor2 and 1.36 for
-    // the row-owner kernel), but from 300 sites on the row-owner kernel with
-    // the Chebyshev expansion, whose gathers are conflict-free, makes up for the
-    // idle SMs (285 vectors, 600 sites: 2.79 against 4.13 ms; 1024 sites, 585
-    // vectors: 4.67 against 6.56); above 1024 sites k_abs_taylor2 with 4 (1440
-    // sites, 585 vectors: 12.1 against 15.8 and 25.0)
-    if (nvec < 8 * sm_count() && !(rv && cheb && N >= 300)) return has4 && N <= 1024 ? 12 : 3;
+    // less than one wave of 8-vector CTAs: from 300 sites on the row-owner kernel,
+    // whose gathers are conflict-free, in spite of idle SMs (300 vectors, 300 sites:
+    // 1.70 ms against 1.86 on the FP32 sliced-ELL kernel with 4 vectors per CTA; 600
+    // sites 2.77 against 4.05; 585 vectors, 1024 sites 4.77 against 6.77), with the
+    // Taylor series of that kernel: the Chebyshev expansion takes 1.61, 2.57 and
+    // 4.15 ms, but its recurrence rounds more (4e-8 of the response against 8e-9 for
+    // either Taylor kernel).  Below, 4 vectors per CTA reach twice the SMs (285
+    // vectors, 229 sites: 1.23 ms against 1.59 for k_abs_taylor2 and 1.36 for the
+    // row-owner kernel); above 1024 sites k_abs_taylor2 with 4 (1440 sites, 585
+    // vectors: 12.1 against 15.8 and 25.0)
+    if (nvec < 8 * sm_count()) return rv && N >= 300 ? 8 : has4 && N <= 1024 ? 12 : 3;
     // whole waves of 8-vector CTAs: the row-owner kernel with the Chebyshev
     // expansion (FP32 lattices up to 1024 sites; on the 1024-site lattice,
     // 100 000 frames: 52.0 ms against 55.8 with the Taylor series and 69.7 on
