@@ -11,11 +11,15 @@
 // SIAM J. Comput. 2 (1973) 60): 5 terms and 6 products while the Gershgorin
 // bound of ||A|| is below 0.2 (remainder 0.2^12 / 12! = 9e-18), else 8 terms and
 // 8 products up to 0.8 (0.8^18 / 18! = 3e-18), the power of two s bringing
-// larger ones there; s doublings cos 2A = 2 cos^2 A - 1, sin 2A = 2 sin A cos A
-// follow, and the phase exp(-i c f).  The doublings amplify rounding like 2^s,
-// as an eigenvalue's rounding grows with ||H f||.  U is rounded to the working
-// precision and truncated by the reference's test, so it equals the
-// eigenvector form to FP64 rounding.
+// larger ones there; s doublings follow, and the phase exp(-i c f).  They double
+// D = cos A - 1, D <- -2 S^2 and S <- 2 S + 2 S D: with cos itself an eigenvalue
+// near c, where cos is near 1, has its error multiplied by 4 in every doubling, so
+// that U U^H strays from 1 (80 sites and two 1500 cm^-1 away: 1e-13 after 4
+// doublings, 2e-11 after 10; now 1e-15 and 5e-15, eigenvectors 3e-15).  What
+// remains is the rounding of an eigenvalue, eps ||H f||, as with eigenvectors: the
+// error of U against 64-bit mantissas is 1e-16 to 2e-15 up to 4 doublings
+// (eigenvectors 1e-15 to 3e-15) and within 3 times the eigenvectors' beyond.  U is
+// rounded to the working precision and truncated by the reference's test.
 //
 // One CTA per frame, frames dealt to as many CTAs as fit the SMs; the six
 // matrices of a frame are in a workspace per CTA that stays in L2.  All of them
@@ -243,20 +247,20 @@ __global__ void __launch_bounds__(256, 2) k_propagators(PropJob P, int tx, int n
         double *Sn = r > 0.2 ? S : X, *f1 = Y, *f2 = Z;
         if (r > 0.2) {
             gemm(Q, S, Z, {cc[6], cc[7], cc[8], X, Y}, {cc[3], cc[4], cc[5], X, Y});
-            gemm(Q, C, Z, {0, 1, 0, S, nullptr}, {cc[0], cc[1], cc[2], X, Y});
+            gemm(Q, C, Z, {0, 1, 0, S, nullptr}, {0, cc[1], cc[2], X, Y});
             gemm(Q, S, Z, {sc[6], sc[7], sc[8], X, Y}, {sc[3], sc[4], sc[5], X, Y});
             // X is only read where it is written, by the same thread
             gemm(Q, X, Z, {0, 1, 0, S, nullptr}, {sc[0], sc[1], sc[2], X, Y});
             gemm(Q, Sn, A, {0, 1, 0, X, nullptr}, zero);
         } else {
-            gemm(Q, C, Z, {cc[3], cc[4], cc[5], X, Y}, {cc[0], cc[1], cc[2], X, Y});
+            gemm(Q, C, Z, {cc[3], cc[4], cc[5], X, Y}, {0, cc[1], cc[2], X, Y});
             gemm(Q, S, Z, {sc[3], sc[4], sc[5], X, Y}, {sc[0], sc[1], sc[2], X, Y});
             gemm(Q, Sn, A, {0, 1, 0, S, nullptr}, zero);
         }
-        double *Cn = C;
+        double *Cn = C;  // cos A - 1
         for (int q = 0; q < s; q++) {
-            gemm(Q, f1, Cn, {0, 2, 0, Cn, nullptr}, {-1, 0, 0, nullptr, nullptr});
-            gemm(Q, f2, Sn, {0, 2, 0, Cn, nullptr}, zero);
+            gemm(Q, f1, Sn, {0, -2, 0, Sn, nullptr}, zero);
+            gemm(Q, f2, Sn, {0, 2, 0, Cn, nullptr}, {0, 2, 0, Sn, nullptr});
             double *sw = Cn;
             Cn = f1;
             f1 = sw;
@@ -268,7 +272,7 @@ __global__ void __launch_bounds__(256, 2) k_propagators(PropJob P, int tx, int n
         sincos(c * P.f, &sp, &cp);
         R2 *Uf = U + (size_t)fr * nn;
         for (int e = tid; e < n * n; e += blockDim.x) {
-            const double co = Cn[e], si = Sn[e];
+            const double co = Cn[e] + (e % (n + 1) == 0 ? 1.0 : 0.0), si = Sn[e];  // the diagonal: every n + 1
             R2 z;
             z.x = (R)(cp * co - sp * si);
             z.y = (R)(-(sp * co + cp * si));
