@@ -388,7 +388,9 @@ struct AbsRun {
         if (estatus.p) {
             if (cudaMemcpy(&h, estatus.p, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess)
                 return nise_fail(c, NISE_ERR_DEVICE, "eigensolver status read failed");
-            if (h) return nise_fail(c, NISE_ERR_DEVICE, "the eigensolver did not converge on a frame");
+            if (h)
+                return nise_fail(c, NISE_ERR_DEVICE,
+                                 diagonalise ? "the eigensolver did not converge on a frame" : NISE_NOT_FINITE);
         }
         return NISE_OK;
     }
@@ -595,13 +597,14 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
             if ((rc = Ue.alloc(c, ubytes))) return rc;
             if (!diagonalise) {
                 if ((rc = eA.alloc(c, propagator_ws_doubles(N, FC)))) return rc;
+                if (propagators_report(N) && (rc = estatus.alloc(c, 1))) return rc;
             } else {
                 if ((rc = efr.upload(c, frames)) || (rc = eV.alloc(c, (size_t)FC * N * N)) ||
                     (rc = ew.alloc(c, (size_t)FC * N)) || (rc = eA.alloc(c, eig_any_ws_doubles(N, FC))) ||
                     (rc = estatus.alloc(c, 1)))
                     return rc;
-                cudaMemsetAsync(estatus.p, 0, sizeof(int), c->stream);
             }
+            if (estatus.p) cudaMemsetAsync(estatus.p, 0, sizeof(int), c->stream);
             // propagate_vec_DIA: f = deltat*icm2ifs*twoPi*sign in float, one full step
             fe = prec == NISE_FP32 ? (double)J.f32_full : J.f;
             const size_t cols = tc_starts ? (size_t)16 * nsamp : (size_t)tc_dia_columns(Jt);
@@ -1005,6 +1008,7 @@ int AbsRun::build_u(long q, long m, void *dst, cudaStream_t s) {
         PJ.nfr = m;
         PJ.f = fe;
         PJ.thres = c->thres;
+        PJ.status = estatus.p;
         return launch_propagators(pr, PJ, dst, eA.p, s);
     }
     EigJob EJ;

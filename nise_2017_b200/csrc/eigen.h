@@ -35,13 +35,18 @@ int launch_build_u_any(int prec, const double *V, const double *w, long nfr, int
 // exp(-i H f) of the frames [f0, f0 + nfr) without eigenvectors
 // (propagators.cu), any n: U[t][a][c] in working precision (prec 0 FP32, 1
 // FP64), exactly symmetric, |U|^2 <= thres dropped when truncate; ws holds
-// propagator_ws_doubles(n, nfr) doubles.
+// propagator_ws_doubles(n, nfr) doubles.  *status (where not null) is set to 1 if
+// a frame has a NaN or an infinity.
 struct PropJob {
     DevTraj T;
     int n, singleshift, truncate;
     long f0, nfr;
     double f;
     float thres;
+    int *status;
 };
+// Whether a job's propagators report such frames: above the size of the Jacobi,
+// where the diagonalisation ended in an error; below, it passed them on.
+inline bool propagators_report(int n) { return n > NISE_EIG_MAX_N; }
 size_t propagator_ws_doubles(int n, long frames);
 int launch_propagators(int prec, const PropJob &P, void *U, double *ws, cudaStream_t s);

@@ -60,6 +60,7 @@ struct nise_ctx {
 void nise_wait_frames(nise_ctx *c, cudaStream_t s, long last_frame);
 void nise_wait_all_frames(nise_ctx *c, cudaStream_t s);
 
+#define NISE_NOT_FINITE "a frame of the Hamiltonian has a NaN or an infinity"
 int nise_fail(nise_ctx *c, int code, const char *fmt, ...);
 int nise_cuda(nise_ctx *c, int e, const char *what);
 float nise_f32(const nise_params &p, int sign, int m);

@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(256, 2) k_propagators(PropJob P, int tx, int n
         for (int a = tid; a < n; a += blockDim.x) {
             double s = 0;
             for (int b = 0; b < n; b++) s += fabs(A[(size_t)b * n + a]);
+            if (P.status && !(s < HUGE_VAL)) *P.status = 1;  // (fmax passes over a NaN)
             r = fmax(r, s);
         }
         r = pu_max(r, red) * fabs(P.f);

@@ -85,6 +85,11 @@ int nise_singles_tables(nise_ctx *c, const DevTraj &T, long fmin, long nf, int s
         const float thr = p.propagation == NISE_PROP_DIAGONAL ? 0.0f : c->thres;
         const bool trunc_singles = thr != 0 && !(thr > 1);
         DevBuf<double> ws;
+        DevBuf<int> status;
+        if (propagators_report(N)) {
+            if ((rc = status.alloc(c, 1))) return rc;
+            cudaMemsetAsync(status.p, 0, sizeof(int), c->stream);
+        }
         if ((rc = ws.alloc(c, propagator_ws_doubles(N, nf))) || (rc = B.U.alloc(c, r2 * (size_t)nf * N * N))) return rc;
         if (doubles_u && (rc = B.rot.alloc(c, r2 * (size_t)nf * N * N))) return rc;
         const int pr = prec == NISE_FP32 ? 0 : 1;
@@ -95,6 +100,7 @@ int nise_singles_tables(nise_ctx *c, const DevTraj &T, long fmin, long nf, int s
         PJ.f0 = fmin;
         PJ.nfr = nf;
         PJ.thres = thr;
+        PJ.status = status.p;
         PJ.truncate = trunc_singles;
         PJ.f = prec == NISE_FP32 ? (double)nise_f32(p, 1, 1) : nise_f64(p, 1, 1);
         if ((rc = nise_cuda(c, launch_propagators(pr, PJ, B.U.p, ws.p, c->stream), "propagator build"))) return rc;
@@ -105,6 +111,14 @@ int nise_singles_tables(nise_ctx *c, const DevTraj &T, long fmin, long nf, int s
             if ((rc = nise_cuda(c, launch_propagators(pr, PJ, B.rot.p, ws.p, c->stream), "doubles propagator build")))
                 return rc;
             c->launches++;
+        }
+        if (status.p) {
+            int bad = 0;
+            if ((rc = nise_cuda(c, (int)cudaMemcpyAsync(&bad, status.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream),
+                                "propagator status")) ||
+                (rc = nise_cuda(c, (int)cudaStreamSynchronize(c->stream), "propagators")))
+                return rc;
+            if (bad) return nise_fail(c, NISE_ERR_DEVICE, NISE_NOT_FINITE);
         }
         S.Ud = B.U.p;
         if (doubles_u) B.Us = B.rot.p;
