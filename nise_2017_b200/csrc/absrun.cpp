@@ -332,6 +332,8 @@ struct AbsRun {
     DevBuf<long> efr;
     DevBuf<double> eV, ew, eA;  // eigenvectors, eigenvalues; workspace of the QR or of the propagators
     bool diagonalise = false;   // kernel_config 2: eigenvectors of every frame
+    double *ws = nullptr;       // the propagators' workspace: eA, or wider while a call runs
+    int ws_ctas = 0;
     // propagators of the frames f0 + [q, q + m) to dst; returns a CUDA error
     int build_u(long q, long m, void *dst, cudaStream_t s);
     DevBuf<int> estatus;
@@ -356,6 +358,7 @@ struct AbsRun {
     }
     int plan(nise_ctx *ctx, bool autotune);
     int enqueue(cudaStream_t s, bool events);
+    int enqueue_job(cudaStream_t s, bool events);
     // The static-coupling series kernels wave by wave, each wave after the
     // energy chunk holding its last frame (and the series tables of the
     // frames up to there): the copy from the host overlaps the propagation.
@@ -596,7 +599,9 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
             for (long t = 0; t < nf; t++) frames[t] = f0 + t;
             if ((rc = Ue.alloc(c, ubytes))) return rc;
             if (!diagonalise) {
-                if ((rc = eA.alloc(c, propagator_ws_doubles(N, FC)))) return rc;
+                ws_ctas = propagator_ctas(N, FC, propagator_held(N));
+                if ((rc = eA.alloc(c, ws_ctas * propagator_ws_doubles(N)))) return rc;
+                ws = eA.p;
                 if (propagators_report(N) && (rc = estatus.alloc(c, 1))) return rc;
             } else {
                 if ((rc = efr.upload(c, frames)) || (rc = eV.alloc(c, (size_t)FC * N * N)) ||
@@ -1009,7 +1014,7 @@ int AbsRun::build_u(long q, long m, void *dst, cudaStream_t s) {
         PJ.f = fe;
         PJ.thres = c->thres;
         PJ.status = estatus.p;
-        return launch_propagators(pr, PJ, dst, eA.p, s);
+        return launch_propagators(pr, PJ, dst, ws, ws_ctas, s);
     }
     EigJob EJ;
     EJ.T = T;
@@ -1223,6 +1228,25 @@ int AbsRun::enqueue_waves(cudaStream_t s) {
 }
 
 int AbsRun::enqueue(cudaStream_t s, bool events) {
+    int rc;
+    // a call by itself (a batch's graph is captured on other streams) builds its
+    // propagators at full width where the device has the memory
+    DevBuf<double> wide;
+    const int held_ctas = ws_ctas;
+    if (scheme == SCHEME_EIGEN && !diagonalise && s == c->stream) {
+        const int want = propagator_ctas(N, FC, kPropagatorRoom);
+        if (want > held_ctas && wide.try_alloc(c, want * propagator_ws_doubles(N))) {
+            ws = wide.p;
+            ws_ctas = want;
+        }
+    }
+    rc = enqueue_job(s, events);
+    ws = eA.p;
+    ws_ctas = held_ctas;
+    return rc;
+}
+
+int AbsRun::enqueue_job(cudaStream_t s, bool events) {
     const int pr = prec == NISE_FP32 ? 0 : 1;
     int rc;
     const bool waves = waves_apply();

@@ -1,6 +1,9 @@
 // Batched FP64 eigendecomposition of per-frame Hamiltonians (eigen.cu).
 #pragma once
 #include <cuda_runtime.h>
+#include <stddef.h>
+
+#include <algorithm>
 
 #include "devtypes.h"
 
@@ -35,8 +38,9 @@ int launch_build_u_any(int prec, const double *V, const double *w, long nfr, int
 // exp(-i H f) of the frames [f0, f0 + nfr) without eigenvectors
 // (propagators.cu), any n: U[t][a][c] in working precision (prec 0 FP32, 1
 // FP64), exactly symmetric, |U|^2 <= thres dropped when truncate; ws holds
-// propagator_ws_doubles(n, nfr) doubles.  *status (where not null) is set to 1 if
-// a frame has a NaN or an infinity.
+// propagator_ws_doubles(n) doubles for each of `ctas` CTAs (the results do not
+// depend on their number).  *status (where not null) is set to 1 if a frame has a
+// NaN or an infinity.
 struct PropJob {
     DevTraj T;
     int n, singleshift, truncate;
@@ -48,5 +52,13 @@ struct PropJob {
 // Whether a job's propagators report such frames: above the size of the Jacobi,
 // where the diagonalisation ended in an error; below, it passed them on.
 inline bool propagators_report(int n) { return n > NISE_EIG_MAX_N; }
-size_t propagator_ws_doubles(int n, long frames);
-int launch_propagators(int prec, const PropJob &P, void *U, double *ws, cudaStream_t s);
+// CTAs for a job of that many frames whose workspaces take at most `room` bytes.
+int propagator_ctas(int n, long frames, size_t room);
+size_t propagator_ws_doubles(int n);
+int launch_propagators(int prec, const PropJob &P, void *U, double *ws, int ctas, cudaStream_t s);
+// The room a plan may hold, next to those of other jobs: what the eigenvectors
+// and the QR workspace of 148 frames take, or 1 GB (up to 274 sites every SM has its
+// CTAs, from 674 on 49 run); and what one call may take while it runs, if the device
+// has it (300 frames of 512 sites, whole job: 30 ms against 60 in the held room).
+inline size_t propagator_held(int n) { return std::max((size_t)1 << 30, (size_t)148 * 16 * n * n); }
+const size_t kPropagatorRoom = (size_t)16 << 30;

@@ -92,6 +92,14 @@ template <typename T> struct DevBuf {
         }
         return NISE_OK;
     }
+    // whether the device had it (no error otherwise)
+    bool try_alloc(nise_ctx *c, size_t count) {
+        s = c->stream;
+        if (cudaMallocAsync((void **)&p, sizeof(T) * count, s) == cudaSuccess) return true;
+        p = nullptr;
+        cudaGetLastError();
+        return false;
+    }
     int upload(nise_ctx *c, const std::vector<T> &h) {
         int rc = alloc(c, h.size());
         if (rc) return rc;

@@ -22,12 +22,13 @@
 // rounded to the working precision and truncated by the reference's test.
 //
 // One CTA per frame, frames dealt to as many CTAs as fit the SMs; the six
-// matrices of a frame are in a workspace per CTA that stays in L2.  All of them
+// matrices of a frame are in a workspace per CTA, which stays in L2 up to about 90
+// sites (three CTAs per SM at 48 sites: 49 MB; two at 200: 570 MB).  All of them
 // are polynomials in H, hence symmetric: only tiles on and above the diagonal
 // are computed, the others mirrored, and both operands of a product are read
 // along rows.  A thread holds 4 x 4 results; the tile is N / ceil(N / 64)
-// rounded up to 4, so little of it is padding.  Bound by operand loads (L2, then
-// shared memory: 8 values for 16 multiply-adds) with two CTAs per SM to hide them: 48
+// rounded up to 4, so little of it is padding.  Bound by operand loads (L2 or
+// device memory, then shared memory: 8 values for 16 multiply-adds) with two CTAs per SM to hide them: 48
 // sites, 1987 frames 0.50 ms (Jacobi 4.8 ms); 200 sites, 595 frames 8.1 ms
 // (Householder and QR 69.3 ms, then 1.4 ms for U).
 #include <algorithm>
@@ -292,30 +293,34 @@ __global__ void __launch_bounds__(256, 2) k_propagators(PropJob P, int tx, int n
 }
 
 struct PuShape {
-    int tx, nt, threads, ctas;
+    int tx, nt, threads;
 };
-PuShape pu_shape(int n, long frames) {
+PuShape pu_shape(int n) {
     PuShape s;
     s.nt = (n + 63) / 64;
     s.tx = (n + 4 * s.nt - 1) / (4 * s.nt);
     s.threads = (s.tx * s.tx + 31) / 32 * 32;
-    // resident CTAs: by threads (128 registers each), and at most 16 GB of workspace
-    const long per_sm = std::max(1, std::min(8, 512 / s.threads));
-    const size_t per = sizeof(double) * kPuMat * (size_t)n * n;
-    s.ctas = (int)std::max(1L, std::min(std::min(frames, per_sm * sm_count()), (long)(((size_t)16 << 30) / per)));
     return s;
 }
 
 }  // namespace
 
-size_t propagator_ws_doubles(int n, long frames) { return (size_t)pu_shape(n, frames).ctas * kPuMat * n * n; }
+// Resident CTAs by threads (128 registers each), and by the room for their
+// workspaces.
+int propagator_ctas(int n, long frames, size_t room) {
+    const long per_sm = std::max(1, std::min(8, 512 / pu_shape(n).threads));
+    return (int)std::max(1L, std::min(std::min(frames, per_sm * sm_count()), (long)(room / (sizeof(double) * propagator_ws_doubles(n)))));
+}
 
-int launch_propagators(int prec, const PropJob &P, void *U, double *ws, cudaStream_t s) {
+size_t propagator_ws_doubles(int n) { return kPuMat * (size_t)n * n; }
+
+int launch_propagators(int prec, const PropJob &P, void *U, double *ws, int ctas, cudaStream_t s) {
     if (P.nfr <= 0) return 0;
-    const PuShape q = pu_shape(P.n, P.nfr);
+    const PuShape q = pu_shape(P.n);
+    ctas = (int)std::min<long>(ctas, P.nfr);
     if (prec == 0)
-        (q.nt > 1 ? k_propagators<float, true> : k_propagators<float, false>)<<<q.ctas, q.threads, 0, s>>>(P, q.tx, q.nt, (float2 *)U, ws);
+        (q.nt > 1 ? k_propagators<float, true> : k_propagators<float, false>)<<<ctas, q.threads, 0, s>>>(P, q.tx, q.nt, (float2 *)U, ws);
     else
-        (q.nt > 1 ? k_propagators<double, true> : k_propagators<double, false>)<<<q.ctas, q.threads, 0, s>>>(P, q.tx, q.nt, (double2 *)U, ws);
+        (q.nt > 1 ? k_propagators<double, true> : k_propagators<double, false>)<<<ctas, q.threads, 0, s>>>(P, q.tx, q.nt, (double2 *)U, ws);
     return (int)cudaGetLastError();
 }

@@ -90,8 +90,13 @@ int nise_singles_tables(nise_ctx *c, const DevTraj &T, long fmin, long nf, int s
             if ((rc = status.alloc(c, 1))) return rc;
             cudaMemsetAsync(status.p, 0, sizeof(int), c->stream);
         }
-        if ((rc = ws.alloc(c, propagator_ws_doubles(N, nf))) || (rc = B.U.alloc(c, r2 * (size_t)nf * N * N))) return rc;
+        if ((rc = B.U.alloc(c, r2 * (size_t)nf * N * N))) return rc;
         if (doubles_u && (rc = B.rot.alloc(c, r2 * (size_t)nf * N * N))) return rc;
+        int ctas = propagator_ctas(N, nf, kPropagatorRoom);
+        if (!ws.try_alloc(c, ctas * propagator_ws_doubles(N))) {
+            ctas = propagator_ctas(N, nf, propagator_held(N));
+            if ((rc = ws.alloc(c, ctas * propagator_ws_doubles(N)))) return rc;
+        }
         const int pr = prec == NISE_FP32 ? 0 : 1;
         PropJob PJ;
         PJ.T = T;
@@ -103,12 +108,12 @@ int nise_singles_tables(nise_ctx *c, const DevTraj &T, long fmin, long nf, int s
         PJ.status = status.p;
         PJ.truncate = trunc_singles;
         PJ.f = prec == NISE_FP32 ? (double)nise_f32(p, 1, 1) : nise_f64(p, 1, 1);
-        if ((rc = nise_cuda(c, launch_propagators(pr, PJ, B.U.p, ws.p, c->stream), "propagator build"))) return rc;
+        if ((rc = nise_cuda(c, launch_propagators(pr, PJ, B.U.p, ws.p, ctas, c->stream), "propagator build"))) return rc;
         c->launches++;
         if (doubles_u) {
             PJ.truncate = 1;
             PJ.f = prec == NISE_FP32 ? (double)nise_f32(p, 1, p.ts) : nise_f64(p, 1, p.ts);
-            if ((rc = nise_cuda(c, launch_propagators(pr, PJ, B.rot.p, ws.p, c->stream), "doubles propagator build")))
+            if ((rc = nise_cuda(c, launch_propagators(pr, PJ, B.rot.p, ws.p, ctas, c->stream), "doubles propagator build")))
                 return rc;
             c->launches++;
         }
