@@ -1073,7 +1073,7 @@ int AbsRun::run_main(cudaStream_t s, int cfg, double2 *dst) {
                     // the last chunk runs on to the last response frame, which needs no propagator
                     const long tb = q + m >= nf ? tc_dia_last_frame(Js) : f0 + q + m - 1;
                     er = launch_abs_dia_tc_frames(T, Ue.p, f0 + q, N, Js, r, tcX.p, derr.p, f0 + q, tb, s);
-                    kernels += 2;
+                    kernels += diagonalise ? 2 : 1;
                 }
                 return er;
             }
@@ -1286,7 +1286,7 @@ int AbsRun::enqueue_job(cudaStream_t s, bool events) {
         for (long q = 0; q < nf && !stream_u; q += FC) {  // streamed: built inside the propagation
             long m = std::min(FC, nf - q);
             if ((rc = nise_cuda(c, build_u(q, m, Ue.p + r2 * (size_t)q * N * N, s), "propagator build"))) return rc;
-            c->launches += 2;
+            c->launches += diagonalise ? 2 : 1;
         }
     }
     }
