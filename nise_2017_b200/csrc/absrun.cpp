@@ -45,6 +45,7 @@ enum Scheme { SCHEME_TROTTER, SCHEME_RK4, SCHEME_TAYLOR, SCHEME_EIGEN };
 //            sliced-ELL kernel with 4 vectors per CTA (k_abs_taylor4).
 typedef std::tuple<int, int, int, int, int> TuneKey;  // scheme, precision, sites, couplings, static
 std::map<TuneKey, int> g_tuned;
+const int NOT_TUNED = -1000;
 std::mutex g_tune_mu;
 
 struct RowCounts {
@@ -349,12 +350,17 @@ struct AbsRun {
     long vec_steps = 0;
     double alg_bytes = 0;  // every frame read once (diagonal or full record) and the dipoles
 
-    // the tuned configuration of this job's key, else `otherwise`
-    int tuned(const TrotterPlan &P, int otherwise = 0) const {
+    // the tuned configuration of this job's key (NOT_TUNED: none), read once per
+    // plan, as another context's tuner may enter one meanwhile: the layouts are
+    // built for the configuration that runs
+    int tuned = NOT_TUNED;
+    void read_tuned() {
         std::lock_guard<std::mutex> lk(g_tune_mu);
-        const auto it = g_tuned.find(TuneKey(scheme, prec, N, scheme == SCHEME_TROTTER ? P.k : 0,
-                                             scheme == SCHEME_TROTTER ? P.rot_static : 0));
-        return it != g_tuned.end() ? it->second : otherwise;
+        const auto it = g_tuned.find(tune_key());
+        if (it != g_tuned.end()) tuned = it->second;
+    }
+    TuneKey tune_key() const {
+        return TuneKey(scheme, prec, N, scheme == SCHEME_TROTTER ? TP.k : 0, scheme == SCHEME_TROTTER ? TP.rot_static : 0);
     }
     int plan(nise_ctx *ctx, bool autotune);
     int enqueue(cudaStream_t s, bool events);
@@ -458,6 +464,7 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
         TP.nf = nf;
         TP.rot_static = p.hamiltonian == NISE_HAM_COUPLING;
         TP.singleshift = c->nshift > 0;
+        read_tuned();
         // the pairs (and so the rotation tables) in level order
         std::vector<int> hperm, hlv;
         rotation_levels(pairs, N, hperm, hlv);
@@ -618,6 +625,7 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
             if (use_tc) cudaMemsetAsync(derr.p, 0, sizeof(int), c->stream);
         } else {
             scheme = SCHEME_TAYLOR;
+            read_tuned();
             // CSR of the static couplings (read cut applied, |J| >= cut kept)
             std::vector<int> rp(N + 1, 0), col;
             std::vector<double> vd;
@@ -790,7 +798,7 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
             }
             // (where its kernel may run: not for the sizes and vectors that
             // default_config gives to the 4-vector kernels)
-            const bool any = autotune || p.kernel_config != 0 || tuned(TP);
+            const bool any = autotune || p.kernel_config != 0 || tuned != NOT_TUNED;
             if (prec == NISE_FP32 && N <= 1024 && (any || plain || nvec >= 8 * sm_count() || N >= 300)) {
                 // Row-owner layout: 8-row slices whose rows alternate in parity, so
                 // that the two rows of a quarter-warp are of different parity, and
@@ -992,7 +1000,8 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
         else return nise_fail(c, NISE_ERR_ARG, "kernel_config %d does not apply to this scheme", k);
         return NISE_OK;
     }
-    config = tuned(TP, config);
+    // (a job of the same size with more couplings may not fit the row-owner kernel)
+    if (tuned != NOT_TUNED && !(scheme == SCHEME_TAYLOR && tuned == 15 && !taylor_rv_runs(T, XP))) config = tuned;
     if (autotune && (scheme == SCHEME_TROTTER || scheme == SCHEME_TAYLOR) && !plain)
         if ((rc = tune())) return rc;
     return NISE_OK;
@@ -1146,8 +1155,7 @@ int AbsRun::tune() {
     cudaEventDestroy(b);
     config = best_cfg;
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tuned[TuneKey(scheme, prec, N, scheme == SCHEME_TROTTER ? TP.k : 0,
-                    scheme == SCHEME_TROTTER ? TP.rot_static : 0)] = best_cfg;
+    g_tuned[tune_key()] = best_cfg;
     return nise_cuda(c, (int)cudaStreamSynchronize(c->stream), "autotuner");
 }
 
