@@ -350,6 +350,11 @@ int nise_backward_absorption(nise_ctx *ctx, const double *site_shift, double cou
  * sites, so neither changes the float operations.  Touches no GPU. */
 int nise_rotation_schedule(const int *ab, int k, int n, int *perm, int *lvptr, int *nlev, int *chkptr, int *nchk,
                            int *flip);
+/* Host-only: whether a job's rotations are put into that order within the chunks
+ * (1) or left in level order (0): its kernel_config, the autotuner's choice
+ * for it if there is one, the rows of operations that are its default (35, 36;
+ * 0: another kernel), and whether it is being tuned. */
+int nise_trotter_needs_bank_order(int kernel_config, int is_tuned, int tuned, int default_rows, int autotune);
 
 /* No counterpart in the reference.  Linear absorption with the Trotter
  * "Coupling" scheme (HamiltonianType Full) for callers whose device memory is

@@ -73,6 +73,16 @@ int default_rows(int N, bool rot_static, int nvec, RowCounts rows, long ops) {
     return rows.n[1] && rot_static && 4 * rows.n[1] < 3 * rows.n[0] ? 36 : 35;
 }
 
+// Whether a Trotter job's rotations need the warp kernels' bank order, which costs
+// the host more than the levels: not where rows run, that is where they were asked
+// for or tuned, or are the default (default_rows' value) of an untuned job; the
+// tuner times both.
+bool needs_bank_order(int kernel_config, int tuned, int default_rows, bool autotune) {
+    auto on_rows = [](int cfg) { return cfg == 35 || cfg == 36; };
+    if (kernel_config != 0) return !on_rows(kernel_config);
+    return autotune || !on_rows(tuned != NOT_TUNED ? tuned : default_rows);
+}
+
 // Trotter: the warp-per-vector kernel where the levels are wide (lattices:
 // ~20 rotations per level) or the job has too few vectors to fill warps of
 // threads (a warp per vector then has the shorter critical path); thread per
@@ -281,6 +291,10 @@ extern "C" int nise_rotation_schedule(const int *ab, int k, int n, int *perm, in
     *nlev = (int)hlv.size() - 1;
     *nchk = (int)hchk.size() - 1;
     return NISE_OK;
+}
+
+extern "C" int nise_trotter_needs_bank_order(int kernel_config, int is_tuned, int tuned, int default_rows, int autotune) {
+    return needs_bank_order(kernel_config, is_tuned ? tuned : NOT_TUNED, default_rows, autotune != 0);
 }
 
 struct AbsRun {
@@ -499,10 +513,8 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
         const bool rows = (asked || rows_ok) && N + 64 <= NISE_ROW_MAX && TP.k <= NISE_ROW_MAX && p.ts >= 1;
         in_order({});
         if (rows && (rc = build_rows())) return rc;
-        // the warp kernels' bank order costs the host more than the levels, so
-        // not where the rows are taken anyway
-        const int cfg = rows ? default_rows(N, TP.rot_static, plain ? 3 : nvec, rows_of(TP), (long)p.ts * (TP.k + 2L * N)) : 0;
-        if (!asked && (!cfg || autotune)) {
+        const int by_rows = rows ? default_rows(N, TP.rot_static, plain ? 3 : nvec, rows_of(TP), (long)p.ts * (TP.k + 2L * N)) : 0;
+        if (needs_bank_order(p.kernel_config, tuned, by_rows, autotune)) {
             std::vector<char> hflip;
             bank_order(pairs, N, hchk, hperm, hflip);
             in_order(hflip);
