@@ -48,29 +48,59 @@ std::map<TuneKey, int> g_tuned;
 const int NOT_TUNED = -1000;
 std::mutex g_tune_mu;
 
+// Rows of 32 (index 0) and of 64 operations of a job: how many make a time step,
+// and the vectors of a CTA that has the schedule in shared memory (0: it does not
+// fit there beside them, or was not built).
 struct RowCounts {
-    int n[2];
+    int n[2], vecs[2];
 };
 
+// Jobs that may run on rows of 32 operations, and on rows of 64 (static couplings;
+// two warps a vector), by size: default_rows' lines, before the rows are made.
+bool rows_possible(int prec, int N, bool rot_static, int nvec) {
+    if (!rot_static) return N <= 128;
+    return N <= (prec == NISE_FP32 ? 80 : 100) || (N <= 400 && nvec <= 8 * sm_count());
+}
+bool rows64_possible(int N, bool rot_static, int nvec) { return rot_static && N <= 400 && nvec <= 4 * sm_count(); }
+
 // Rows of operations, where they are the fastest Trotter kernel: 35 (a warp
-// per vector, rows of 32), 36 (two warps, rows of 64) or 0.  rows.n[w]: rows of 32
-// (w = 0) and 64 per time step of `ops` operations, 0 where they do not fit.
-// Per-frame couplings up to 128 sites: 16-site chain, 1482 vectors, 0.67 ms
-// against 1.02 (warp per level) and 1.85 (thread per vector); 64-site chain 0.84
-// against 2.4 and 8.0; 64 sites all coupled 3.2 against 3.9.  Static couplings:
-// up to 100 sites (64-site lattice, 2982 vectors, 3.1 against 3.9 ms for two
-// vectors per warp), and up to 400 with few vectors (372 sites, 285 vectors, 3.0
-// against 4.0 ms; with 1476 vectors 12.6 against 8.0; 547 sites, 585 vectors,
-// 5.8 against 5.6: full rows meet more bank conflicts than the levels' chunks,
-// which are ordered against them).  Rows of 64 where they are fewer by a quarter
-// (372 sites: 3.0 against 3.6; 64 sites: 1.18 against 0.78).  Above about 860
-// operations per row and vector the SMs' warps are all busy and a thread per
-// vector is faster (16-site chain, 7422 vectors: 1.9 against 2.2 ms).
-int default_rows(int N, bool rot_static, int nvec, RowCounts rows, long ops) {
-    const bool few = nvec < 8 * sm_count();
-    if (!rows.n[0] || !(rot_static ? N <= 100 || (few && N <= 400) : N <= 128) || (double)nvec * rows.n[0] >= 860.0 * ops)
-        return 0;
-    return rows.n[1] && rot_static && 4 * rows.n[1] < 3 * rows.n[0] ? 36 : 35;
+// per vector, rows of 32), 36 (two warps, rows of 64) or 0.  `ops` operations and
+// `chunks` level chunks make a time step.  Only with the schedule in shared memory:
+// read from L2 a row takes three times as long (128 sites all coupled, 6 vectors: 8.2
+// ms, warp per level 3.6; 100 sites, 1800 vectors 12.0 and 8.3).
+// - All vectors in one wave of CTAs: per-frame couplings up to 128 sites (16-site
+//   chain, 1482 vectors, 0.67 ms against 1.02 for a warp per level and 1.85 for a
+//   thread per vector; 64 sites all coupled, 900 vectors 1.61 against 2.55; 120 sites
+//   all coupled, 60 vectors 2.8 against 3.3), static ones up to 400 (64-site lattice,
+//   1170 vectors, 0.49 against 0.89; 400 sites, 600 vectors 1.87 against 2.07; 547
+//   sites, 585 vectors, 5.8 against 5.6: full rows meet more bank conflicts than the
+//   levels' chunks, which are ordered against them).  Rows of 64 where they are fewer
+//   by a quarter and make one wave (372 sites: 3.0 against 3.6; 64 sites: 1.18 against
+//   0.78; in a second wave, 200 sites, 600 vectors: 1.79 against 0.95).
+// - More waves: against a thread per vector (narrow levels) until the SMs' warps are
+//   all busy, about 860 operations per row and vector (16-site chain, 7422 vectors: 2.2
+//   against 1.9 ms); static couplings against two vectors per warp up to 80 sites in
+//   FP32 (80 sites, 1200 vectors 1.07 against 1.13; 100 sites 1.22 against 1.11), 100 in
+//   FP64 (1200 vectors 1.97 against 2.81); wide levels of per-frame couplings where the
+//   waves' rows are fewer than the chunks by 5 %, with eight vectors per CTA, in FP64 also
+//   with four, whose wave takes half as long (48 sites all coupled, 1800 vectors 2.59
+//   against 2.95; with a short last wave, 64 sites of 6 neighbours, 2400 vectors: 1.30
+//   against 1.09; FP64, 64 sites all coupled, 3000 vectors 9.6 against 11.4).
+// - Wide levels of per-frame couplings from 16 time points on: below, the copy of the
+//   schedule costs more than its rows save (100 sites all coupled, 6 vectors, 8 points:
+//   0.50 against 0.45; 0.09 ms once against 0.007 a step).
+int default_rows(int prec, int N, bool rot_static, bool wide, int nvec, int tmax, RowCounts rows, long ops, long chunks) {
+    const long sms = sm_count();
+    auto waves = [&](int w) { return (nvec + rows.vecs[w] * sms - 1) / (rows.vecs[w] * sms); };
+    if (!rows.vecs[0] || !rows_possible(prec, N, rot_static, nvec) || (double)nvec * rows.n[0] >= 860.0 * ops) return 0;
+    if (rows64_possible(N, rot_static, nvec) && rows.vecs[1] && waves(1) == 1 && 4 * rows.n[1] < 3 * rows.n[0]) return 36;
+    if (!rot_static && wide && tmax < 16) return 0;
+    if (waves(0) == 1) return 35;
+    if (rot_static) return N <= (prec == NISE_FP32 ? 80 : 100) ? 35 : 0;
+    if (!wide) return 35;
+    const double wave = prec == NISE_FP32 ? 1.0 : rows.vecs[0] / 8.0;  // of a CTA of eight
+    return rows.vecs[0] >= (prec == NISE_FP32 ? 8 : 4) &&
+                   1.05 * wave * waves(0) * rows.n[0] * 8 * sms < (double)chunks * nvec ? 35 : 0;
 }
 
 // Whether a Trotter job's rotations need the warp kernels' bank order, which costs
@@ -88,9 +118,9 @@ bool needs_bank_order(int kernel_config, int tuned, int default_rows, bool autot
 // threads (a warp per vector then has the shorter critical path); thread per
 // vector for chains (one rotation per level) with many vectors.
 int default_config(int scheme, int N, bool plain, bool cheb, int K, int nchk, int nvec, bool has4, bool rv,
-                   bool rot_static, RowCounts rows, long ops) {
+                   bool rot_static, int by_rows) {
     if (scheme == SCHEME_TROTTER) {
-        if (const int r = default_rows(N, rot_static, nvec, rows, ops)) return r;
+        if (by_rows) return by_rows;
         // a warp per two vectors once there are 8 or more vectors per SM (static
         // couplings; 1024-site lattice, 1185 vectors: 39.3 against 43.9 ms),
         // else a warp per vector (C4's 585-vector jobs: 18.6 against 25.5 ms at
@@ -315,12 +345,7 @@ struct AbsRun {
     DevBuf<uint32_t> row_ab[2];  // rows of 32 and of 64 operations
     DevBuf<uint16_t> row_id[2];
     RowPlan row[2] = {};
-    RowCounts rows_of(const TrotterPlan &P) const {
-        RowCounts r = {{0, 0}};
-        for (int w = 0; w < 2; w++)
-            if (trotter_rows_fit(prec == NISE_FP32 ? 0 : 1, P, row[w], 32 * (w + 1))) r.n[w] = row[w].nrow;
-        return r;
-    }
+    int by_rows = 0;  // the rows that are the job's default (35, 36), or 0
     TrotterPlan TP;
     // RK4
     DevBuf<int2> dent;
@@ -496,10 +521,12 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
         // The whole step as rows, from the level order (every site's order is
         // the same), for the sizes default_config takes them at, or on demand.
         const bool asked = p.kernel_config == 35 || p.kernel_config == 36;
-        const bool rows_ok = p.kernel_config == 0 && N <= (TP.rot_static ? 400 : 128);
+        const int nv = plain ? 3 : nvec;
+        const bool both = autotune || tuned == 35 || tuned == 36;  // the tuner's candidates
+        const bool wanted = p.kernel_config == 0 && (both ? N <= (TP.rot_static ? 400 : 128) : rows_possible(prec, N, TP.rot_static, nv));
         auto build_rows = [&]() -> int {
             for (int w = 0; w < 2; w++) {
-                if (w == 1 && !TP.rot_static && p.kernel_config != 36) break;  // never the default
+                if (w == 1 && p.kernel_config != 36 && !(TP.rot_static && (both || rows64_possible(N, true, nv)))) break;
                 std::vector<uint32_t> ab;
                 std::vector<uint16_t> id;
                 row[w].nrow = nise_row_schedule(lpairs, N, p.ts, 32 * (w + 1), ab, id);
@@ -510,10 +537,17 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
             }
             return NISE_OK;
         };
-        const bool rows = (asked || rows_ok) && N + 64 <= NISE_ROW_MAX && TP.k <= NISE_ROW_MAX && p.ts >= 1;
+        const bool rows = (asked || wanted) && N + 64 <= NISE_ROW_MAX && TP.k <= NISE_ROW_MAX && p.ts >= 1;
         in_order({});
         if (rows && (rc = build_rows())) return rc;
-        const int by_rows = rows ? default_rows(N, TP.rot_static, plain ? 3 : nvec, rows_of(TP), (long)p.ts * (TP.k + 2L * N)) : 0;
+        if (rows && p.kernel_config == 0) {
+            RowCounts r;
+            for (int w = 0; w < 2; w++) {
+                r.n[w] = row[w].nrow;
+                r.vecs[w] = trotter_rows_vecs(prec == NISE_FP32 ? 0 : 1, TP, row[w], 32 * (w + 1), nv);
+            }
+            by_rows = default_rows(prec, N, TP.rot_static, TP.k >= 4 * nchk, nv, tmax, r, (long)p.ts * (TP.k + 2L * N), (long)p.ts * nchk);
+        }
         if (needs_bank_order(p.kernel_config, tuned, by_rows, autotune)) {
             std::vector<char> hflip;
             bank_order(pairs, N, hchk, hperm, hflip);
@@ -996,8 +1030,7 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
     }
     config = default_config(scheme, N, plain, cheb, TP.k, nchk, plain ? 3 : nvec, dell4.p != nullptr,
                             scheme == SCHEME_TAYLOR && taylor_rv_runs(T, XP),
-                            scheme == SCHEME_TROTTER && TP.rot_static,
-                            scheme == SCHEME_TROTTER ? rows_of(TP) : RowCounts{{0, 0}}, (long)p.ts * (TP.k + 2L * N));
+                            scheme == SCHEME_TROTTER && TP.rot_static, by_rows);
     if (p.kernel_config != 0) {  // forced by the caller
         const int k = p.kernel_config;
         if (scheme == SCHEME_EIGEN && (k == 2 || k == 16 || k == 17)) return NISE_OK;

@@ -134,6 +134,9 @@ int launch_abs_trotter_wv2(int prec, const DevTraj &T, const TrotterPlan &P, con
 // The same from rows of 32 or 64 operations (nise_row_schedule of P.pairs),
 // bitwise identical to all of these; whether one vector fits shared memory.
 bool trotter_rows_fit(int prec, const TrotterPlan &P, const RowPlan &Q, int width);
+// Vectors per CTA of a job of nvec with the schedule in shared memory; 0 where it is
+// read from L2 or does not fit.
+int trotter_rows_vecs(int prec, const TrotterPlan &P, const RowPlan &Q, int width, int nvec);
 int launch_abs_trotter_rows(int prec, const DevTraj &T, const TrotterPlan &P, const RowPlan &Q, int width,
                             const AbsJob &J, double2 *resp, cudaStream_t s);
 int launch_prep_rk4(int prec, const DevTraj &T, const Rk4Plan &P, double fsub, float fsub32, cudaStream_t s);

@@ -66,6 +66,13 @@ bool trotter_rows_fit(int prec, const TrotterPlan &P, const RowPlan &Q, int widt
                .vecs > 0;
 }
 
+int trotter_rows_vecs(int prec, const TrotterPlan &P, const RowPlan &Q, int width, int nvec) {
+    if (!Q.ab) return 0;
+    const RowShape h = prec == 0 ? rows_shape<float>(P.n, P.k, P.rot_static, Q.nrow, width / 32, nvec, sm_count())
+                                 : rows_shape<double>(P.n, P.k, P.rot_static, Q.nrow, width / 32, nvec, sm_count());
+    return h.stage ? h.vecs : 0;
+}
+
 int launch_abs_trotter_rows(int prec, const DevTraj &T, const TrotterPlan &P, const RowPlan &Q, int width,
                             const AbsJob &J, double2 *resp, cudaStream_t s) {
     if (J.nsamp <= 0) return 0;
