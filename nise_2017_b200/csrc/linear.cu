@@ -440,10 +440,8 @@ int run_lin(const LinJob &J, const RowPlan &Q, double2 *out, int nch, int first,
         if ((e = (int)cudaFuncSetAttribute(k_lin_dia<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(VG * row))))
             return e;
         k_lin_dia<R><<<(unsigned)(J.S * ((J.nvec + VG - 1) / VG)), nw + nr, VG * row, st>>>(J, VG, nr);
-    } else if (Q.ab && (double)nv * Q.nrow < 860.0 * J.ts * (J.K + 2.0 * J.n) &&
-               rows_shape<R>(J.n, J.K, J.rot_static, Q.nrow, 1, nv, sm_count()).vecs > 0) {
-        // Trotter: a warp per vector, until the vectors fill threads (the same
-        // line as for absorption)
+    } else if (rows_pay<R>(J.n, J.K, J.rot_static, J.ts, Q, nv, sm_count())) {
+        // Trotter: a warp per vector
         const RowShape h = rows_shape<R>(J.n, J.K, J.rot_static, Q.nrow, 1, nv, sm_count());
         if ((e = (int)cudaFuncSetAttribute(k_lin_rows<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.bytes)))
             return e;

@@ -141,3 +141,16 @@ template <typename R> inline RowShape rows_shape(int n, int K, bool rot_static, 
     s.bytes = base + s.vecs * per;
     return s;
 }
+
+// Whether `vectors` go through the rows faster than a thread each (k_lin, k2d_gb1,
+// k2d_gb3, k2d_se): until the vectors fill the threads, in FP32 about 860 operations
+// per row and vector, 580 where the schedule is read from L2, in FP64 600 and 350.
+// Measured: 16-site chain, 7422 vectors, 2.2 against 1.9 ms; the t3 vectors of 1500
+// start points of 5 sites 4.0 against 0.73; FP64, 100 sites all coupled, 10 000 vectors
+// (read from L2) 61 against 57, 3 sites, 1200 vectors of t3 0.34 against 0.31.
+template <typename R> inline bool rows_pay(int n, int K, bool rot_static, int ts, const RowPlan &Q, long vectors, int sms) {
+    if (!Q.ab) return false;
+    const RowShape h = rows_shape<R>(n, K, rot_static, Q.nrow, 1, vectors, sms);
+    const double most = sizeof(R) == 4 ? (h.stage ? 860 : 580) : (h.stage ? 600 : 350);
+    return h.vecs > 0 && (double)vectors * Q.nrow < most * ts * (K + 2.0 * n);
+}

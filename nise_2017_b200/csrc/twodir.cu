@@ -2036,16 +2036,16 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf, const RowPlan &Q) {
     if ((e = smem_attr(k2d_gb1<R>, sm))) return e;
     if ((e = smem_attr(k2d_gb3<R>, sm))) return e;
     if ((e = smem_attr(k2d_se<R>, sm))) return e;
-    // Trotter: a warp per vector where its state and tables fit shared memory
-    const bool rows = Q.ab && rows_shape<R>(D.n, D.K, D.rot_static, Q.nrow, 1, 1, 1).vecs > 0;
-    if (rows) {
+    // Trotter: a warp per vector while the vectors do not fill the threads
+    auto rows = [&](long vectors) { return rows_pay<R>(D.n, D.K, D.rot_static, D.ts, Q, vectors, sm_count()); };
+    if (rows((long)D.S * 3 * P)) {
         if ((e = run_rows<R>(k2d_gb1_rows<R>, D, Q, (long)D.S * 3 * P, st))) return e;
     } else {
         k2d_gb1<R><<<(D.S * 3 * P + B - 1) / B, B, sm, st>>>(D);
     }
     c->launches++;
     if (D.gb) {
-        if (rows) {
+        if (rows((long)D.S * 3)) {
             if ((e = run_rows<R>(k2d_gb3_rows<R>, D, Q, (long)D.S * 3, st))) return e;
         } else {
             k2d_gb3<R><<<(D.S * 3 + B - 1) / B, B, sm, st>>>(D);
@@ -2062,7 +2062,7 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf, const RowPlan &Q) {
             c->launches++;
         }
         int nv = D.S * (3 + 3 * D.T1);
-        if (rows) {
+        if (rows(nv)) {
             if ((e = run_rows<R>(k2d_se_rows<R>, D, Q, nv, st))) return e;
         } else {
             k2d_se<R><<<(nv + B - 1) / B, B, sm, st>>>(D);
