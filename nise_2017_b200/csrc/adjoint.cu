@@ -1122,9 +1122,13 @@ struct AdjSched {
     DevBuf<uint2> s1, sW;
     DevBuf<uint32_t> parts;
     DevBuf<int> iso;
-    int build(nise_ctx *c, const std::vector<int2> &pairs, AdjPlan &P) {
+    int build(nise_ctx *c, const std::vector<int2> &pairs, AdjPlan &P, int nsamp) {
         // one vector's state, its adjoint and gradient on a warp of three: up
-        // to 1600 sites; above, a thread per vector
+        // to 1600 sites; above, a thread per vector, and where the vectors fill the
+        // threads: from about 390 operations per row and vector on (model and
+        // gradient, RunTimes 48, all coupled: 5 sites, 400 start points 1.44 ms against
+        // 1.72 with a thread per vector, 800 2.30 against 1.83, 3000 6.9 against 2.5; 8
+        // sites, 3000 11.1 against 4.2)
         P.W = 1;
         if (P.n > NISE_SCHED_MAX_N || P.k > NISE_SCHED_MAX_K || adj_bwd_bytes(P.n, P.k, 1, false) > 220 * 1024 || P.ts < 1)
             return NISE_OK;
@@ -1147,8 +1151,12 @@ struct AdjSched {
         } else {
             rW = r1;
         }
-        P.mat = mat(P.W);
         P.nrowW = (int)(rW.size() / 32);
+        if (3.0 * nsamp * P.nrowW / P.W >= 390.0 * P.ts * (P.k + 2.0 * P.n)) {
+            P.W = 1;
+            return NISE_OK;
+        }
+        P.mat = mat(P.W);
         P.niso = (int)is.size();
         // the rotation's packed sites beside each entry, two idle rows on either
         // side (the kernels read two rows ahead, in both directions).  With `mat`
@@ -1218,7 +1226,7 @@ int adj_forward(nise_ctx *c, const double *shift, double scale, int K, AdjRun &R
     P.scale = scale;
     P.f = nise_f64(p, 1, p.ts);
     std::vector<double> hs(shift, shift + N);
-    if ((rc = Q.build(c, pairs, P))) return rc;
+    if ((rc = Q.build(c, pairs, P, R.nsamp))) return rc;
     if ((rc = dshift.upload(c, hs)) || (rc = dpairs.upload(c, pairs.empty() ? std::vector<int2>(1) : pairs)) ||
         (rc = U.alloc(c, (size_t)R.nf * N)) || (rc = rot.alloc(c, (size_t)R.nf * (P.k ? P.k : 1))) ||
         (rc = jf.alloc(c, (size_t)R.nf * (P.k ? P.k : 1) * (P.mat ? 2 : 1))) || (rc = ckpt.alloc(c, (size_t)nvec * P.nck * N)))
