@@ -708,7 +708,7 @@ extern "C" int nise_propagate(nise_ctx *c, const float *H, void *re, void *im, i
     cudaMemcpyAsync(dH.p, H, sizeof(float) * nvec * c->nn2, cudaMemcpyHostToDevice, c->stream);
     cudaMemcpyAsync(dr.p, re, rsz * nvec * N, cudaMemcpyHostToDevice, c->stream);
     cudaMemcpyAsync(di.p, im, rsz * nvec * N, cudaMemcpyHostToDevice, c->stream);
-    // a CTA per vector; a thread per vector where that does not fit
+    // a CTA per vector; a thread per vector where that does not fit or is faster
     const double f64 = nise_f64(p, sign, p.ts);
     const float f32 = nise_f32(p, sign, p.ts);
     int e;

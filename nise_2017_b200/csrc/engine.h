@@ -189,7 +189,8 @@ int launch_step_rk4(int prec, int n, float cut, const float *H, void *re, void *
 int launch_step_taylor(int prec, int n, const float *H, void *re, void *im, int nvec, double f, cudaStream_t s);
 // The same with a CTA per vector; cudaErrorNotSupported where a vector's tables
 // exceed shared memory (Trotter, above about 220 sites) or its rows a CTA (RK4
-// and the exact step, above 1024).
+// and the exact step, above 1024), and where so many vectors of so few sites are
+// faster on a thread each.
 int launch_step_coupling_cta(int prec, int n, float cut, const float *H, void *re, void *im, int nvec, int ts,
                              double fsub, float fsub32, cudaStream_t s);
 int launch_step_rk4_row(int prec, int n, float cut, const float *H, void *re, void *im, int nvec, int ts, double fsub,

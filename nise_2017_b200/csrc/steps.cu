@@ -154,7 +154,10 @@ __global__ void __launch_bounds__(1024) k_step_taylor_cta(int n, const float *H,
 template <typename R>
 int run_coupling(int n, float cut, const float *H, R *re, R *im, int nvec, int ts, R fsub, cudaStream_t s) {
     const size_t bytes = sizeof(typename Vec2<R>::T) * (2 * (size_t)n + (size_t)n * (n - 1) / 2);
-    if (bytes > 220 * 1024) return (int)cudaErrorNotSupported;
+    // a thread per vector again where the vectors fill the threads: whole calls of 2, 8
+    // and 16 sites with 50 000 vectors 0.39, 1.51 and 3.78 ms against 0.33, 1.32 and 3.66,
+    // with 10 000 0.12, 0.38 and 0.87 against 0.11, 0.39 and 1.04
+    if (bytes > 220 * 1024 || nvec >= 2500L * n) return (int)cudaErrorNotSupported;
     const int e = (int)cudaFuncSetAttribute(k_step_coupling_cta<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e) return e;
     k_step_coupling_cta<R><<<nvec, (n + 63) / 64 * 32, bytes, s>>>(n, cut, H, re, im, ts, fsub);
@@ -181,7 +184,9 @@ int launch_step_coupling_cta(int prec, int n, float cut, const float *H, void *r
 }
 
 int launch_step_taylor_cta(int prec, int n, const float *H, void *re, void *im, int nvec, double f, cudaStream_t s) {
-    if (n > 1024) return (int)cudaErrorNotSupported;
+    // below 8 sites a thread per vector where the vectors fill the threads: 5 sites, 50 000
+    // vectors 0.84 against 0.76 ms, 10 000 0.20 and 0.20; 8 sites are no slower here
+    if (n > 1024 || (n < 8 && nvec >= 2500 * n)) return (int)cudaErrorNotSupported;
     return prec == 0 ? run_taylor<float>(n, H, (float *)re, (float *)im, nvec, f, s)
                      : run_taylor<double>(n, H, (double *)re, (double *)im, nvec, f, s);
 }
