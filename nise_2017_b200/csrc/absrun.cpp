@@ -587,7 +587,10 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
         if ((rc = dent.upload(c, ent)) || (rc = rkval.alloc(c, rsz * (size_t)nf * RP.k))) return rc;
         RP.entries = dent.p;
         RP.val = rkval.p;
-        if (N <= NISE_RK4_ROW_MAX_N) {
+        // (many start points of a few sites fill the GPU with a thread per vector: 2
+        // sites, 3 entries, RunTimes 48, 1200 start points 0.70 ms either way, 4000 1.88
+        // against 0.78 ms; 5 sites, 15 entries, 4000 2.77 against 2.22)
+        if (N <= NISE_RK4_ROW_MAX_N && (plain || nsamp < 200L * RP.k + 500)) {
             // every row's entries in ascending neighbour order: the entry list
             // visits row i with its lower neighbours, itself, its upper ones
             std::vector<std::vector<uint32_t>> row(N);
@@ -1093,7 +1096,7 @@ int AbsRun::run_main(cudaStream_t s, int cfg, double2 *dst) {
             if (cfg > 0) return launch_abs_trotter_lv(pr, T, TP, Js, r, lvptr.p, nlev, cfg, s);
             return launch_abs_trotter(pr, T, TP, Js, r, s);
         case SCHEME_RK4:
-            // a thread per site row up to the size that a CTA holds, a thread per vector above
+            // a thread per site row where the plan made the row lists, else a thread per vector
             return RP.rows ? launch_abs_rk4_row(pr, T, RP, Js, r, s) : launch_abs_rk4(pr, T, RP, Js, r, s);
         case SCHEME_TAYLOR: {
             TaylorPlan P = XP;
