@@ -194,10 +194,6 @@ __global__ void __launch_bounds__(NT, 1)
     // site of this lane's row in its it-th slice (n: none)
     const uint32_t *wrow = rows + warp * kRvMaxIT * 8 + r;
     auto site = [&](int it) { return (int)NISE_RV_ROW(wrow[8 * it]); };
-    // a warp without slices (small lattices leave most without) has no part in the
-    // terms; with as few slice places as the busiest warp needs (IT), 16 sites, 4500
-    // vectors, 64 steps take 1.04 ms, 1.70 when every warp went through four places
-    const bool idle = (int)NISE_RV_ROW(rows[warp * kRvMaxIT * 8]) >= n;
 #pragma unroll
     for (int it = 0; it < IT; it++) {
         const int i = site(it);
@@ -313,15 +309,17 @@ __global__ void __launch_bounds__(NT, 1)
             const float4 *src = cur + (size_t)((k - 1) & 1) * n * 4;
             float4 *dst = cur + (size_t)(k & 1) * n * 4;
             const char *srcc = (const char *)(src + c);
-            if (idle) {
-                __syncthreads();
-                continue;
-            }
             const float4 *tp = tri + 8 * NISE_RV_FIRST(wrow[0]) + r;
             float4 w = *tp;
 #pragma unroll
             for (int it = 0; it < IT; it++) {
                 const uint32_t wd = wrow[8 * it];
+                // no slice: small lattices leave most places of most warps empty (16
+                // sites, 4500 vectors, 64 steps 1.70 ms when they were gone through, 1.34
+                // now).  Not an instantiation with fewer places: with two, the Chebyshev
+                // sums of 768 threads came out wrong from 100 sites on, with or without
+                // this line, and the source does not show why.
+                if (IT <= 4 && wd << 12 == (uint32_t)n << 12) continue;
                 const int i = NISE_RV_ROW(wd);
                 const float4 own = i < n ? src[(size_t)i * 4 + c] : make_float4(0.f, 0.f, 0.f, 0.f);
                 float a0 = d0[it] * own.x, b0 = d0[it] * own.y;
@@ -419,14 +417,10 @@ int launch_abs_taylor_rv(const DevTraj &T, const TaylorPlan &P, const AbsJob &J,
     if (!taylor_rv_fits(T, P)) return (int)cudaErrorNotSupported;
     const int sh = P.rv_shape, it = P.ell8_it[sh];
     if (sh == 0) {
-        if (it <= 1) return run_rv<1, 768>(T, P, J, resp, v0, nvec, s);
-        if (it <= 2) return run_rv<2, 768>(T, P, J, resp, v0, nvec, s);
         if (it <= 4) return run_rv<4, 768>(T, P, J, resp, v0, nvec, s);
         if (it <= 6) return run_rv<6, 768>(T, P, J, resp, v0, nvec, s);
         return run_rv<8, 768>(T, P, J, resp, v0, nvec, s);
     }
-    if (it <= 1) return run_rv<1, 1024>(T, P, J, resp, v0, nvec, s);
-    if (it <= 2) return run_rv<2, 1024>(T, P, J, resp, v0, nvec, s);
     if (it <= 4) return run_rv<4, 1024>(T, P, J, resp, v0, nvec, s);
     if (it <= 6) return run_rv<6, 1024>(T, P, J, resp, v0, nvec, s);
     return run_rv<8, 1024>(T, P, J, resp, v0, nvec, s);

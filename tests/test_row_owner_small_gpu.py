@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 SPARSE_FP32 = 3e-6  # FP32 series vs the exact propagator
 
 
-@pytest.mark.parametrize("n, cut", [(1, 2.0), (7, 2.0), (8, 2.0), (9, 2.0), (9, 1e6), (33, 60.0), (193, 2.0)])
+@pytest.mark.parametrize("n, cut", [(1, 2.0), (7, 2.0), (8, 2.0), (9, 2.0), (9, 1e6), (33, 60.0), (100, 2.0), (193, 2.0), (300, 2.0), (385, 2.0)])
 def test_row_owner_on_small_lattices(n, cut, tmp_path):
     frames = 470
     files = synth.write(synth.c1_spec(n_sites=n, frames=frames, seed=n + 2), str(tmp_path))
