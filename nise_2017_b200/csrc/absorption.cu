@@ -1490,13 +1490,6 @@ int lanes_for(size_t bytes_per_lane, int want) {
 
 const size_t kMaxSmem = 227 * 1024;  // dynamic shared memory per CTA on sm_100
 
-template <typename K>
-int set_smem(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024)
-        return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    return 0;
-}
-
 }  // namespace
 
 // ------------------------------------------------------------ launchers
@@ -1525,10 +1518,10 @@ int launch_abs_trotter(int prec, const DevTraj &T, const TrotterPlan &P, const A
     int grid = (nvec + B - 1) / B;
     int e;
     if (prec == 0) {
-        if ((e = set_smem(k_abs_trotter<float>, smem))) return e;
+        if ((e = allow_smem(k_abs_trotter<float>, smem))) return e;
         k_abs_trotter<float><<<grid, B, smem, s>>>(T, P, J, resp, nvec);
     } else {
-        if ((e = set_smem(k_abs_trotter<double>, smem))) return e;
+        if ((e = allow_smem(k_abs_trotter<double>, smem))) return e;
         k_abs_trotter<double><<<grid, B, smem, s>>>(T, P, J, resp, nvec);
     }
     return (int)cudaGetLastError();
@@ -1540,10 +1533,10 @@ int launch_abs_trotter_lv(int prec, const DevTraj &T, const TrotterPlan &P, cons
     const size_t smem = (size_t)3 * P.n * ((prec == 0 ? sizeof(float2) : sizeof(double2)) + sizeof(float));
     int e;
     if (prec == 0) {
-        if ((e = set_smem(k_abs_trotter_lv<float>, smem))) return e;
+        if ((e = allow_smem(k_abs_trotter_lv<float>, smem))) return e;
         k_abs_trotter_lv<float><<<J.nsamp, threads, smem, s>>>(T, P, J, resp, lvptr, nlev);
     } else {
-        if ((e = set_smem(k_abs_trotter_lv<double>, smem))) return e;
+        if ((e = allow_smem(k_abs_trotter_lv<double>, smem))) return e;
         k_abs_trotter_lv<double><<<J.nsamp, threads, smem, s>>>(T, P, J, resp, lvptr, nlev);
     }
     return (int)cudaGetLastError();
@@ -1601,7 +1594,7 @@ int launch_abs_trotter_wv(int prec, const DevTraj &T, const TrotterPlan &P, cons
     int e;
 #define NISE_WV(RT, SMT)                                                                         \
     do {                                                                                       \
-        if ((e = set_smem(k_abs_trotter_wv<RT, SMT>, smem))) return e;                         \
+        if ((e = allow_smem(k_abs_trotter_wv<RT, SMT>, smem))) return e;                         \
         k_abs_trotter_wv<RT, SMT><<<grid, 32 * W, smem, s>>>(T, P, J, resp, nvec, chk, nchk, us); \
     } while (0)
     if (prec == 0) {
@@ -1644,7 +1637,7 @@ int launch_abs_trotter_wv2(int prec, const DevTraj &T, const TrotterPlan &P, con
     int e;
 #define NISE_WV2(RT, SMT)                                                                    \
     do {                                                                                   \
-        if ((e = set_smem(k_abs_trotter_wv2<RT, SMT>, smem))) return e;                    \
+        if ((e = allow_smem(k_abs_trotter_wv2<RT, SMT>, smem))) return e;                    \
         k_abs_trotter_wv2<RT, SMT><<<grid, 32 * W, smem, s>>>(T, P, J, resp, nvec, chk, nchk); \
     } while (0)
     if (prec == 0) {
@@ -1674,10 +1667,10 @@ int launch_abs_rk4(int prec, const DevTraj &T, const Rk4Plan &P, const AbsJob &J
     int grid = (nvec + B - 1) / B;
     int e;
     if (prec == 0) {
-        if ((e = set_smem(k_abs_rk4<float>, smem))) return e;
+        if ((e = allow_smem(k_abs_rk4<float>, smem))) return e;
         k_abs_rk4<float><<<grid, B, smem, s>>>(T, P, J, resp, nvec);
     } else {
-        if ((e = set_smem(k_abs_rk4<double>, smem))) return e;
+        if ((e = allow_smem(k_abs_rk4<double>, smem))) return e;
         k_abs_rk4<double><<<grid, B, smem, s>>>(T, P, J, resp, nvec);
     }
     return (int)cudaGetLastError();
@@ -1697,7 +1690,7 @@ static int run_taylor(const DevTraj &T, const TaylorPlan &P, const AbsJob &J, do
     int NT = 512;
     size_t smem = 2 * (size_t)P.n * G * sizeof(typename Vec2<R>::T) + (NT / 32) * 2 * G * sizeof(double);
     int e;
-    if ((e = set_smem(k_abs_taylor<R, G, RPT>, smem))) return e;
+    if ((e = allow_smem(k_abs_taylor<R, G, RPT>, smem))) return e;
     int grid = (nvec + G - 1) / G;
     k_abs_taylor<R, G, RPT><<<grid, NT, smem, s>>>(T, P, J, resp, nvec);
     return (int)cudaGetLastError();
@@ -1709,7 +1702,7 @@ static int run_taylor2(const DevTraj &T, const TaylorPlan &P, const AbsJob &J, d
     const int NT = 512;
     size_t smem = 2 * (size_t)P.n * (G + 2) * sizeof(typename Vec2<R>::T) + (NT / 32) * G * 2 * sizeof(double);
     int e;
-    if ((e = set_smem(k_abs_taylor2<R, G, IT>, smem))) return e;
+    if ((e = allow_smem(k_abs_taylor2<R, G, IT>, smem))) return e;
     k_abs_taylor2<R, G, IT><<<(nvec + G - 1) / G, NT, smem, s>>>(T, P, J, resp, nvec);
     return (int)cudaGetLastError();
 }
@@ -1724,7 +1717,7 @@ template <int IT>
 static int run_taylor4(const DevTraj &T, const TaylorPlan &P, const AbsJob &J, double2 *resp, int nvec, cudaStream_t s) {
     size_t smem = (size_t)P.n * 4 * sizeof(float2) + 16 * 4 * 2 * sizeof(double);
     int e;
-    if ((e = set_smem(k_abs_taylor4<IT>, smem))) return e;
+    if ((e = allow_smem(k_abs_taylor4<IT>, smem))) return e;
     k_abs_taylor4<IT><<<(nvec + 3) / 4, 512, smem, s>>>(T, P, J, resp, nvec);
     return (int)cudaGetLastError();
 }
@@ -1738,7 +1731,7 @@ template <int IT>
 static int run_cheb3(const DevTraj &T, const TaylorPlan &P, const AbsJob &J, double2 *resp, int nvec, cudaStream_t s) {
     size_t smem = cheb3_smem(P);
     int e;
-    if ((e = set_smem(k_abs_cheb3<IT>, smem))) return e;
+    if ((e = allow_smem(k_abs_cheb3<IT>, smem))) return e;
     k_abs_cheb3<IT><<<(nvec + 7) / 8, 512, smem, s>>>(T, P, J, resp, nvec, (const EllEnt<float> *)P.ell, P.ell_sptr,
                                                       P.ell_nslices, P.ell_nent, P.cheb_inv_r, P.cheb_coef,
                                                       P.ell_rows);
@@ -1751,7 +1744,7 @@ static int run_taylor3_g(const DevTraj &T, const TaylorPlan &P, const AbsJob &J,
     if (nvec <= 0) return 0;
     size_t smem = taylor3_smem(P, sizeof(R), G, NT);
     int e;
-    if ((e = set_smem(k_abs_taylor3<R, IT, G, NT, CHEB>, smem))) return e;
+    if ((e = allow_smem(k_abs_taylor3<R, IT, G, NT, CHEB>, smem))) return e;
     k_abs_taylor3<R, IT, G, NT, CHEB><<<(nvec + G - 1) / G, NT, smem, s>>>(
         T, P, J, resp, v0, nvec, (const EllEnt<R> *)P.ell, P.ell_sptr, P.ell_nslices, P.ell_nent, P.ell_rows);
     return (int)cudaGetLastError();
@@ -1997,11 +1990,11 @@ int launch_step_coupling(int prec, int n, float cut, const float *H, void *re, v
     size_t smem = per_lane * B;
     int e;
     if (prec == 0) {
-        if ((e = set_smem(k_step_coupling<float>, smem))) return e;
+        if ((e = allow_smem(k_step_coupling<float>, smem))) return e;
         k_step_coupling<float><<<(nvec + B - 1) / B, B, smem, s>>>(n, cut, H, (float *)re, (float *)im, nvec, ts,
                                                                    fsub32);
     } else {
-        if ((e = set_smem(k_step_coupling<double>, smem))) return e;
+        if ((e = allow_smem(k_step_coupling<double>, smem))) return e;
         k_step_coupling<double><<<(nvec + B - 1) / B, B, smem, s>>>(n, cut, H, (double *)re, (double *)im, nvec,
                                                                     ts, fsub);
     }
@@ -2021,11 +2014,11 @@ int launch_step_rk4(int prec, int n, float cut, const float *H, void *re, void *
     if ((e = (int)cudaMallocAsync((void **)&ent, sizeof(int2) * (size_t)kmax * nvec, s))) return e;
     if ((e = (int)cudaMallocAsync(&val, rsz * (size_t)kmax * nvec, s))) return e;
     if (prec == 0) {
-        if ((e = set_smem(k_step_rk4<float>, smem))) return e;
+        if ((e = allow_smem(k_step_rk4<float>, smem))) return e;
         k_step_rk4<float><<<(nvec + B - 1) / B, B, smem, s>>>(n, cut, H, (float *)re, (float *)im, nvec, ts, fsub32,
                                                               ent, (float *)val, kmax);
     } else {
-        if ((e = set_smem(k_step_rk4<double>, smem))) return e;
+        if ((e = allow_smem(k_step_rk4<double>, smem))) return e;
         k_step_rk4<double><<<(nvec + B - 1) / B, B, smem, s>>>(n, cut, H, (double *)re, (double *)im, nvec, ts,
                                                                fsub, ent, (double *)val, kmax);
     }
@@ -2041,10 +2034,10 @@ int launch_step_taylor(int prec, int n, const float *H, void *re, void *im, int 
     size_t smem = per_lane * B;
     int e;
     if (prec == 0) {
-        if ((e = set_smem(k_step_taylor<float>, smem))) return e;
+        if ((e = allow_smem(k_step_taylor<float>, smem))) return e;
         k_step_taylor<float><<<(nvec + B - 1) / B, B, smem, s>>>(n, H, (float *)re, (float *)im, nvec, f);
     } else {
-        if ((e = set_smem(k_step_taylor<double>, smem))) return e;
+        if ((e = allow_smem(k_step_taylor<double>, smem))) return e;
         k_step_taylor<double><<<(nvec + B - 1) / B, B, smem, s>>>(n, H, (double *)re, (double *)im, nvec, f);
     }
     return (int)cudaGetLastError();

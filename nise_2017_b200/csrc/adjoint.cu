@@ -1042,15 +1042,14 @@ int launch_adj_fwd(const DevTraj &T, const AdjPlan &P, const AbsJob &J, double2 
         const bool sm = adj_fwd_bytes(P.n, P.k, P.W, true) <= kAdjShared;
         const size_t by = P.mat ? adj_mat_fwd_bytes(P.n, P.k, P.W) : adj_fwd_bytes(P.n, P.k, P.W, sm);
         auto kern = P.mat ? k_adj_fwd_mat : sm ? k_adj_fwd_warp<true> : k_adj_fwd_warp<false>;
-        if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)by)) return (int)e;
+        if (const int e = allow_smem(kern, by)) return e;
         kern<<<J.nsamp, 96, by, s>>>(T, P, J, resp, ckpt);
         return (int)cudaGetLastError();
     }
     const size_t lb = sizeof(double2) * P.n;
     const int B = lanes_adj(lb);
     const size_t sm = lb * B;
-    cudaError_t e = cudaFuncSetAttribute(k_adj_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e) return (int)e;
+    if (const int e = allow_smem(k_adj_fwd, sm)) return e;
     k_adj_fwd<<<(nvec + B - 1) / B, B, sm, s>>>(T, P, J, resp, ckpt);
     return (int)cudaGetLastError();
 }
@@ -1062,14 +1061,13 @@ int launch_adj_bwd(const DevTraj &T, const AdjPlan &P, const AbsJob &J, const do
         const bool sm = adj_bwd_bytes(P.n, P.k, P.W, true) <= kAdjShared;
         const size_t by = P.mat ? adj_mat_bwd_bytes(P.n, P.k, P.W) : adj_bwd_bytes(P.n, P.k, P.W, sm);
         auto kern = P.mat ? k_adj_bwd_mat : sm ? k_adj_bwd_warp<true> : k_adj_bwd_warp<false>;
-        if (cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)by)) return (int)e;
+        if (const int e = allow_smem(kern, by)) return e;
         kern<<<J.nsamp, 96, by, s>>>(T, P, J, G, ckpt, gshift_part, gscale_part);
     } else {
         const size_t lb = (2 * sizeof(double2) + sizeof(double)) * P.n;
         const int B = lanes_adj(lb);
         const size_t sm = lb * B;
-        cudaError_t e = cudaFuncSetAttribute(k_adj_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        if (e) return (int)e;
+        if (const int e = allow_smem(k_adj_bwd, sm)) return e;
         k_adj_bwd<<<(nvec + B - 1) / B, B, sm, s>>>(T, P, J, G, ckpt, gshift_part, gscale_part);
     }
     k_adj_reduce<<<(P.n + 127) / 128, 128, 0, s>>>(gshift_part, nvec, P.n, gshift);

@@ -69,3 +69,18 @@ __device__ __forceinline__ float traj_mu(const DevTraj &T, long t, int x, int i)
     return T.dipole[t * T.d_words + 1 + x * T.n + i];
 }
 
+// Lets a kernel be launched with `bytes` of dynamic shared memory.  The limit belongs
+// to the kernel in the whole process, and contexts on other threads launch it with
+// other sizes, so it is never set to one launch's size (another thread could lower
+// it between this call and the launch): it is raised once, to what the device allows
+// beside the kernel's static shared memory (at most 24 KB in this library, so that up
+// to 20 KB need no more than the 48 KB that every launch may have).
+template <typename K> int allow_smem(K kernel, size_t bytes) {
+    if (bytes <= 20 * 1024) return 0;
+    cudaFuncAttributes a;
+    const int e = (int)cudaFuncGetAttributes(&a, kernel);
+    if (e || (size_t)a.maxDynamicSharedSizeBytes >= bytes) return e;
+    const size_t most = 227 * 1024 - a.sharedSizeBytes;
+    if (bytes > most) return (int)cudaErrorInvalidValue;
+    return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}

@@ -361,8 +361,7 @@ template <int NC>
 int run_tc_apply(const float2 *U, int n, const float *xr, const float *xi, float *yr, float *yi, int *err,
                  cudaStream_t s, int sets = 1, size_t us = 0) {
     const size_t sm = tc_apply_smem<NC>();
-    cudaError_t e = cudaFuncSetAttribute(k_tc_apply<NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return (int)e;
+    if (const int e = allow_smem(k_tc_apply<NC>, sm)) return e;
     k_tc_apply<NC><<<dim3((n + kTcRows - 1) / kTcRows, sets), kTcThreads, sm, s>>>(U, us, n, xr, xi, yr, yi, err);
     return (int)cudaGetLastError();
 }

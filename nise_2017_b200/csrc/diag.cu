@@ -167,8 +167,7 @@ int run_abs_dia(const DevTraj &T, const typename Vec2<R>::T *U, long f0, int n, 
     const bool stage = one && all <= 227 * 1024;
     const size_t sm = stage ? all : base;
     auto kern = stage ? k_abs_dia<R, 1, true> : one ? k_abs_dia<R, 1, false> : k_abs_dia<R, 3, false>;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return (int)e;
+    if (const int e = allow_smem(kern, sm)) return e;
     kern<<<J.nsamp, threads, sm, s>>>(T, U, f0, n, own ? work / 32 : 0, J, resp);
     return (int)cudaGetLastError();
 }
@@ -180,14 +179,12 @@ int launch_build_u(int prec, const double *V, const double *w, long nfr, int n, 
                    void *U, cudaStream_t s) {
     if (nfr <= 0) return 0;
     size_t sm = dia_build_smem(n);
-    cudaError_t e;
+    int e;
     if (prec == 0) {
-        if ((e = cudaFuncSetAttribute(k_build_u<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)))
-            return (int)e;
+        if ((e = allow_smem(k_build_u<float>, sm))) return e;
         k_build_u<float><<<(unsigned)nfr, 256, sm, s>>>(V, w, n, f, thres, truncate, (float2 *)U);
     } else {
-        if ((e = cudaFuncSetAttribute(k_build_u<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)))
-            return (int)e;
+        if ((e = allow_smem(k_build_u<double>, sm))) return e;
         k_build_u<double><<<(unsigned)nfr, 256, sm, s>>>(V, w, n, f, thres, truncate, (double2 *)U);
     }
     return (int)cudaGetLastError();

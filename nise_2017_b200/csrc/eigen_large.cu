@@ -358,8 +358,7 @@ int launch_eig_large(const EigJob &J, const long *frames_dev, long nframes, doub
                      int *status, cudaStream_t s) {
     if (nframes <= 0) return 0;
     const size_t sm = eig_large_smem(J.n);
-    cudaError_t e = cudaFuncSetAttribute(k_eig_large, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-    if (e != cudaSuccess) return (int)e;
+    if (const int e = allow_smem(k_eig_large, sm)) return e;
     k_eig_large<<<(unsigned)nframes, kEgNT, sm, s>>>(J, frames_dev, A_ws, Z, w, status);
     return (int)cudaGetLastError();
 }

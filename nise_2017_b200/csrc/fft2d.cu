@@ -30,6 +30,7 @@
 #include <cstring>
 #include <vector>
 
+#include "common.cuh"
 #include "nise_b200.h"
 
 extern "C" void nise_set_global_error(const char *msg);
@@ -125,8 +126,7 @@ int transform(std::vector<double2> &a, int n, double2 *d0, double2 *d1) {
     const int threads = 128, bx = (n + threads - 1) / threads;
     const size_t sm = sizeof(double2) * n;
     cudaError_t e = cudaMemcpy(d0, a.data(), bytes, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && sm > 48 * 1024)
-        e = cudaFuncSetAttribute(k_dft_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e == cudaSuccess) e = (cudaError_t)allow_smem(k_dft_pass, sm);
     if (e == cudaSuccess) {
         k_dft_pass<<<dim3(bx, n), threads, sm>>>(d0, d1, n, 1, n);  // along the last index (t3)
         k_dft_pass<<<dim3(bx, n), threads, sm>>>(d1, d0, n, n, 1);  // along the first index (t1)

@@ -437,23 +437,19 @@ int run_lin(const LinJob &J, const RowPlan &Q, double2 *out, int nch, int first,
         int VG = (int)std::min<long>(std::min(64, (J.nvec + 3) / 4 * 4), std::max<long>(4, nv / (2 * sm_count()) / 4 * 4));
         while (VG > 4 && VG * row > 200 * 1024) VG -= 4;
         const int tiles = J.n * (VG / 4), nr = (VG * J.nread + 31) / 32 * 32, nw = std::min((tiles + 31) / 32 * 32, 768);
-        if ((e = (int)cudaFuncSetAttribute(k_lin_dia<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(VG * row))))
-            return e;
+        if ((e = allow_smem(k_lin_dia<R>, VG * row))) return e;
         k_lin_dia<R><<<(unsigned)(J.S * ((J.nvec + VG - 1) / VG)), nw + nr, VG * row, st>>>(J, VG, nr);
     } else if (rows_pay<R>(J.n, J.K, J.rot_static, J.ts, Q, nv, sm_count())) {
         // Trotter: a warp per vector
         const RowShape h = rows_shape<R>(J.n, J.K, J.rot_static, Q.nrow, 1, nv, sm_count());
-        if ((e = (int)cudaFuncSetAttribute(k_lin_rows<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.bytes)))
-            return e;
+        if ((e = allow_smem(k_lin_rows<R>, h.bytes))) return e;
         k_lin_rows<R><<<(unsigned)((nv + h.vecs - 1) / h.vecs), 32 * h.vecs, h.bytes, st>>>(J, Q, h.stage);
     } else {
         size_t lane_b = singles_lane_bytes<R>(J.n, J.prop);
         int B = 64;
         while (B > 1 && (size_t)B * lane_b > 200 * 1024) B >>= 1;
         size_t sm = lane_b * B;
-        if (sm > 48 * 1024 &&
-            (e = (int)cudaFuncSetAttribute(k_lin<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm)))
-            return e;
+        if ((e = allow_smem(k_lin<R>, sm))) return e;
         k_lin<R><<<(unsigned)((nv + B - 1) / B), B, sm, st>>>(J);
     }
     if ((e = (int)cudaGetLastError())) return e;
@@ -545,10 +541,10 @@ int lum_weights(nise_ctx *c, const DevTraj &T, int begin, int end, int singleshi
     auto weigh = [&](int i0, int i1) -> int {
         if (i1 <= i0) return 0;
         if (large) {
-            cudaFuncSetAttribute(k_lum_exact<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            allow_smem(k_lum_exact<true>, sm);
             k_lum_exact<true><<<i1 - i0, 256, sm, st>>>(T, N, p.sample, begin, V.p, w.p, dit.p + i0, kBT, init.p);
         } else {
-            cudaFuncSetAttribute(k_lum_exact<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            allow_smem(k_lum_exact<false>, sm);
             k_lum_exact<false><<<i1 - i0, 256, sm, st>>>(T, N, p.sample, begin, V.p, w.p, dit.p + i0, kBT, init.p);
         }
         c->launches++;

@@ -175,10 +175,7 @@ int run_rk4_row(const DevTraj &T, const Rk4Plan &P, const AbsJob &J, double2 *re
     auto kern = warp ? (sm ? k_abs_rk4_row<R, true, true> : k_abs_rk4_row<R, false, true>)
                      : (sm ? k_abs_rk4_row<R, true, false> : k_abs_rk4_row<R, false, false>);
     const size_t bytes = sm ? all : base;
-    if (bytes > 48 * 1024) {
-        const int e = (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        if (e) return e;
-    }
+    if (const int e = allow_smem(kern, bytes)) return e;
     kern<<<J.nsamp, 3 * G, bytes, s>>>(T, P, J, resp, G);
     return (int)cudaGetLastError();
 }
@@ -285,8 +282,7 @@ int run_step_rk4(int n, float cut, const float *H, R *re, R *im, int nvec, int t
     const size_t base = sizeof(double2) * 2 * (size_t)n + sizeof(R) * 2 * n, all = base + sizeof(float) * (size_t)n * (n + 1) / 2;
     const bool vs = all <= 200 * 1024;
     auto kern = vs ? k_step_rk4_row<R, true> : k_step_rk4_row<R, false>;
-    const int e = (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(vs ? all : base));
-    if (e) return e;
+    if (const int e = allow_smem(kern, vs ? all : base)) return e;
     kern<<<nvec, (n + 31) / 32 * 32, vs ? all : base, s>>>(n, cut, H, re, im, ts, fsub);
     return (int)cudaGetLastError();
 }

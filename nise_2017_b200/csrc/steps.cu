@@ -158,8 +158,7 @@ int run_coupling(int n, float cut, const float *H, R *re, R *im, int nvec, int t
     // and 16 sites with 50 000 vectors 0.39, 1.51 and 3.78 ms against 0.33, 1.32 and 3.66,
     // with 10 000 0.12, 0.38 and 0.87 against 0.11, 0.39 and 1.04
     if (bytes > 220 * 1024 || nvec >= 2500L * n) return (int)cudaErrorNotSupported;
-    const int e = (int)cudaFuncSetAttribute(k_step_coupling_cta<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e) return e;
+    if (const int e = allow_smem(k_step_coupling_cta<R>, bytes)) return e;
     k_step_coupling_cta<R><<<nvec, (n + 63) / 64 * 32, bytes, s>>>(n, cut, H, re, im, ts, fsub);
     return (int)cudaGetLastError();
 }
@@ -169,8 +168,7 @@ int run_taylor(int n, const float *H, R *re, R *im, int nvec, double f, cudaStre
     const size_t base = sizeof(typename Vec2<R>::T) * 2 * (size_t)n, all = base + sizeof(float) * (size_t)n * (n + 1) / 2;
     const bool hs = all <= 200 * 1024;
     auto kern = hs ? k_step_taylor_cta<R, true> : k_step_taylor_cta<R, false>;
-    const int e = (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(hs ? all : base));
-    if (e) return e;
+    if (const int e = allow_smem(kern, hs ? all : base)) return e;
     kern<<<nvec, (n + 31) / 32 * 32, hs ? all : base, s>>>(n, H, re, im, f);
     return (int)cudaGetLastError();
 }

@@ -384,9 +384,7 @@ template <int IT, int NT, bool CHEB>
 int run_rv1(const DevTraj &T, const TaylorPlan &P, const AbsJob &J, double2 *resp, int v0, int nvec, cudaStream_t s) {
     const size_t smem = rv_layout(P.n, P.ell8_ntg, NT / 32).total;
     const int sh = P.rv_shape;
-    cudaError_t e =
-        cudaFuncSetAttribute(k_abs_taylor_rv<IT, NT, CHEB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
+    if (const int e = allow_smem(k_abs_taylor_rv<IT, NT, CHEB>, smem)) return e;
     k_abs_taylor_rv<IT, NT, CHEB><<<(nvec + kRvG - 1) / kRvG, NT, smem, s>>>(T, P, J, resp, v0, nvec,
                                                                                P.ell8_tri[sh], P.ell8_rows[sh]);
     return (int)cudaGetLastError();

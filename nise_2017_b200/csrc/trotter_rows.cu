@@ -49,9 +49,7 @@ int run(const DevTraj &T, const SinglesTab &D, const RowPlan &Q, const AbsJob &J
     const int nvec = 3 * J.nsamp;
     const RowShape h = rows_shape<R>(D.n, D.K, D.rot_static, Q.nrow, TW, nvec, sm_count());
     if (!h.vecs) return (int)cudaErrorNotSupported;
-    const int e = (int)cudaFuncSetAttribute(k_abs_trotter_rows<R, TW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            (int)h.bytes);
-    if (e) return e;
+    if (const int e = allow_smem(k_abs_trotter_rows<R, TW>, h.bytes)) return e;
     k_abs_trotter_rows<R, TW><<<(nvec + h.vecs - 1) / h.vecs, 32 * TW * h.vecs, h.bytes, s>>>(T, D, Q, J, resp, nvec,
                                                                                              h.stage);
     return (int)cudaGetLastError();

@@ -330,7 +330,7 @@ template <typename R, typename Kern>
 int run_rows(Kern kern, const TwoD &D, const RowPlan &Q, long vectors, cudaStream_t st) {
     const RowShape h = rows_shape<R>(D.n, D.K, D.rot_static, Q.nrow, 1, vectors, sm_count());
     if (!h.vecs) return (int)cudaErrorNotSupported;
-    if (const int e = (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)h.bytes)) return e;
+    if (const int e = allow_smem(kern, h.bytes)) return e;
     kern<<<(unsigned)((vectors + h.vecs - 1) / h.vecs), 32 * h.vecs, h.bytes, st>>>(D, Q, h.stage);
     return (int)cudaGetLastError();
 }
@@ -2011,13 +2011,6 @@ int launch_2d_leftr(const TwoD &D, int prec, cudaStream_t s) {
 }
 
 
-template <typename K>
-int smem_attr(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024)
-        return (int)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    return 0;
-}
-
 int lanes_for2(size_t bytes_per_lane, int want) {
     int b = want;
     while (b > 1 && (size_t)b * bytes_per_lane > 200 * 1024) b >>= 1;
@@ -2033,9 +2026,9 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf, const RowPlan &Q) {
     int B = lanes_for2(lane_b, 64);
     size_t sm = lane_b * B;
     const int P = (D.T1 + 1) / 2;
-    if ((e = smem_attr(k2d_gb1<R>, sm))) return e;
-    if ((e = smem_attr(k2d_gb3<R>, sm))) return e;
-    if ((e = smem_attr(k2d_se<R>, sm))) return e;
+    if ((e = allow_smem(k2d_gb1<R>, sm))) return e;
+    if ((e = allow_smem(k2d_gb3<R>, sm))) return e;
+    if ((e = allow_smem(k2d_se<R>, sm))) return e;
     // Trotter: a warp per vector while the vectors do not fill the threads
     auto rows = [&](long vectors) { return rows_pay<R>(D.n, D.K, D.rot_static, D.ts, Q, vectors, sm_count()); };
     if (rows((long)D.S * 3 * P)) {
@@ -2056,7 +2049,7 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf, const RowPlan &Q) {
         if (D.T2 > 0) {
             size_t lb2 = 2 * (size_t)D.n * sizeof(R2);
             int B2 = lanes_for2(lb2, 64);
-            if ((e = smem_attr(k2d_t2<R>, lb2 * B2))) return e;
+            if ((e = allow_smem(k2d_t2<R>, lb2 * B2))) return e;
             int nv = D.S * (3 + 3 * D.T1);
             k2d_t2<R><<<(nv + B2 - 1) / B2, B2, lb2 * B2, st>>>(D);
             c->launches++;
@@ -2082,7 +2075,7 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf, const RowPlan &Q) {
             const bool sm = all <= 227 * 1024;  // up to 53 sites
             auto kern = sm ? (D.trunc ? k2d_doubles_sparse32<true, true> : k2d_doubles_sparse32<true, false>)
                            : (D.trunc ? k2d_doubles_sparse32<false, true> : k2d_doubles_sparse32<false, false>);
-            if ((e = smem_attr(kern, sm ? all : small))) return e;
+            if ((e = allow_smem(kern, sm ? all : small))) return e;
             if (!sm && (e = (int)cudaMallocAsync(&ws, sizeof(float) * 4 * VC * N2 * ctas, st))) return e;
             kern<<<ctas, threads, sm ? all : small, st>>>(D, vps, NG, 1.0f, (float *)ws);
         } else {
@@ -2093,10 +2086,10 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf, const RowPlan &Q) {
             const size_t all = sizeof(double2) * mat * (1 + 2 * VC) + small;
             const int ctas = D.S * ((vps + VC - 1) / VC);
             if (all <= 227 * 1024) {  // up to 68 sites
-                if ((e = smem_attr(k2d_doubles_sparse64<true>, all))) return e;
+                if ((e = allow_smem(k2d_doubles_sparse64<true>, all))) return e;
                 k2d_doubles_sparse64<true><<<ctas, 256, all, st>>>(D, vps, VC, nullptr);
             } else {
-                if ((e = smem_attr(k2d_doubles_sparse64<false>, small))) return e;
+                if ((e = allow_smem(k2d_doubles_sparse64<false>, small))) return e;
                 if ((e = (int)cudaMallocAsync(&ws, sizeof(double2) * mat * 2 * VC * ctas, st))) return e;
                 k2d_doubles_sparse64<false><<<ctas, 256, small, st>>>(D, vps, VC, (double2 *)ws);
             }
@@ -2150,7 +2143,7 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf, const RowPlan &Q) {
             int np = std::min(tw == 1 ? 4 : 8, (vps + 1) / 2);
             while (np > 1 && bytes_pair(np) > 227 * 1024) np--;
             auto kern = tw == 1 ? k2d_doubles_pair<false> : k2d_doubles_pair<true>;
-            if ((e = smem_attr(kern, bytes_pair(np)))) return e;
+            if ((e = allow_smem(kern, bytes_pair(np)))) return e;
             kern<<<D.S * ((vps + 2 * np - 1) / (2 * np)), 32 * tw * np, bytes_pair(np), st>>>(
                 D, vps, (const Dcoef<float> *)cf, 1.0f, -1.0f);
         } else if (sizeof(R) == 8 && D.n > 32 && D.n <= 64 && c->p.kernel_config != 1) {
@@ -2160,16 +2153,16 @@ int run_chunk(nise_ctx *c, TwoD &D, Dcoef<R> *cf, const RowPlan &Q) {
             const size_t dsm2 = bytes_duo(np, tab);
             if (dsm2 > 220 * 1024) return (int)cudaErrorNotSupported;
             const int cps2 = (vps + np - 1) / np;
-            if ((e = smem_attr(k2d_doubles_duo<double>, dsm2))) return e;
+            if ((e = allow_smem(k2d_doubles_duo<double>, dsm2))) return e;
             k2d_doubles_duo<double><<<D.S * cps2, 64 * np, dsm2, st>>>(D, vps, (Dcoef<double> *)cf, tab);
         } else if (D.n <= 32) {
-            if ((e = smem_attr(k2d_doubles<R, 1>, dsm))) return e;
+            if ((e = allow_smem(k2d_doubles<R, 1>, dsm))) return e;
             k2d_doubles<R, 1><<<D.S * cps, 32 * nwarps, dsm, st>>>(D, vps, cf, use_tab);
         } else if (D.n <= 64) {
-            if ((e = smem_attr(k2d_doubles<R, 2>, dsm))) return e;
+            if ((e = allow_smem(k2d_doubles<R, 2>, dsm))) return e;
             k2d_doubles<R, 2><<<D.S * cps, 32 * nwarps, dsm, st>>>(D, vps, cf, use_tab);
         } else {
-            if ((e = smem_attr(k2d_doubles<R, 4>, dsm))) return e;
+            if ((e = allow_smem(k2d_doubles<R, 4>, dsm))) return e;
             k2d_doubles<R, 4><<<D.S * cps, 32 * nwarps, dsm, st>>>(D, vps, cf, use_tab);
         }
         c->launches++;
