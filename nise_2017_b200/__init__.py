@@ -41,7 +41,7 @@ EXPORTED = [
     "nise_backward_absorption", "nise_absorption_tune", "nise_batch_create", "nise_batch_run", "nise_batch_result",
     "nise_batch_spectrum", "nise_batch_timing", "nise_batch_error", "nise_batch_destroy", "nise_set_trajectory_onfly",
     "nise_set_operators", "nise_linear", "nise_linear_file", "nise_write_td", "nise_translate",
-    "nise_rotation_schedule",
+    "nise_rotation_schedule", "nise_trotter_needs_bank_order",
 ]
 
 
