@@ -634,11 +634,11 @@ int AbsRun::plan(nise_ctx *ctx, bool autotune) {
             tc_starts = use_tc && !plain && N <= 1024 && tc_dia_starts_pays(J, N, nf) &&
                         r2 * (size_t)nf * N * N <= ((size_t)8 << 30);
             stream_u = use_tc && !plain && !tc_starts;
-            if (N > (stream_u || tc_starts ? 2048 : 1024))
+            if (N > (stream_u ? 2048 : 1024))
                 return nise_fail(c, NISE_ERR_UNSUPPORTED,
                                  "the eigen route (Threshold > 0, per-frame couplings, kernel_config 2) is limited to "
                                  "%d sites here (2048 with the tensor-core apply of a batched FP32 job)",
-                                 stream_u || tc_starts ? 2048 : 1024);
+                                 stream_u ? 2048 : 1024);
             // frames per eigensolver launch (one CTA per frame): a wave of
             // the 148 SMs, or as many as 1 GB of eigenvectors, QR workspace
             // (and streamed U) holds, at most 16 GB
@@ -1121,8 +1121,8 @@ int AbsRun::run_main(cudaStream_t s, int cfg, double2 *dst) {
         }
         default:
             if (stream_u) {
-                // chunks of FC frames: eigendecompositions, propagators, then
-                // the tensor-core steps of those frames
+                // chunks of FC frames: their propagators, then the tensor-core
+                // steps of those frames
                 int er = 0;
                 for (long q = 0; q < nf && !er; q += FC) {
                     const long m = std::min(FC, nf - q);
