@@ -92,7 +92,7 @@ bool rows64_possible(int N, bool rot_static, int nvec) { return rot_static && N 
 int default_rows(int prec, int N, bool rot_static, bool wide, int nvec, int tmax, RowCounts rows, long ops, long chunks) {
     const long sms = sm_count();
     auto waves = [&](int w) { return (nvec + rows.vecs[w] * sms - 1) / (rows.vecs[w] * sms); };
-    if (!rows.vecs[0] || !rows_possible(prec, N, rot_static, nvec) || (double)nvec * rows.n[0] >= 860.0 * ops) return 0;
+    if (!rows.vecs[0] || tmax < 2 || !rows_possible(prec, N, rot_static, nvec) || (double)nvec * rows.n[0] >= 860.0 * ops) return 0;
     if (rows64_possible(N, rot_static, nvec) && rows.vecs[1] && waves(1) == 1 && 4 * rows.n[1] < 3 * rows.n[0]) return 36;
     if (!rot_static && wide && tmax < 16) return 0;
     if (waves(0) == 1) return 35;

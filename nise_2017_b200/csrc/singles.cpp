@@ -65,7 +65,8 @@ int nise_singles_tables(nise_ctx *c, const DevTraj &T, long fmin, long nf, int s
         c->launches += 1 + P.rot_static;
         S.U = B.U.p;
         S.rot = B.rot.p;
-        if (N + 64 <= NISE_ROW_MAX && K <= NISE_ROW_MAX && p.ts >= 1) {
+        // (a single coupling leaves nothing to put side by side)
+        if (K >= 2 && N + 64 <= NISE_ROW_MAX && K <= NISE_ROW_MAX && p.ts >= 1) {
             std::vector<uint32_t> ab;
             std::vector<uint16_t> id;
             pairs.pop_back();

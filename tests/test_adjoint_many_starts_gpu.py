@@ -38,3 +38,26 @@ def test_many_start_points(n, tmp_path):
             out[begin, end] = end * np.concatenate([sr, si, g[0], [g[1], g[2]]])
     assert helpers.rel(out[0, few] + out[few, most], out[0, most]) < 1e-10
     assert best[0, most] < 0.3 * most / few * best[0, few], best
+
+
+@pytest.mark.parametrize("n, geometry", [(300, synth.LATTICE), (5, synth.CLUSTER)])
+def test_next_to_no_steps(n, geometry, tmp_path):
+    """RunTimes 1: no schedule is made for a job without steps (and 2 and 9 on either
+    side of its line for 5 sites), the spectrum is that of the FP64 absorption."""
+    files = synth.write(synth.c3_spec(n_sites=n, frames=60, geometry=geometry, seed=n), str(tmp_path))
+    best = {}
+    for T in (1, 2, 9, 16):
+        kw = synth.c3_keywords(Singles=n, Length=60, RunTimes="%d 0 0" % T, Samplerate=3, EndPoint=14, FFT=64, Lifetime=900)
+        with nise.Context(nise.params_from_keywords(kw, files, precision=nise.FP64)) as c:
+            c.load_files()
+            times = []
+            for _ in range(5):
+                t = time.perf_counter()
+                w, sr, si = c.absorption_model(np.zeros(n), 1.0, 900.0)
+                times.append(time.perf_counter() - t)
+            best[T] = min(times)
+            re, im, count = c.absorption()
+            _, er, ei = c.absorption_fft(re, im, count)
+        assert helpers.rel(sr + 1j * si, er + 1j * ei) < 1e-9
+    if n == 300:
+        assert best[1] < 0.6 * best[2], best
